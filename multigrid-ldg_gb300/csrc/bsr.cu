@@ -19,6 +19,7 @@
 
 #include "api.cuh"
 #include "master_tables.inc"
+#include "repeat.cuh"
 #include "rowdot.cuh"
 
 using namespace mg;
@@ -679,6 +680,7 @@ mgldg_bsr::~mgldg_bsr() {
     dfree(lo32);
     dfree(blk);
     dfree(diag);
+    delete rep;
 }
 
 namespace mg {

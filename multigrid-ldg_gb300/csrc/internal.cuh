@@ -155,6 +155,10 @@ inline void check_launch() { MG_CHECK_CUDA(cudaGetLastError()); }
 
 }  // namespace mg
 
+namespace mg {
+struct RepTable;
+}
+
 // ------------------------------------------------------------- BSR matrix --
 // Block-CSR with sorted columns.  Values are either one block per stored
 // entry (blk == null) or a table of distinct blocks indexed through blk
@@ -180,6 +184,7 @@ struct mgldg_bsr {
     int* blk = nullptr;          // optional block indirection
     std::vector<int> h_blk;
     int64_t nuniq = 0;
+    mg::RepTable* rep = nullptr; // table form of a level operator with few distinct blocks (repeat.cuh)
     int* diag = nullptr;         // per row: position of the diagonal block or -1
     std::vector<int> h_diag;
     ~mgldg_bsr();

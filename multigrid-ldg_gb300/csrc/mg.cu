@@ -26,6 +26,7 @@
 #include "api.cuh"
 #include "mg.cuh"
 #include "tail.cuh"
+#include "repeat.cuh"
 #include "rowdot.cuh"
 
 using namespace mg;
@@ -122,7 +123,8 @@ static void relax(mgldg_mg* m, int i, int n, bool reverse, bool xzero = false) {
     }
     for (int k = 0; k < n; ++k) {
         const bool z = xzero && k == 0;
-        if (!(f16 && jacobi_f16_t<T>(m->ctx, L.A, LV<T>::D(L), LV<T>::b(L), LV<T>::x(L), LV<T>::xt(L),
+        if (!rep_jacobi<T>(m->ctx, L.A, LV<T>::b(L), LV<T>::x(L), LV<T>::xt(L), (T)m->p.omega, z, f16) &&
+            !(f16 && jacobi_f16_t<T>(m->ctx, L.A, LV<T>::D(L), LV<T>::b(L), LV<T>::x(L), LV<T>::xt(L),
                                       (T)m->p.omega, z)))
             jacobi_sweep<T>(m->ctx, L.A, vals, LV<T>::D(L), LV<T>::b(L), LV<T>::x(L), LV<T>::xt(L), (T)m->p.omega,
                             z);
@@ -192,7 +194,10 @@ static void vcycle(mgldg_mg* m, int i, bool xzero) {
     relax<T>(m, i, m->p.npre, false, xzero);
     // r = b - A x ; b_c = T^T r ; x_c = 0
     ctx->cur_level = i;
-    if (!(m->p.precision == MGLDG_PREC_MIXED_F16 &&
+    const bool f16 = m->p.precision == MGLDG_PREC_MIXED_F16;
+    if (!rep_spmv<T>(ctx, L.A, T(-1), LV<T>::x(L), T(1), LV<T>::b(L), LV<T>::r(L), nullptr, nullptr, nullptr,
+                     MGLDG_K_SPMV, f16) &&
+        !(f16 &&
           spmv_f16_t<T>(ctx, L.A, T(-1), LV<T>::x(L), T(1), LV<T>::b(L), LV<T>::r(L))))
         spmv<T>(ctx, L.A, T(-1), LV<T>::x(L), T(1), LV<T>::b(L), LV<T>::r(L));
     spmv<T>(ctx, L.Tt, T(1), LV<T>::r(L), T(0), (const T*)nullptr, LV<T>::b(C), nullptr, nullptr, nullptr,
@@ -402,22 +407,9 @@ __global__ void __launch_bounds__(256) k_pcg_dir(int64_t n, const PcgScalars* sc
 // as float pairs, each product a*d formed as the exact FP32 product of the
 // high parts (its error recovered with an FMA) plus the two cross terms,
 // accumulated as an unnormalised (sum, error) float pair with a two-sum per
-// product (Dekker's and Knuth's error-free transformations).  Relative error
+// product (df_fma, rowdot.cuh).  Relative error
 // of a row sum about 2^-44 of sum |a d|; the lane pair's sums, the output
 // and the fused q.d are FP64.  16 x 16 blocks, one warp per block row.
-// (explicitly rounded operations: a product contracted into the two-sum's
-// addition would break the error-free identities)
-__device__ __forceinline__ void df_fma(float& sh, float& sl, float ah, float al, float dh, float dl) {
-    const float p = __fmul_rn(ah, dh);
-    const float pe = fmaf(ah, dh, -p);
-    const float t = fmaf(ah, dl, fmaf(al, dh, pe));
-    const float s = __fadd_rn(sh, p);
-    const float bb = __fsub_rn(s, sh);
-    const float e = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bb)), __fsub_rn(p, bb));
-    sh = s;
-    sl = __fadd_rn(sl, __fadd_rn(e, t));
-}
-
 __global__ void __launch_bounds__(256) k_spmv_df64(int nbr, const int* __restrict__ row_ptr,
                                                    const int* __restrict__ col_idx, const float* __restrict__ ahi,
                                                    const float* __restrict__ alo, const float* __restrict__ dhi,
@@ -569,6 +561,7 @@ static int launch_rows_df64(mgldg_ctx* ctx, const mgldg_bsr* A, const mgldg_mg* 
 }
 
 static void spmv_df64(mgldg_ctx* ctx, const mgldg_bsr* A, const mgldg_mg* m, double* partials, int* np) {
+    if (rep_df64(ctx, A, m->dhi, m->dlo, m->d, m->q, partials, np)) return;
     if (A->br == 16) {
         const int grid = std::max(1, std::min(std::min((A->nbr + 7) / 8, ctx->sm_count * 16), ctx->n_partials));
         {
@@ -589,6 +582,14 @@ static void spmv_df64(mgldg_ctx* ctx, const mgldg_bsr* A, const mgldg_mg* m, dou
         }
     }
     check_launch();
+}
+
+// the CG's FP64 products (table form of the operator where it has one)
+static void outer_spmv(mgldg_ctx* ctx, const mgldg_bsr* A, double alpha, const double* x, double beta,
+                       const double* yin, double* y, const double* dotv = nullptr, double* partials = nullptr,
+                       int* np = nullptr) {
+    if (!rep_spmv<double>(ctx, A, alpha, x, beta, yin, y, dotv, partials, np, MGLDG_K_SPMV))
+        spmv<double>(ctx, A, alpha, x, beta, yin, y, dotv, partials, np);
 }
 
 static void drop_pcg_graph(mgldg_mg* m) {
@@ -706,7 +707,7 @@ static void pcg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const
     int np = 0;
     // q = A d ; alpha = delta_new / d.q
     if (df) spmv_df64(ctx, A, m, part, &np);
-    else spmv<double>(ctx, A, 1.0, m->d, 0.0, nullptr, m->q, m->d, part, &np);
+    else outer_spmv(ctx, A, 1.0, m->d, 0.0, nullptr, m->q, m->d, part, &np);
     {
         Launch L(ctx, MGLDG_K_VECTOR);
         k_pcg_alpha<<<1, 256, 0, ctx->stream>>>(m->sc, part, np);
@@ -719,7 +720,7 @@ static void pcg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const
             k_pcg_update<<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->d, m->q, x, m->r, 0, part);
         }
         check_launch();
-        spmv<double>(ctx, A, -1.0, x, 1.0, b, m->r, m->r, part, &np);
+        outer_spmv(ctx, A, -1.0, x, 1.0, b, m->r, m->r, part, &np);
     } else {
         {
             Launch L(ctx, MGLDG_K_VECTOR);
@@ -847,7 +848,7 @@ static void pcg_dev(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const doubl
     int np = 0;
     // r = b - A x ; d = M(r) ; delta_new = delta_0 = r.d
     const bool df = df64_ok(m, A) && m->dhi;
-    spmv<double>(ctx, A, -1.0, x, 1.0, b, m->r);
+    outer_spmv(ctx, A, -1.0, x, 1.0, b, m->r);
     if (m->L.empty()) {
         precon(m, m->r, m->d);
         dot_partials<double>(ctx, (int)n, m->r, m->d, part, &np);
@@ -969,10 +970,14 @@ static void level_alloc(mgldg_ctx* ctx, mgldg_mg* m, LevelData& L, bool need_sch
         MG_CHECK_CUDA(cudaMemsetAsync(dstatus, 0, sizeof(int), ctx->stream));
         L.Dinv = dalloc<double>((size_t)L.ne * L.b * L.b);
         block_inverse(ctx, L.A, L.Dinv, dstatus);
+        RepProbe probe;
+        const bool probed = rep_probe(ctx, L.A, probe);
         int h = 0;
         download(ctx, &h, dstatus, 1);
         sync(ctx);
         MG_REQUIRE(h == 0, MGLDG_ERR_NOT_SPD, "singular diagonal block in a level matrix");
+        // operators made of a few distinct blocks get their table form
+        if (probed) rep_finish(ctx, const_cast<mgldg_bsr*>(L.A), L.Dinv, probe);
     } catch (...) {
         dfree(dstatus);
         throw;

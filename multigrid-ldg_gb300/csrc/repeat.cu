@@ -1,0 +1,1008 @@
+// repeat.cu -- level operators with few distinct blocks.
+//
+// On grids with constant coefficients the LDG operator and every Galerkin
+// coarse operator consist of a handful of distinct blocks (17 on every level
+// of a uniform grid, tens to hundreds on an adaptive quadtree), and most
+// off-diagonal blocks have only P nonzero rows or columns of P^2.  The general
+// kernels read all blocks from HBM (1.3 GB per FP32 product of 512 x 512 Q3)
+// and are bound by it, or by the FP64 pipes; here the distinct blocks sit in
+// shared memory, a product moves its vectors and indices only, and all-zero
+// block rows (or columns) are skipped.  Level 0 of 512 x 512 Q3, event times
+// before and after: FP32 sweeps (three full, one from x = 0) 213 -> 36 us on
+// average, FP32 residual 240 -> 34 us, double-float product 410 -> 147 us;
+// 256 x 256 Q3 FP64 sweeps 174 -> 105 us, residual 185 -> 90 us.  What is
+// left: vector traffic and shared-memory reads (FP32), the FP64 pipes (FP64
+// and the conversions of the double-float product).
+//
+// Mapping: the rows are sorted by class (same sequence of table entries) and
+// a warp's rows belong to one class, so a block value read once from shared
+// memory serves all of them.  16 x 16 blocks: two lanes per row, one per
+// column half, E = 1, 2 or 4 rows per lane pair; smaller blocks: one lane per
+// row.  The sums run in the general kernels' order (16 x 16: the two column
+// halves in block order, then their sum; smaller blocks: one sum per column
+// over the blocks, then the columns), and a skipped product is one with a
+// zero block entry, so for finite vectors the results are the general
+// kernels' values.
+#include <algorithm>
+#include <memory>
+#include <type_traits>
+#include <unordered_map>
+
+#include "api.cuh"
+#include "repeat.cuh"
+#include "rowdot.cuh"
+
+using namespace mg;
+
+namespace mg {
+
+RepTable::~RepTable() {
+    if (blk) cudaFree(blk);
+    if (pool) cudaFree(pool);
+    if (slots) cudaFree(slots);
+}
+RepProbe::~RepProbe() {
+    if (mem) cudaFree(mem);
+}
+
+// -------------------------------------------------------------- detection --
+namespace {
+constexpr int kMaxUniq = 2048;    // most distinct blocks kept
+constexpr int kHash = 8192;       // hash slots
+struct HashSlot {
+    unsigned long long key;       // block hash, 0: empty
+    int first;                    // smallest block index with this hash
+    int id;                       // table entry (second step)
+};
+}  // namespace
+
+__device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
+    // finaliser of the SplitMix64 generator (Steele, Lea, Flood 2014)
+    z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ULL;
+    z = (z ^ (z >> 27)) * 0x94d049bb133111ebULL;
+    return z ^ (z >> 31);
+}
+
+__global__ void k_rep_clear(HashSlot* slots, int* head) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < kHash) slots[t] = HashSlot{0ULL, 0x7fffffff, -1};
+    if (t < 2) head[t] = 0;
+}
+
+// One warp per block: hash of its values (with -0 taken as +0), entered into
+// the hash table with the smallest block index.  Once more than kMaxUniq
+// distinct hashes were met the warps stop: an operator without repeated
+// blocks costs this kernel a few microseconds.
+__global__ void __launch_bounds__(256) k_rep_hash(int64_t nnzb, int bsz, const double* __restrict__ val,
+                                                  HashSlot* slots, int* head, int* __restrict__ slot_of) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t k = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); k < nnzb; k += (int64_t)gridDim.x * 8) {
+        if (*(volatile int*)&head[1]) return;
+        unsigned long long h = 0;
+        for (int e = lane; e < bsz; e += 32) {
+            const unsigned long long bits = (unsigned long long)__double_as_longlong(__ldg(val + k * bsz + e) + 0.0);
+            h += mix64(bits + 0x9e3779b97f4a7c15ULL * (unsigned long long)(e + 1));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+        if (lane == 0) {
+            if (h == 0) h = 1;
+            int s = (int)(h & (kHash - 1));
+            int found = -1;
+            for (int probe = 0; probe < kHash; ++probe) {
+                unsigned long long cur = *(volatile unsigned long long*)&slots[s].key;
+                if (cur == 0) {
+                    cur = atomicCAS(&slots[s].key, 0ULL, h);
+                    if (cur == 0) {
+                        if (atomicAdd(&head[0], 1) >= kMaxUniq) *(volatile int*)&head[1] = 1;
+                        cur = h;
+                    }
+                }
+                if (cur == h) {
+                    found = s;
+                    break;
+                }
+                if (*(volatile int*)&head[1]) break;
+                s = (s + 1) & (kHash - 1);
+            }
+            if (found >= 0) {
+                if (*(volatile int*)&slots[found].first > (int)k) atomicMin(&slots[found].first, (int)k);
+                slot_of[k] = found;
+            }
+        }
+    }
+}
+
+// table entry of every block, checked value by value against the entry's
+// first block (a hash collision sets head[1] and the table is not used)
+__global__ void __launch_bounds__(256) k_rep_assign(int64_t nnzb, int bsz, const double* __restrict__ val,
+                                                    const HashSlot* __restrict__ slots, int* head,
+                                                    int* slot_of) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t k = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); k < nnzb; k += (int64_t)gridDim.x * 8) {
+        const HashSlot s = slots[slot_of[k]];
+        bool same = true;
+        for (int e = lane; e < bsz; e += 32)
+            same = same && __double_as_longlong(__ldg(val + k * bsz + e) + 0.0) ==
+                               __double_as_longlong(__ldg(val + (int64_t)s.first * bsz + e) + 0.0);
+        same = __all_sync(0xffffffffu, same);
+        if (lane == 0) {
+            if (!same) head[1] = 1;
+            slot_of[k] = s.id;
+        }
+    }
+}
+
+// first value of line l of an image block, and the block's size
+template <class T, int B>
+struct Img {
+    static constexpr int LD = (B + 3) / 4 * 4;
+    static constexpr int PAD = B == 16 ? 16 / (int)sizeof(T) : 0;
+    static constexpr int SIZE = B * LD + PAD;
+    static __host__ __device__ constexpr int line(int l) { return l * LD + (B == 16 && l >= 8 ? PAD : 0); }
+};
+
+// images of one table entry per CTA (the diagonal entries also fill their
+// inverse block): T = double, float
+template <class T, int B>
+__device__ void fill_image(T* img, const double* a, bool cols, int part) {
+    using I = Img<T, B>;
+    for (int e = threadIdx.x; e < B * I::LD; e += blockDim.x) {
+        const int l = e / I::LD, q = e % I::LD;
+        const double v = q < B ? (cols ? a[q * B + l] : a[l * B + q]) + 0.0 : 0.0;
+        img[I::line(l) + q] = part == 0 ? (T)v : (T)(v - (double)(float)v);
+    }
+}
+
+template <int B>
+__global__ void __launch_bounds__(256) k_rep_tables(const double* __restrict__ val, const int* __restrict__ first,
+                                                    const int* __restrict__ drow, const int* __restrict__ didx,
+                                                    const double* __restrict__ Dinv, RepView t) {
+    __shared__ unsigned rm, cm;
+    __shared__ unsigned long long mx;
+    const int u = blockIdx.x;
+    const double* a = val + (size_t)first[u] * (B * B);
+    if (threadIdx.x == 0) rm = cm = 0u, mx = 0ULL;
+    __syncthreads();
+    for (int e = threadIdx.x; e < B * B; e += blockDim.x) {
+        const double v = fabs(a[e]);
+        if (v != 0.0) {
+            atomicOr(&rm, 1u << (e / B));
+            atomicOr(&cm, 1u << (e % B));
+            atomicMax(&mx, (unsigned long long)__double_as_longlong(v));   // nonnegative doubles order as integers
+        }
+    }
+    __syncthreads();
+    // small blocks are always read by columns
+    const bool cols = B != 16 || __popc(rm) > __popc(cm);
+    using I8 = Img<double, B>;
+    using I4 = Img<float, B>;
+    fill_image<double, B>(t.i64 + (size_t)u * I8::SIZE, a, cols, 0);
+    fill_image<float, B>(t.i32 + (size_t)u * I4::SIZE, a, cols, 0);
+    fill_image<float, B>(t.ilo + (size_t)u * I4::SIZE, a, cols, 1);
+    const double s = mx ? __longlong_as_double((long long)mx) : 1.0;
+    for (int e = threadIdx.x; e < B * B; e += blockDim.x)
+        t.i16[(size_t)u * I4::SIZE + I4::line(e / B) + e % B] = __half2float(__float2half_rn((float)(a[e] / s)));
+    if (drow[u] >= 0) {
+        const double* D = Dinv + (size_t)drow[u] * (B * B);
+        const size_t at = t.nuniq + didx[u];
+        fill_image<double, B>(t.i64 + at * I8::SIZE, D, false, 0);
+        fill_image<float, B>(t.i32 + at * I4::SIZE, D, false, 0);
+        fill_image<float, B>(t.i16 + at * I4::SIZE, D, false, 0);
+    }
+    if (threadIdx.x == 0) {
+        t.mask[u] = rm | (cm << 16);
+        t.s16[u] = (float)s;
+    }
+}
+
+// Rows from which a level is looked at: below, a launch is latency (copying
+// the images, one class after another) and the general kernels, with a warp
+// per row, end sooner.  Measured Jacobi sweeps (event times, us, slot /
+// general): 16 x 16 FP32 16,384 rows 13.1 / 20.3, 4,096 rows 12.6 / 10.0; FP64
+// 16,384 rows 36.9 / 55.9, 4,096 rows 27.8 / 20.0; 9 x 9 FP32 65,536 rows
+// 14.7 / 29.8, 16,384 rows 11.2 / 10.9; FP64 16,384 rows 25.8 / 27.9; 4 x 4
+// FP32 65,536 rows 9.7 / 11.0, 16,384 rows 8.1 / 7.4.
+static int rep_min_rows(int b) { return b == 16 ? 8192 : (b == 9 ? 16384 : 32768); }
+
+static bool rep_shape(const mgldg_bsr* A) {
+    return A->br == A->bc && A->nbr == A->nbc && !A->blk && (A->br == 4 || A->br == 9 || A->br == 16) &&
+           A->nbr >= rep_min_rows(A->br) && A->nnzb < (1LL << 31);
+}
+
+bool rep_probe(mgldg_ctx* ctx, const mgldg_bsr* A, RepProbe& p) {
+    if (!rep_shape(A) || A->rep) return false;
+    const size_t bytes = 16 + kHash * sizeof(HashSlot) + (size_t)A->nnzb * sizeof(int);
+    p.mem = dalloc<char>(bytes);
+    int* head = (int*)p.mem;
+    HashSlot* slots = (HashSlot*)((char*)p.mem + 16);
+    int* slot_of = (int*)(slots + kHash);
+    k_rep_clear<<<kHash / 256, 256, 0, ctx->stream>>>(slots, head);
+    const int g = (int)std::min<int64_t>((A->nnzb + 7) / 8, ctx->sm_count * 8);
+    {
+        Launch L(ctx, MGLDG_K_SETUP);
+        k_rep_hash<<<g, 256, 0, ctx->stream>>>(A->nnzb, (int)A->bsz(), A->val, slots, head, slot_of);
+    }
+    check_launch();
+    download(ctx, p.head, head, 2);
+    return true;
+}
+
+void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
+    // the caller has synchronised: p.head is valid.  A table pays when a
+    // block is used several times.
+    const int nu = p.head[0];
+    if (!p.mem || p.head[1] || nu < 1 || (int64_t)nu * 4 > A->nnzb) return;
+    int* head = (int*)p.mem;
+    HashSlot* slots = (HashSlot*)((char*)p.mem + 16);
+    int* slot_of = (int*)(slots + kHash);
+    const int b = A->br, n = A->nbr, ld = (b + 3) / 4 * 4;
+    std::vector<HashSlot> hs(kHash);
+    download(ctx, hs.data(), slots, hs.size());
+    sync(ctx);
+    // table entries in the order of their first blocks (independent of the
+    // order in which the hashing warps arrived)
+    std::vector<int> order;
+    for (int s = 0; s < kHash; ++s)
+        if (hs[s].key) order.push_back(s);
+    std::sort(order.begin(), order.end(), [&](int x, int y) { return hs[x].first < hs[y].first; });
+    std::vector<int> first(nu), drow(nu, -1);
+    for (int u = 0; u < nu; ++u) {
+        hs[order[u]].id = u;
+        first[u] = hs[order[u]].first;
+    }
+    upload(ctx, slots, hs.data(), hs.size());
+    const int g = (int)std::min<int64_t>((A->nnzb + 7) / 8, ctx->sm_count * 8);
+    {
+        Launch L(ctx, MGLDG_K_SETUP);
+        k_rep_assign<<<g, 256, 0, ctx->stream>>>(A->nnzb, (int)A->bsz(), A->val, slots, head, slot_of);
+    }
+    check_launch();
+    std::vector<int> id(A->nnzb);
+    download(ctx, p.head, head, 2);
+    download(ctx, id.data(), slot_of, id.size());
+    sync(ctx);
+    if (p.head[1]) return;   // two different blocks with one hash
+    // ---- row classes ----
+    const int* rp = A->h_row_ptr.data();
+    const int* ci = A->h_col_idx.data();
+    std::vector<int> cls_of(n), cls;     // cls: kRepCls ints per class
+    bool ok = true;
+    {
+        std::unordered_map<uint64_t, std::vector<int>> seen;
+        uint64_t last_key = 0;
+        int last = -1;
+        for (int i = 0; i < n && ok; ++i) {
+            const int k0 = rp[i], nb = rp[i + 1] - k0, dk = A->h_diag[i];
+            if (nb < 1 || nb > kRepMaxNb || dk < 0) {
+                ok = false;
+                break;
+            }
+            uint64_t key = (uint64_t)nb * 64 + (uint64_t)(dk - k0);
+            for (int q = 0; q < nb; ++q) key = key * 0x100000001b3ULL + (uint64_t)id[k0 + q] + 1;   // FNV-style
+            drow[id[dk]] = drow[id[dk]] < 0 ? i : drow[id[dk]];
+            auto same = [&](int c) {
+                const int* d = &cls[(size_t)c * kRepCls];
+                return d[0] == nb && d[1] == id[dk] && std::equal(d + 4, d + 4 + nb, id.begin() + k0);
+            };
+            int c = -1;
+            if (last >= 0 && key == last_key && same(last)) {
+                c = last;
+            } else {
+                std::vector<int>& v = seen[key];
+                for (int q : v)
+                    if (same(q)) c = q;
+                if (c < 0) {
+                    c = (int)(cls.size() / kRepCls);
+                    v.push_back(c);
+                    cls.resize(cls.size() + kRepCls, 0);
+                    int* d = &cls[(size_t)c * kRepCls];
+                    d[0] = nb;
+                    d[1] = id[dk];
+                    std::copy(id.begin() + k0, id.begin() + k0 + nb, d + 4);
+                }
+            }
+            last = c;
+            last_key = key;
+            cls_of[i] = c;
+        }
+    }
+    if (!ok) return;
+    const int ncls = (int)(cls.size() / kRepCls);
+    // ---- slots: the rows of a chunk sorted by class, each class padded to
+    // whole groups.  Chunks of 4,096 consecutive rows keep a warp's gathers
+    // within one stretch of the vectors; with many classes one chunk wastes
+    // fewer slots. ----
+    const int gs = b != 16 ? 32 : (n >= 131072 ? 64 : (n >= 32768 ? 32 : 16));
+    const int chunk = ncls <= 32 ? 4096 : n;
+    std::vector<int> rows, gcls;
+    {
+        std::vector<int> cnt(ncls + 1), pos(ncls);
+        for (int s = 0; s < n; s += chunk) {
+            const int e = std::min(n, s + chunk);
+            std::fill(cnt.begin(), cnt.end(), 0);
+            for (int i = s; i < e; ++i) cnt[cls_of[i]]++;
+            size_t at = rows.size();
+            for (int c = 0; c < ncls; ++c) {
+                pos[c] = (int)at;
+                const size_t w = ((size_t)cnt[c] + gs - 1) / gs * gs;
+                gcls.insert(gcls.end(), w / 16, c);
+                at += w;
+            }
+            rows.resize(at, -1);
+            for (int i = s; i < e; ++i) rows[pos[cls_of[i]]++] = i;
+        }
+    }
+    // more than twice as many slots as rows: rare classes, mostly idle lanes
+    const int nslots = rows.size() > 2 * (size_t)n ? 0 : (int)rows.size();
+    std::unique_ptr<RepTable> t(new RepTable());
+    t->b = b;
+    t->ld = ld;
+    t->nbr = n;
+    t->nuniq = nu;
+    t->ncls = ncls;
+    t->gs = gs;
+    t->nslots = nslots;
+    // the classes name their inverse diagonal block by its place in the image
+    std::vector<int> didx(nu, -1);
+    for (int u = 0; u < nu; ++u)
+        if (drow[u] >= 0) didx[u] = t->ndiag++;
+    for (int c = 0; c < ncls; ++c) cls[(size_t)c * kRepCls + 1] = didx[cls[(size_t)c * kRepCls + 1]];
+    // ---- device tables ----
+    const size_t nimg = (size_t)nu + t->ndiag;
+    const size_t v8 = (size_t)(b == 16 ? Img<double, 16>::SIZE : b * ld) * nimg;
+    const size_t v4 = (size_t)(b == 16 ? Img<float, 16>::SIZE : b * ld) * nimg;
+    t->pool = dalloc<char>(v8 * 8 + 3 * v4 * 4 + (size_t)nu * 8);
+    MG_CHECK_CUDA(cudaMemsetAsync(t->pool, 0, v8 * 8 + 3 * v4 * 4, ctx->stream));
+    t->i64 = (double*)t->pool;
+    t->i32 = (float*)(t->i64 + v8);
+    t->ilo = t->i32 + v4;
+    t->i16 = t->ilo + v4;
+    t->s16 = t->i16 + v4;
+    t->mask = (unsigned*)(t->s16 + nu);
+    t->blk = dalloc<int>(A->nnzb);
+    int* dint = (int*)slots;   // the hash slots are done with: three index lists go there
+    upload(ctx, dint, first.data(), first.size());
+    upload(ctx, dint + nu, drow.data(), drow.size());
+    upload(ctx, dint + 2 * nu, didx.data(), didx.size());
+    {
+        Launch L(ctx, MGLDG_K_SETUP);
+        const RepView& v = *t;
+        if (b == 4) k_rep_tables<4><<<nu, 256, 0, ctx->stream>>>(A->val, dint, dint + nu, dint + 2 * nu, Dinv, v);
+        else if (b == 9) k_rep_tables<9><<<nu, 256, 0, ctx->stream>>>(A->val, dint, dint + nu, dint + 2 * nu, Dinv, v);
+        else k_rep_tables<16><<<nu, 256, 0, ctx->stream>>>(A->val, dint, dint + nu, dint + 2 * nu, Dinv, v);
+    }
+    check_launch();
+    MG_CHECK_CUDA(cudaMemcpyAsync(t->blk, slot_of, (size_t)A->nnzb * sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
+    if (nslots) {
+        std::vector<int> cols((size_t)kRepMaxNb * nslots);
+        int most = 0;
+        for (int c = 0; c < ncls; ++c) most = std::max(most, cls[(size_t)c * kRepCls]);
+        for (int s = 0; s < nslots; ++s) {
+            // padding slots read what their group's first row reads
+            const int i = rows[s] >= 0 ? rows[s] : rows[s / gs * gs];
+            const int nb = rp[i + 1] - rp[i];
+            for (int q = 0; q < most; ++q) cols[(size_t)q * nslots + s] = ci[rp[i] + std::min(q, nb - 1)];
+        }
+        const size_t nc = cls.size(), ng = gcls.size();
+        t->slots = dalloc<int>(nc + ng + nslots + (size_t)most * nslots + 16);
+        t->cls = (int*)t->slots;
+        t->cols = t->cls + nc;
+        t->rows = t->cols + (size_t)most * nslots;
+        t->gcls = t->rows + nslots;
+        upload(ctx, t->cls, cls.data(), nc);
+        upload(ctx, t->cols, cols.data(), (size_t)most * nslots);
+        upload(ctx, t->rows, rows.data(), nslots);
+        upload(ctx, t->gcls, gcls.data(), ng);
+        sync(ctx);   // the host arrays go out of scope
+    }
+    sync(ctx);
+    A->rep = t.release();
+}
+
+// ---------------------------------------------------------------- kernels --
+namespace {
+
+constexpr int kRepSmem = 100 * 1024;   // largest shared-memory image (two CTAs per SM)
+
+template <class T>
+struct RepArgs {
+    int nwarps, nslots, nimg, nuniq;
+    const int *gcls, *rows, *cols, *cls;
+    const unsigned* mask;
+    const T* img;
+    const float* scale;   // FP16 form: block scales
+    const T *x, *b;
+    T* y;
+    T alpha, beta, omega;
+    int xzero;
+    const T* dotv;
+    int self_dot;
+    double* partials;
+};
+
+__device__ __forceinline__ float fma_(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return fma(a, b, c); }
+
+// N values (N * sizeof(T) a multiple of 16) with 16-byte accesses; ldc: plain
+// loads, for a line that the same lane may write later
+template <int N>
+__device__ __forceinline__ void lds(const float* p, float (&v)[N]) {
+#pragma unroll
+    for (int q = 0; q < N / 4; ++q) {
+        const float4 t = reinterpret_cast<const float4*>(p)[q];
+        v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
+    }
+}
+template <int N>
+__device__ __forceinline__ void lds(const double* p, double (&v)[N]) {
+#pragma unroll
+    for (int q = 0; q < N / 2; ++q) {
+        const double2 t = reinterpret_cast<const double2*>(p)[q];
+        v[2 * q] = t.x; v[2 * q + 1] = t.y;
+    }
+}
+template <int N>
+__device__ __forceinline__ void ldg(const float* p, float (&v)[N]) {
+#pragma unroll
+    for (int q = 0; q < N / 4; ++q) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p) + q);
+        v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
+    }
+}
+template <int N>
+__device__ __forceinline__ void ldg(const double* p, double (&v)[N]) {
+#pragma unroll
+    for (int q = 0; q < N / 2; ++q) {
+        const double2 t = __ldg(reinterpret_cast<const double2*>(p) + q);
+        v[2 * q] = t.x; v[2 * q + 1] = t.y;
+    }
+}
+__device__ __forceinline__ void st8(float* p, const float (&v)[8]) {
+    reinterpret_cast<float4*>(p)[0] = make_float4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<float4*>(p)[1] = make_float4(v[4], v[5], v[6], v[7]);
+}
+__device__ __forceinline__ void st8(double* p, const double (&v)[8]) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) reinterpret_cast<double2*>(p)[q] = make_double2(v[2 * q], v[2 * q + 1]);
+}
+
+// copies the image (nvec 16-byte words) to shared memory
+__device__ __forceinline__ void load_image(const void* g, void* s, int nvec) {
+    const float4* gp = reinterpret_cast<const float4*>(g);
+    float4* sp = reinterpret_cast<float4*>(s);
+#pragma unroll 8
+    for (int i = threadIdx.x; i < nvec; i += blockDim.x) sp[i] = __ldg(gp + i);
+    __syncthreads();
+}
+
+// CTA sum of dacc into partials[blockIdx.x] (fixed order)
+__device__ __forceinline__ void rep_partial(double dacc, double* partials) {
+    __shared__ double sm[8];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) dacc += __shfl_xor_sync(0xffffffffu, dacc, o);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = dacc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += sm[w];
+        partials[blockIdx.x] = t;
+    }
+}
+
+// the lane pair (column halves) holds two partial sums of 16 rows each; the
+// lane gets the sums of the 8 rows of its half
+template <class T>
+__device__ __forceinline__ void pair_sum(const T (&p)[16], int half, T (&s)[8]) {
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const T other = __shfl_xor_sync(0xffffffffu, half ? p[r] : p[r + 8], 1);
+        s[r] = (half ? p[r + 8] : p[r]) + other;
+    }
+}
+
+// p[e] += the lane's column half of (A x)_i for its E rows (slots slot + 16 e)
+template <class T, int E, bool F16>
+__device__ __forceinline__ void acc16(const RepArgs<T>& a, const T* simg, const int* cls, int slot, int half,
+                                      T (&p)[E][16]) {
+    using I = Img<T, 16>;
+    const int nb = __ldg(cls);
+    int id = __ldg(cls + 4);
+#pragma unroll 1
+    for (int k = 0; k < nb; ++k) {
+        T xv[E][8];
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+            ldg<8>(a.x + (size_t)__ldg(a.cols + (size_t)k * a.nslots + slot + 16 * e) * 16 + 8 * half, xv[e]);
+        const unsigned m = __ldg(a.mask + id), rm = m & 0xffffu, cm = m >> 16;
+        const T* ab = simg + id * I::SIZE;
+        if (F16 || __popc(rm) <= __popc(cm)) {
+            const T sc = F16 ? (T)__ldg(a.scale + id) : T(0);
+#pragma unroll
+            for (int r = 0; r < 16; ++r)
+                if ((rm >> r) & 1u) {
+                    T av[8];
+                    lds<8>(ab + I::line(r) + 8 * half, av);
+#pragma unroll
+                    for (int e = 0; e < E; ++e) {
+                        if (F16) {
+                            T t = av[0] * xv[e][0];
+#pragma unroll
+                            for (int c = 1; c < 8; ++c) t = fma_(av[c], xv[e][c], t);
+                            p[e][r] = fma_(sc, t, p[e][r]);
+                        } else {
+#pragma unroll
+                            for (int c = 0; c < 8; ++c) p[e][r] = fma_(av[c], xv[e][c], p[e][r]);
+                        }
+                    }
+                }
+        } else {
+            const unsigned any = cm | (cm >> 8);
+            const T* ac = ab + (half ? I::line(8) : 0);
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+                if ((any >> c) & 1u) {
+                    T av[16];
+                    lds<16>(ac + c * 16, av);
+#pragma unroll
+                    for (int e = 0; e < E; ++e)
+#pragma unroll
+                        for (int r = 0; r < 16; ++r) p[e][r] = fma_(av[r], xv[e][c], p[e][r]);
+                }
+        }
+        if (k + 1 < nb) id = __ldg(cls + 5 + k);
+    }
+}
+
+// 16 x 16 blocks.  JACOBI: y = x + omega Dinv (b - A x); else y = alpha A x + beta b
+template <class T, int E, bool JACOBI, bool F16>
+__global__ void __launch_bounds__(128) k_rep16(const RepArgs<T> a) {
+    using I = Img<T, 16>;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    T* simg = reinterpret_cast<T*>(smraw);
+    const bool zero = JACOBI && a.xzero;
+    // the sweep from x = 0 reads the inverse diagonal blocks only
+    const int first = zero ? a.nuniq : 0;
+    load_image(a.img + (size_t)first * I::SIZE, simg + first * I::SIZE,
+               (a.nimg - first) * (I::SIZE * (int)sizeof(T) / 16));
+    const int lane = threadIdx.x & 31, half = lane & 1;
+    double dacc = 0;
+    for (int w = blockIdx.x * 4 + (threadIdx.x >> 5); w < a.nwarps; w += gridDim.x * 4) {
+        const int slot = w * 16 * E + (lane >> 1);
+        const int* cls = a.cls + (size_t)__ldg(a.gcls + w * E) * kRepCls;
+        T p[E][16];
+#pragma unroll
+        for (int e = 0; e < E; ++e)
+#pragma unroll
+            for (int r = 0; r < 16; ++r) p[e][r] = T(0);
+        if (!zero) acc16<T, E, F16>(a, simg, cls, slot, half, p);
+        if constexpr (JACOBI) {
+            T t[E][8];
+            size_t o[E];
+            bool live[E];
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const int row = __ldg(a.rows + slot + 16 * e);
+                live[e] = row >= 0;
+                o[e] = (size_t)max(row, 0) * 16 + 8 * half;
+                T bv[8];
+                ldg<8>(a.b + o[e], bv);
+                if (zero) {
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) t[e][r] = bv[r];
+                } else {
+                    pair_sum(p[e], half, t[e]);
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) t[e][r] = bv[r] - t[e][r];
+                }
+            }
+            const T* D = simg + (size_t)(a.nuniq + __ldg(cls + 1)) * I::SIZE;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                T dv[8];
+                lds<8>(D + I::line(r) + 8 * half, dv);
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    T y = dv[0] * t[e][0];
+#pragma unroll
+                    for (int c = 1; c < 8; ++c) y = fma_(dv[c], t[e][c], y);
+                    p[e][r] = y;
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                T yv[8], xi[8];
+                pair_sum(p[e], half, yv);
+                if (zero) {
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) xi[r] = T(0);
+                } else {
+                    ldg<8>(a.x + o[e], xi);
+                }
+#pragma unroll
+                for (int r = 0; r < 8; ++r) xi[r] = xi[r] + a.omega * yv[r];
+                if (live[e]) st8(a.y + o[e], xi);
+            }
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                T s[8];
+                pair_sum(p[e], half, s);
+                const int row = __ldg(a.rows + slot + 16 * e);
+                if (row < 0) continue;
+                const size_t o = (size_t)row * 16 + 8 * half;
+                T v[8], bv[8];
+                if (a.beta != T(0)) lds<8>(a.b + o, bv);   // yin may be y: plain loads, this lane's entries only
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    v[r] = a.alpha * s[r];
+                    if (a.beta != T(0)) v[r] += a.beta * bv[r];
+                }
+                st8(a.y + o, v);
+                if (a.self_dot) {
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) dacc += (double)v[r] * (double)v[r];
+                } else if (a.dotv) {
+                    ldg<8>(a.dotv + o, bv);
+#pragma unroll
+                    for (int r = 0; r < 8; ++r) dacc += (double)v[r] * (double)bv[r];
+                }
+            }
+        }
+    }
+    if (!JACOBI && a.partials) rep_partial(dacc, a.partials);
+}
+
+// Blocks of 4 and 9, one row per lane: CB columns at a time, one sum per
+// (row, column) over the row's blocks, then the columns in order.
+template <class T, int B, bool JACOBI>
+__global__ void __launch_bounds__(128) k_repc(const RepArgs<T> a) {
+    using I = Img<T, B>;
+    constexpr int CB = B == 9 ? 3 : 4, LD = I::LD;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    T* simg = reinterpret_cast<T*>(smraw);
+    const bool zero = JACOBI && a.xzero;
+    const int first = zero ? a.nuniq : 0;
+    load_image(a.img + (size_t)first * I::SIZE, simg + first * I::SIZE,
+               (a.nimg - first) * (I::SIZE * (int)sizeof(T) / 16));
+    const int lane = threadIdx.x & 31;
+    double dacc = 0;
+    for (int w = blockIdx.x * 4 + (threadIdx.x >> 5); w < a.nwarps; w += gridDim.x * 4) {
+        const int slot = w * 32 + lane;
+        const int* cls = a.cls + (size_t)__ldg(a.gcls + 2 * w) * kRepCls;
+        T s[B];
+#pragma unroll
+        for (int r = 0; r < B; ++r) s[r] = T(0);
+        if (!zero) {
+            const int nb = __ldg(cls);
+#pragma unroll 1
+            for (int cb = 0; cb < B; cb += CB) {
+                T acc[CB][B];
+#pragma unroll
+                for (int q = 0; q < CB; ++q)
+#pragma unroll
+                    for (int r = 0; r < B; ++r) acc[q][r] = T(0);
+#pragma unroll 2
+                for (int k = 0; k < nb; ++k) {
+                    const int id = __ldg(cls + 4 + k);
+                    const unsigned cm = __ldg(a.mask + id) >> (16 + cb);
+                    if (!(cm & ((1u << CB) - 1u))) continue;
+                    const T* ac = simg + id * I::SIZE + cb * LD;
+                    const T* xp = a.x + (size_t)__ldg(a.cols + (size_t)k * a.nslots + slot) * B + cb;
+                    T xv[CB];
+#pragma unroll
+                    for (int q = 0; q < CB; ++q) xv[q] = __ldg(xp + q);
+#pragma unroll
+                    for (int q = 0; q < CB; ++q) {
+                        if (!((cm >> q) & 1u)) continue;
+                        T av[LD];
+                        lds<LD>(ac + q * LD, av);
+#pragma unroll
+                        for (int r = 0; r < B; ++r) acc[q][r] = fma_(av[r], xv[q], acc[q][r]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < CB; ++q)
+#pragma unroll
+                    for (int r = 0; r < B; ++r) s[r] += acc[q][r];
+            }
+        }
+        const int row = __ldg(a.rows + slot);
+        const size_t o = (size_t)max(row, 0) * B;
+        if constexpr (JACOBI) {
+            const T* D = simg + (size_t)(a.nuniq + __ldg(cls + 1)) * I::SIZE;
+#pragma unroll
+            for (int r = 0; r < B; ++r) s[r] = __ldg(a.b + o + r) - s[r];
+#pragma unroll
+            for (int r = 0; r < B; ++r) {
+                T dv[LD];
+                lds<LD>(D + r * LD, dv);
+                T y = T(0);
+#pragma unroll
+                for (int c = 0; c < B; ++c) y = fma_(dv[c], s[c], y);
+                const T xi = zero ? T(0) : __ldg(a.x + o + r);
+                if (row >= 0) a.y[o + r] = xi + a.omega * y;
+            }
+        } else if (row >= 0) {
+#pragma unroll
+            for (int r = 0; r < B; ++r) {
+                T v = a.alpha * s[r];
+                if (a.beta != T(0)) v += a.beta * a.b[o + r];
+                a.y[o + r] = v;
+                if (a.self_dot) dacc += (double)v * (double)v;
+                else if (a.dotv) dacc += (double)v * (double)__ldg(a.dotv + o + r);
+            }
+        }
+    }
+    if (!JACOBI && a.partials) rep_partial(dacc, a.partials);
+}
+
+struct RepDfArgs {
+    int nwarps, nslots, nuniq;
+    const int *gcls, *rows, *cols, *cls;
+    const unsigned* mask;
+    const float *img, *imglo;
+    const float *xh, *xl;
+    const double* d;
+    double* q;
+    double* partials;
+};
+
+// q = A d in double-float arithmetic, 16 x 16 blocks, two lanes per row: a
+// float-pair sum per row and column half, their FP64 sum, the partial d.q
+__global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
+    using I = Img<float, 16>;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    float* sh_ = reinterpret_cast<float*>(smraw);
+    float* sl_ = sh_ + a.nuniq * I::SIZE;
+    load_image(a.img, sh_, a.nuniq * (I::SIZE / 4));
+    load_image(a.imglo, sl_, a.nuniq * (I::SIZE / 4));
+    const int lane = threadIdx.x & 31, half = lane & 1;
+    double dacc = 0;
+    for (int w = blockIdx.x * 4 + (threadIdx.x >> 5); w < a.nwarps; w += gridDim.x * 4) {
+        const int slot = w * 16 + (lane >> 1);
+        const int* cls = a.cls + (size_t)__ldg(a.gcls + w) * kRepCls;
+        const int nb = __ldg(cls);
+        float sh[16], sl[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) sh[r] = sl[r] = 0.f;
+#pragma unroll 1
+        for (int k = 0; k < nb; ++k) {
+            const int id = __ldg(cls + 4 + k);
+            const unsigned m = __ldg(a.mask + id), rm = m & 0xffffu, cm = m >> 16;
+            const size_t xo = (size_t)__ldg(a.cols + (size_t)k * a.nslots + slot) * 16 + 8 * half;
+            float xh[8], xl[8];
+            ldg<8>(a.xh + xo, xh);
+            ldg<8>(a.xl + xo, xl);
+            const int bo = id * I::SIZE;
+            if (__popc(rm) <= __popc(cm)) {
+#pragma unroll
+                for (int r = 0; r < 16; ++r)
+                    if ((rm >> r) & 1u) {
+                        float ah[8], al[8];
+                        lds<8>(sh_ + bo + I::line(r) + 8 * half, ah);
+                        lds<8>(sl_ + bo + I::line(r) + 8 * half, al);
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) df_fma(sh[r], sl[r], ah[c], al[c], xh[c], xl[c]);
+                    }
+            } else {
+                const unsigned any = cm | (cm >> 8);
+                const int co = bo + (half ? I::line(8) : 0);
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    if ((any >> c) & 1u) {
+                        float ah[16], al[16];
+                        lds<16>(sh_ + co + c * 16, ah);
+                        lds<16>(sl_ + co + c * 16, al);
+#pragma unroll
+                        for (int r = 0; r < 16; ++r) df_fma(sh[r], sl[r], ah[r], al[r], xh[c], xl[c]);
+                    }
+            }
+        }
+        double v[16], qv[8];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) v[r] = (double)sh[r] + (double)sl[r];
+        pair_sum(v, half, qv);
+        const int row = __ldg(a.rows + slot);
+        if (row >= 0) {
+            const size_t o = (size_t)row * 16 + 8 * half;
+            double dv[8];
+            ldg<8>(a.d + o, dv);
+            st8(a.q + o, qv);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) dacc += qv[r] * dv[r];
+        }
+    }
+    rep_partial(dacc, a.partials);
+}
+
+// the same for blocks of 4 and 9, one lane per row: one float-pair sum per
+// (row, column) over the row's blocks, summed over the columns in FP64
+template <int B>
+__global__ void __launch_bounds__(128) k_repc_df64(const RepDfArgs a) {
+    using I = Img<float, B>;
+    constexpr int LD = I::LD;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    float* sh_ = reinterpret_cast<float*>(smraw);
+    float* sl_ = sh_ + a.nuniq * I::SIZE;
+    load_image(a.img, sh_, a.nuniq * (I::SIZE / 4));
+    load_image(a.imglo, sl_, a.nuniq * (I::SIZE / 4));
+    const int lane = threadIdx.x & 31;
+    double dacc = 0;
+    for (int w = blockIdx.x * 4 + (threadIdx.x >> 5); w < a.nwarps; w += gridDim.x * 4) {
+        const int slot = w * 32 + lane;
+        const int* cls = a.cls + (size_t)__ldg(a.gcls + 2 * w) * kRepCls;
+        const int nb = __ldg(cls);
+        double v[B];
+#pragma unroll
+        for (int r = 0; r < B; ++r) v[r] = 0.0;
+#pragma unroll 1
+        for (int c = 0; c < B; ++c) {
+            float sh[B], sl[B];
+#pragma unroll
+            for (int r = 0; r < B; ++r) sh[r] = sl[r] = 0.f;
+#pragma unroll 2
+            for (int k = 0; k < nb; ++k) {
+                const int id = __ldg(cls + 4 + k);
+                if (!((__ldg(a.mask + id) >> (16 + c)) & 1u)) continue;
+                const size_t xo = (size_t)__ldg(a.cols + (size_t)k * a.nslots + slot) * B + c;
+                const float xh = __ldg(a.xh + xo), xl = __ldg(a.xl + xo);
+                float ah[LD], al[LD];
+                lds<LD>(sh_ + id * I::SIZE + c * LD, ah);
+                lds<LD>(sl_ + id * I::SIZE + c * LD, al);
+#pragma unroll
+                for (int r = 0; r < B; ++r) df_fma(sh[r], sl[r], ah[r], al[r], xh, xl);
+            }
+#pragma unroll
+            for (int r = 0; r < B; ++r) v[r] += (double)sh[r] + (double)sl[r];
+        }
+        const int row = __ldg(a.rows + slot);
+        if (row >= 0) {
+            const size_t o = (size_t)row * B;
+#pragma unroll
+            for (int r = 0; r < B; ++r) {
+                a.q[o + r] = v[r];
+                dacc += v[r] * __ldg(a.d + o + r);
+            }
+        }
+    }
+    rep_partial(dacc, a.partials);
+}
+
+template <class T>
+RepArgs<T> rep_args(const RepTable* t, bool f16) {
+    RepArgs<T> a{};
+    a.nslots = t->nslots;
+    a.nuniq = t->nuniq;
+    a.nimg = t->nuniq + t->ndiag;
+    a.gcls = t->gcls;
+    a.rows = t->rows;
+    a.cols = t->cols;
+    a.cls = t->cls;
+    a.mask = t->mask;
+    if constexpr (std::is_same<T, float>::value) {
+        a.img = f16 ? t->i16 : t->i32;
+        a.scale = t->s16;
+    } else {
+        a.img = t->i64;
+    }
+    return a;
+}
+
+// one launch of a slot kernel (128 threads, `smem` bytes of images): as many
+// CTAs as fit at once, so that each copies the images once; false when the
+// images are too large
+template <class K, class A>
+bool rep_launch_k(mgldg_ctx* ctx, K kern, const A& a, size_t smem, int kclass, int* npart) {
+    if (smem > (size_t)kRepSmem) return false;
+    if (smem > 48 * 1024)
+        MG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRepSmem));
+    int per_sm = 0;
+    MG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 128, smem));
+    int grid = std::max(1, std::min((a.nwarps + 3) / 4, std::max(1, per_sm) * ctx->sm_count));
+    if (npart) grid = std::min(grid, ctx->n_partials);
+    {
+        Launch L(ctx, kclass);
+        kern<<<grid, 128, smem, ctx->stream>>>(a);
+    }
+    check_launch();
+    if (npart) *npart = grid;
+    return true;
+}
+
+template <class T, bool JACOBI>
+bool rep_launch(mgldg_ctx* ctx, const RepTable* t, RepArgs<T>& a, bool f16, int kclass, int* npart) {
+    const int E = std::is_same<T, float>::value ? t->gs / 16 : 1;
+    a.nwarps = t->b == 16 ? t->nslots / (16 * E) : t->nslots / 32;
+    const size_t smem = (size_t)a.nimg * sizeof(T) *
+                        (t->b == 16 ? Img<T, 16>::SIZE : (t->b == 9 ? Img<T, 9>::SIZE : Img<T, 4>::SIZE));
+    if (t->b == 4) return rep_launch_k(ctx, k_repc<T, 4, JACOBI>, a, smem, kclass, npart);
+    if (t->b == 9) return rep_launch_k(ctx, k_repc<T, 9, JACOBI>, a, smem, kclass, npart);
+    if constexpr (std::is_same<T, float>::value) {
+        if (f16) {
+            if (E == 4) return rep_launch_k(ctx, k_rep16<float, 4, JACOBI, true>, a, smem, kclass, npart);
+            if (E == 2) return rep_launch_k(ctx, k_rep16<float, 2, JACOBI, true>, a, smem, kclass, npart);
+            return rep_launch_k(ctx, k_rep16<float, 1, JACOBI, true>, a, smem, kclass, npart);
+        }
+        if (E == 4) return rep_launch_k(ctx, k_rep16<float, 4, JACOBI, false>, a, smem, kclass, npart);
+        if (E == 2) return rep_launch_k(ctx, k_rep16<float, 2, JACOBI, false>, a, smem, kclass, npart);
+        return rep_launch_k(ctx, k_rep16<float, 1, JACOBI, false>, a, smem, kclass, npart);
+    } else {
+        return rep_launch_k(ctx, k_rep16<double, 1, JACOBI, false>, a, smem, kclass, npart);
+    }
+}
+
+}  // namespace
+
+static bool rep_used(const RepTable* t) { return t && t->nslots; }
+
+template <class T>
+bool rep_spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const T* yin, T* y, const T* dotv,
+              double* partials, int* npart, int kclass, bool f16) {
+    const RepTable* t = A->rep;
+    if (!rep_used(t)) return false;
+    // 16 x 16: whole 16-byte words of every vector (the general kernels read
+    // only x that way)
+    if (t->b == 16 && ((uintptr_t)x | (uintptr_t)(beta != T(0) ? yin : nullptr) | (uintptr_t)y | (uintptr_t)dotv) % 16)
+        return false;
+    f16 = f16 && t->b == 16;   // smaller blocks keep FP32 in the F16 form
+    RepArgs<T> a = rep_args<T>(t, f16);
+    a.x = x;
+    a.b = yin;
+    a.y = y;
+    a.alpha = alpha;
+    a.beta = beta;
+    a.self_dot = (dotv != nullptr && dotv == y) ? 1 : 0;
+    a.dotv = a.self_dot ? nullptr : dotv;
+    a.partials = partials;
+    return rep_launch<T, false>(ctx, t, a, f16, kclass, npart);
+}
+template bool rep_spmv<float>(mgldg_ctx*, const mgldg_bsr*, float, const float*, float, const float*, float*,
+                              const float*, double*, int*, int, bool);
+template bool rep_spmv<double>(mgldg_ctx*, const mgldg_bsr*, double, const double*, double, const double*, double*,
+                               const double*, double*, int*, int, bool);
+
+template <class T>
+bool rep_jacobi(mgldg_ctx* ctx, const mgldg_bsr* A, const T* b, const T* xin, T* xout, T omega, bool xzero, bool f16) {
+    const RepTable* t = A->rep;
+    if (!rep_used(t)) return false;
+    f16 = f16 && t->b == 16;   // smaller blocks keep FP32 in the F16 form
+    RepArgs<T> a = rep_args<T>(t, f16);
+    a.x = xin;
+    a.b = b;
+    a.y = xout;
+    a.omega = omega;
+    a.xzero = xzero ? 1 : 0;
+    return rep_launch<T, true>(ctx, t, a, f16, MGLDG_K_JACOBI, nullptr);
+}
+template bool rep_jacobi<float>(mgldg_ctx*, const mgldg_bsr*, const float*, const float*, float*, float, bool, bool);
+template bool rep_jacobi<double>(mgldg_ctx*, const mgldg_bsr*, const double*, const double*, double*, double, bool,
+                                 bool);
+
+bool rep_df64(mgldg_ctx* ctx, const mgldg_bsr* A, const float* dhi, const float* dlo, const double* d, double* q,
+              double* partials, int* npart) {
+    const RepTable* t = A->rep;
+    if (!rep_used(t)) return false;
+    RepDfArgs a{};
+    a.nwarps = t->nslots / (t->b == 16 ? 16 : 32);
+    a.nslots = t->nslots;
+    a.nuniq = t->nuniq;
+    a.gcls = t->gcls;
+    a.rows = t->rows;
+    a.cols = t->cols;
+    a.cls = t->cls;
+    a.mask = t->mask;
+    a.img = t->i32;
+    a.imglo = t->ilo;
+    a.xh = dhi;
+    a.xl = dlo;
+    a.d = d;
+    a.q = q;
+    a.partials = partials;
+    const size_t s = 2 * sizeof(float) * t->nuniq;
+    if (t->b == 4) return rep_launch_k(ctx, k_repc_df64<4>, a, s * Img<float, 4>::SIZE, MGLDG_K_SPMV, npart);
+    if (t->b == 9) return rep_launch_k(ctx, k_repc_df64<9>, a, s * Img<float, 9>::SIZE, MGLDG_K_SPMV, npart);
+    return rep_launch_k(ctx, k_rep16_df64, a, s * Img<float, 16>::SIZE, MGLDG_K_SPMV, npart);
+}
+
+}  // namespace mg

@@ -1,0 +1,73 @@
+// repeat.cuh -- level operators with few distinct blocks (repeat.cu).
+#pragma once
+
+#include "internal.cuh"
+
+namespace mg {
+
+// Table form of a square block-sparse operator whose blocks repeat (grids
+// with constant coefficients: 17 distinct blocks on every uniform level).
+// A stored block k is table entry blk[k]; rows with the same sequence of
+// table entries form a class, and the slots list the rows class by class, gs
+// to a group, so that a warp applies one block to many rows at once.
+//
+// Images: the value tables as the kernels hold them in shared memory, first
+// the nuniq blocks (by rows, or by columns where fewer columns than rows hold
+// nonzeros), then the ndiag distinct inverse diagonal blocks (by rows); a
+// block is b lines of ld values, for b = 16 with 16 bytes between lines 7 and
+// 8 (the two column halves of a line pair then lie in different banks).
+struct RepView {
+    int b = 0, ld = 0, nbr = 0, nuniq = 0, ndiag = 0, ncls = 0;
+    int gs = 16;                   // slots per group, every group one class
+    int nslots = 0;                // 0: too many classes for the slot kernels
+    int* blk = nullptr;            // [nnzb] table entry of every stored block
+    unsigned* mask = nullptr;      // [nuniq] nonzero rows | nonzero columns << 16
+    int* cls = nullptr;            // [ncls][kRepCls]: blocks per row, inverse diagonal block, -, -, entries
+    int* gcls = nullptr;           // [nslots / 16] class of 16 consecutive slots
+    int* rows = nullptr;           // [nslots] row, -1: padding
+    int* cols = nullptr;           // [most blocks per row][nslots] block columns
+    double* i64 = nullptr;         // FP64 image
+    float *i32 = nullptr, *ilo = nullptr;   // FP32 image and the blocks' low halves (val = i32 + ilo)
+    float *i16 = nullptr, *s16 = nullptr;   // block-scaled FP16 values (all by rows), their scales
+};
+struct RepTable : RepView {
+    void* pool = nullptr;          // owns the value tables and mask
+    void* slots = nullptr;         // owns cls, gcls, rows, cols
+    RepTable() = default;
+    RepTable(const RepTable&) = delete;
+    RepTable& operator=(const RepTable&) = delete;
+    ~RepTable();
+};
+constexpr int kRepMaxNb = 12;            // longest row
+constexpr int kRepCls = kRepMaxNb + 4;   // ints per class
+
+// Looks for repeated blocks in A (square blocks of 4, 9 or 16) in two steps, so that the first one's result travels with a
+// synchronisation of the caller: rep_probe queues the block hashing,
+// rep_finish reads its result, checks every block against its table entry and
+// attaches the table to A (or leaves A as it is).  Dinv: A's inverse diagonal
+// blocks.
+struct RepProbe {
+    void* mem = nullptr;
+    int nslot = 0;
+    int head[2] = {0, 0};   // distinct blocks (host copy), overflow
+    RepProbe() = default;
+    RepProbe(const RepProbe&) = delete;
+    RepProbe& operator=(const RepProbe&) = delete;
+    ~RepProbe();
+};
+bool rep_probe(mgldg_ctx* ctx, const mgldg_bsr* A, RepProbe& p);
+void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p);
+
+// y = alpha A x + beta yin with the dot epilogue of spmv; false: no table
+template <class T>
+bool rep_spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const T* yin, T* y, const T* dotv,
+              double* partials, int* npart, int kclass, bool f16 = false);
+// damped block-Jacobi sweep (xzero: x = 0, not read); false: no table
+template <class T>
+bool rep_jacobi(mgldg_ctx* ctx, const mgldg_bsr* A, const T* b, const T* xin, T* xout, T omega, bool xzero,
+                bool f16 = false);
+// q = A d in double-float arithmetic and the partial sums of d.q
+bool rep_df64(mgldg_ctx* ctx, const mgldg_bsr* A, const float* dhi, const float* dlo, const double* d, double* q,
+              double* partials, int* npart);
+
+}  // namespace mg

@@ -32,6 +32,22 @@ __device__ __forceinline__ void vfma(float& acc, const float4& a, const float4& 
     acc = fmaf(a.w, b.w, acc);
 }
 
+// One product a*d of float pairs added to the float pair (sh, sl): the exact
+// FP32 product of the high parts (its error recovered with an FMA) plus the
+// two cross terms, added with a two-sum (Dekker's and Knuth's error-free
+// transformations; explicitly rounded operations, a contraction would break
+// them).
+__device__ __forceinline__ void df_fma(float& sh, float& sl, float ah, float al, float dh, float dl) {
+    const float p = __fmul_rn(ah, dh);
+    const float pe = fmaf(ah, dh, -p);
+    const float t = fmaf(ah, dl, fmaf(al, dh, pe));
+    const float s = __fadd_rn(sh, p);
+    const float bb = __fsub_rn(s, sh);
+    const float e = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bb)), __fsub_rn(p, bb));
+    sh = s;
+    sl = __fadd_rn(sl, __fadd_rn(e, t));
+}
+
 // can this block shape use 128-bit loads for every lane chunk?
 template <class T, int BR, int BC>
 struct RowVec {

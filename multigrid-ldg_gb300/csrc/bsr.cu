@@ -21,6 +21,7 @@
 #include "master_tables.inc"
 #include "repeat.cuh"
 #include "rowdot.cuh"
+#include "rowsplit.cuh"
 
 using namespace mg;
 
@@ -508,6 +509,11 @@ void spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const
             if (npart) *npart = 0;
             return;
         }
+    }
+    // few long block rows: blocks of a row dealt to several lane groups
+    if (!A->blk && !dotv && !partials && split_spmv<T>(ctx, A, bsr_vals<T>(A), alpha, x, beta, yin, y, kclass)) {
+        if (npart) *npart = 0;
+        return;
     }
     // operators stored as a small block table (interpolation on quadtrees)
     if (A->blk && !dotv && !partials && A->nuniq <= 16) {

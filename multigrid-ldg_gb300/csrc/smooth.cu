@@ -25,6 +25,7 @@
 
 #include "api.cuh"
 #include "rowdot.cuh"
+#include "rowsplit.cuh"
 #include "smooth.cuh"
 
 using namespace mg;
@@ -785,6 +786,7 @@ void jacobi_sweep(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, const T* Di
     if constexpr (std::is_same<T, float>::value) {
         if (bulk_jacobi_f32(ctx, A, vals, Dinv, b, xin, xout, omega, xzero)) return;
     }
+    if (split_jacobi(ctx, A, vals, Dinv, b, xin, xout, omega, xzero)) return;
     if (!A->blk) switch (A->br) {
             case 3: launch_jacobi_rows<T, 3>(ctx, A, vals, Dinv, b, xin, xout, omega, xzero); return;
             case 4: launch_jacobi_rows<T, 4>(ctx, A, vals, Dinv, b, xin, xout, omega, xzero); return;

@@ -243,6 +243,25 @@ __global__ void __launch_bounds__(256) k_out_dot(int64_t n, const T* __restrict_
     }
 }
 
+// the partial sums alone (the PCG reads the V-cycle's output where it is)
+template <class T>
+__global__ void __launch_bounds__(256) k_out_part(int64_t n, const T* __restrict__ xl, const double* __restrict__ b,
+                                                  double* __restrict__ partials) {
+    __shared__ double sm[8];
+    double acc = 0;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
+        acc += b[i] * widen(xl[i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        for (int w = 0; w < 8; ++w) t += sm[w];
+        partials[blockIdx.x] = t;
+    }
+}
+
 template <class T>
 static void out_dot(mgldg_ctx* ctx, int64_t n, const T* xl, const double* b, double* s, double* partials) {
     const int g = reduce_grid((int)std::min<int64_t>(n, 1 << 30));
@@ -328,20 +347,15 @@ __global__ void k_pcg_alpha(PcgScalars* sc, const double* partials, int np) {
     }
 }
 
-// it < 0: the iteration index is the device-side counter
-__global__ void k_pcg_rr(PcgScalars* sc, const double* partials, int np, double* hist, int it) {
+// ||r|| into the history at the device-side iteration index, then
+// delta_new = r.z and beta
+__global__ void k_pcg_beta(PcgScalars* sc, const double* prr, int nrr, const double* prz, int nrz, double* hist) {
     __shared__ double sm[32];
-    double rr = block_total(partials, np, sm);
+    const double rr = block_total(prr, nrr, sm);
+    const double rs = block_total(prz, nrz, sm);
     if (threadIdx.x == 0) {
         sc->rr = rr;
-        hist[it >= 0 ? it : sc->it] = sqrt(rr);
-    }
-}
-
-__global__ void k_pcg_beta(PcgScalars* sc, const double* partials, int np) {
-    __shared__ double sm[32];
-    double rs = block_total(partials, np, sm);
-    if (threadIdx.x == 0) {
+        hist[sc->it] = sqrt(rr);
         sc->delta_old = sc->delta_new;
         sc->delta_new = rs;
         double b = rs / sc->delta_old;
@@ -364,40 +378,105 @@ __global__ void k_pcg_cond(const PcgScalars* sc, double tol2, int maxit, cudaGra
     cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
-// x += alpha d ; (r -= alpha q) ; partial r.r
-__global__ void __launch_bounds__(256) k_pcg_update(int64_t n, const PcgScalars* sc, const double* __restrict__ d,
-                                                    const double* __restrict__ q, double* __restrict__ x,
-                                                    double* __restrict__ r, int update_r, double* partials) {
+// The CG's vector work of one iteration, in three passes over the vectors (of
+// 4.2 million entries a pass is 17-30 us of HBM time; the split into update,
+// copy into the V-cycle, copy out of it and direction moved 470 MB per
+// iteration, these 350 MB):
+//   k_pcg_update  r -= alpha q, the V-cycle's FP32 right-hand side, partial r.r
+//   k_out_part    partial r.z with z read where the V-cycle left it
+//   k_pcg_dir     x += alpha d, d = z + beta d (and d's float pair)
+// x is updated last because its old direction d is read there anyway.
+
+// x += alpha d (residual-replacement iterations update x before r = b - A x)
+__global__ void __launch_bounds__(256) k_pcg_xupdate(int64_t n, const PcgScalars* sc, const double* __restrict__ d,
+                                                     double* __restrict__ x) {
+    const double alpha = sc->alpha;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
+        x[i] += alpha * d[i];
+}
+
+// r -= alpha q ; b32 = (float) r when given ; partial r.r.  Two entries per
+// thread and round (r, q and b32 are the library's own, 16-byte aligned).
+__global__ void __launch_bounds__(256) k_pcg_update(int64_t n, const PcgScalars* sc, const double* __restrict__ q,
+                                                    double* __restrict__ r, float* __restrict__ b32,
+                                                    double* partials) {
     __shared__ double sm[8];
     const double alpha = sc->alpha;
     double s = 0;
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
-        x[i] += alpha * d[i];
-        if (update_r) {
-            double v = r[i] - alpha * q[i];
-            r[i] = v;
-            s += v * v;
-        }
+    const int64_t n2 = n / 2;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n2; i += (int64_t)gridDim.x * 256) {
+        const double2 rv = reinterpret_cast<const double2*>(r)[i], qv = reinterpret_cast<const double2*>(q)[i];
+        const double v0 = rv.x - alpha * qv.x, v1 = rv.y - alpha * qv.y;
+        reinterpret_cast<double2*>(r)[i] = make_double2(v0, v1);
+        if (b32) reinterpret_cast<float2*>(b32)[i] = make_float2(narrow(v0), narrow(v1));
+        s += v0 * v0;
+        s += v1 * v1;
     }
-    if (update_r) {
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        const double v = r[n - 1] - alpha * q[n - 1];
+        r[n - 1] = v;
+        if (b32) b32[n - 1] = narrow(v);
+        s += v * v;
+    }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0;
-            for (int w = 0; w < 8; ++w) t += sm[w];
-            partials[blockIdx.x] = t;
-        }
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        for (int w = 0; w < 8; ++w) t += sm[w];
+        partials[blockIdx.x] = t;
     }
 }
 
-// d = s + beta d
-__global__ void __launch_bounds__(256) k_pcg_dir(int64_t n, const PcgScalars* sc, const double* __restrict__ s,
-                                                 double* __restrict__ d) {
-    const double beta = sc->beta;
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256)
-        d[i] = s[i] + beta * d[i];
+__device__ __forceinline__ double2 ld2(const double* p, int64_t i) { return reinterpret_cast<const double2*>(p)[i]; }
+__device__ __forceinline__ double2 ld2(const float* p, int64_t i) {
+    const float2 v = reinterpret_cast<const float2*>(p)[i];
+    return make_double2(widen(v.x), widen(v.y));
+}
+
+// (x += alpha d when xupd) ; d = z + beta d ; d's float pair when hi is given.
+// Two entries per thread and round; the caller's x may be 8-byte aligned only
+// (xvec = 0: its entries are read one by one).
+template <class T>
+__global__ void __launch_bounds__(256) k_pcg_dir(int64_t n, const PcgScalars* sc, const T* __restrict__ z,
+                                                 double* __restrict__ d, double* __restrict__ x, int xupd, int xvec,
+                                                 float* __restrict__ hi, float* __restrict__ lo) {
+    const double beta = sc->beta, alpha = sc->alpha;
+    const int64_t n2 = n / 2;
+    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n2; i += (int64_t)gridDim.x * 256) {
+        const double2 dv = ld2(d, i), zv = ld2(z, i);
+        if (xupd) {
+            double2 xv;
+            if (xvec) xv = ld2(x, i);
+            else xv = make_double2(x[2 * i], x[2 * i + 1]);
+            xv.x += alpha * dv.x;
+            xv.y += alpha * dv.y;
+            if (xvec) {
+                reinterpret_cast<double2*>(x)[i] = xv;
+            } else {
+                x[2 * i] = xv.x;
+                x[2 * i + 1] = xv.y;
+            }
+        }
+        const double v0 = zv.x + beta * dv.x, v1 = zv.y + beta * dv.y;
+        reinterpret_cast<double2*>(d)[i] = make_double2(v0, v1);
+        if (hi) {
+            float2 h, l;
+            split_pair(v0, h.x, l.x);
+            split_pair(v1, h.y, l.y);
+            reinterpret_cast<float2*>(hi)[i] = h;
+            reinterpret_cast<float2*>(lo)[i] = l;
+        }
+    }
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
+        const int64_t i = n - 1;
+        const double dv = d[i];
+        if (xupd) x[i] += alpha * dv;
+        const double v = (double)z[i] + beta * dv;
+        d[i] = v;
+        if (hi) split_pair(v, hi[i], lo[i]);
+    }
 }
 
 // ------------------------------------------------- double-float outer product --
@@ -528,20 +607,6 @@ __global__ void __launch_bounds__(256) k_split(int64_t n, const double* __restri
     }
 }
 
-// d = s + beta d, and its float pair
-__global__ void __launch_bounds__(256) k_pcg_dir_split(int64_t n, const PcgScalars* sc, const double* __restrict__ s,
-                                                       double* __restrict__ d, float* __restrict__ hi,
-                                                       float* __restrict__ lo) {
-    const double beta = sc->beta;
-    for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
-        const double v = s[i] + beta * d[i];
-        d[i] = v;
-        const float h = (float)v;
-        hi[i] = h;
-        lo[i] = (float)(v - (double)h);
-    }
-}
-
 static bool df64_shape(int b) { return b == 3 || b == 4 || b == 6 || b == 8 || b == 9 || b == 10 || b == 16; }
 
 static bool df64_ok(const mgldg_mg* m, const mgldg_bsr* A) {
@@ -600,9 +665,9 @@ static void drop_pcg_graph(mgldg_mg* m) {
 static void ensure_pcg(mgldg_mg* m, mgldg_ctx* ctx, int64_t n, int maxit) {
     if (m->pcg_n != n || m->pcg_maxit < maxit) drop_pcg_graph(m);
     if (m->pcg_n != n) {
-        dfree(m->r); dfree(m->d); dfree(m->q); dfree(m->s); dfree(m->dhi); dfree(m->dlo);
+        dfree(m->r); dfree(m->d); dfree(m->q); dfree(m->dhi); dfree(m->dlo);
         m->dhi = m->dlo = nullptr;
-        m->r = dalloc<double>(n); m->d = dalloc<double>(n); m->q = dalloc<double>(n); m->s = dalloc<double>(n);
+        m->r = dalloc<double>(n); m->d = dalloc<double>(n); m->q = dalloc<double>(n);
         if (m->p.precision != MGLDG_PREC_FP64) {
             m->dhi = dalloc<float>(n);
             m->dlo = dalloc<float>(n);
@@ -695,16 +760,54 @@ void mg_precon_eager(mgldg_mg* m, const double* r, double* s) {
 }
 void mg_take_errors(mgldg_mg* m) { take_errors(m); }
 
+// z = V-cycle(r) from x = 0 for the CG, without copies of the FP64 vectors:
+// in the mixed forms the level's FP32 right-hand side has been written by the
+// caller, in FP64 the level reads r itself (unless the one-level hierarchy
+// projects its right-hand side in place); the result stays in the level's x.
+// partial r.z goes to part (grid CTAs).
+static void cg_precon(mgldg_mg* m, double* r, double* part, int grid) {
+    mgldg_ctx* ctx = m->ctx;
+    LevelData& L = m->L[0];
+    struct LevelReset {
+        mgldg_ctx* c;
+        ~LevelReset() { c->cur_level = -1; }
+    } reset{ctx};
+    const bool z = zero_start(m, 0);
+    if (m->p.precision != MGLDG_PREC_FP64) {
+        if (!z) MG_CHECK_CUDA(cudaMemsetAsync(L.x32, 0, L.n * sizeof(float), ctx->stream));
+        vcycle<float>(m, 0, z);
+        Launch K(ctx, MGLDG_K_VECTOR);
+        k_out_part<float><<<grid, 256, 0, ctx->stream>>>(L.n, L.x32, r, part);
+    } else {
+        if (!z) MG_CHECK_CUDA(cudaMemsetAsync(L.x, 0, L.n * sizeof(double), ctx->stream));
+        if (m->L.size() == 1 && m->p.mean_project) {
+            MG_CHECK_CUDA(cudaMemcpyAsync(L.bb, r, L.n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+            vcycle<double>(m, 0, z);
+        } else {
+            struct Borrow {
+                double *&p, *own;
+                ~Borrow() { p = own; }
+            } borrow{L.bb, L.bb};
+            L.bb = r;
+            vcycle<double>(m, 0, z);
+        }
+        Launch K(ctx, MGLDG_K_VECTOR);
+        k_out_part<double><<<grid, 256, 0, ctx->stream>>>(L.n, L.x, r, part);
+    }
+    check_launch();
+}
+
 // One PCG iteration (krylov.h:43-61) on the context's stream: q = A d,
-// alpha, x += alpha d with r -= alpha q (or, when `replace`, r = b - A x),
-// ||r|| into the history at the device-side iteration index, s = M(r),
-// delta_new = r.s, beta (which advances the iteration counter), d = s + beta d.
-// `eager`: the preconditioner's launches are issued directly (inside a graph
-// capture) instead of replaying its own graph.
+// alpha, r -= alpha q (or, when `replace`, x += alpha d and r = b - A x),
+// s = M(r), ||r|| into the history at the device-side iteration index,
+// delta_new = r.s, beta (which advances the iteration counter), x += alpha d,
+// d = s + beta d.
 static void pcg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const double* b, double* x, int64_t n,
-                          bool df, int grid_vec, bool replace, bool eager) {
+                          bool df, int grid_vec, bool replace) {
     double* part = ctx->d_partials;
-    int np = 0;
+    double* prr = part + ctx->n_partials / 2;   // r.r partials, read with r.z's
+    const bool mixed = m->p.precision != MGLDG_PREC_FP64;
+    int np = 0, nrr = grid_vec;
     // q = A d ; alpha = delta_new / d.q
     if (df) spmv_df64(ctx, A, m, part, &np);
     else outer_spmv(ctx, A, 1.0, m->d, 0.0, nullptr, m->q, m->d, part, &np);
@@ -713,46 +816,41 @@ static void pcg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const
         k_pcg_alpha<<<1, 256, 0, ctx->stream>>>(m->sc, part, np);
     }
     check_launch();
+    float* b32 = mixed && !m->L.empty() ? m->L[0].b32 : nullptr;
     if (replace) {
         // x += alpha d ; r = b - A x (residual replacement)
         {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_pcg_update<<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->d, m->q, x, m->r, 0, part);
+            k_pcg_xupdate<<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->d, x);
         }
         check_launch();
-        outer_spmv(ctx, A, -1.0, x, 1.0, b, m->r, m->r, part, &np);
+        outer_spmv(ctx, A, -1.0, x, 1.0, b, m->r, m->r, prr, &nrr);
+        if (b32) convert<double, float>(ctx, n, m->r, b32);
     } else {
         {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_pcg_update<<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->d, m->q, x, m->r, 1, part);
+            k_pcg_update<<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->q, m->r, b32, prr);
         }
         check_launch();
-        np = grid_vec;
     }
+    // s = M(r) ; delta_new = r.s ; beta ; x += alpha d ; d = s + beta d
+    np = grid_vec;
+    if (m->L.empty()) dot_partials<double>(ctx, (int)n, m->r, m->r, part, &np);
+    else cg_precon(m, m->r, part, grid_vec);
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_pcg_rr<<<1, 256, 0, ctx->stream>>>(m->sc, part, np, m->hist, -1);
-    }
-    check_launch();
-    // s = M(r) ; delta_new = r.s (summed by the V-cycle's output kernel) ;
-    // beta ; d = s + beta d
-    if (m->L.empty()) {
-        precon(m, m->r, m->s);
-        dot_partials<double>(ctx, (int)n, m->r, m->s, part, &np);
-    } else {
-        if (eager) vcycle_dev(m, m->r, m->s, true, part);
-        else precon(m, m->r, m->s, part);
-        np = reduce_grid((int)std::min<int64_t>(n, 1 << 30));
-    }
-    {
-        Launch L(ctx, MGLDG_K_VECTOR);
-        k_pcg_beta<<<1, 256, 0, ctx->stream>>>(m->sc, part, np);
+        k_pcg_beta<<<1, 256, 0, ctx->stream>>>(m->sc, prr, nrr, part, np, m->hist);
     }
     check_launch();
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        if (df) k_pcg_dir_split<<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->s, m->d, m->dhi, m->dlo);
-        else k_pcg_dir<<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->s, m->d);
+        const int xupd = replace ? 0 : 1, xvec = (uintptr_t)x % 16 == 0;
+        float *hi = df ? m->dhi : nullptr, *lo = df ? m->dlo : nullptr;
+        if (b32)
+            k_pcg_dir<float><<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->L[0].x32, m->d, x, xupd, xvec, hi, lo);
+        else
+            k_pcg_dir<double><<<grid_vec, 256, 0, ctx->stream>>>(n, m->sc, m->L.empty() ? m->r : m->L[0].x, m->d, x,
+                                                                 xupd, xvec, hi, lo);
     }
     check_launch();
 }
@@ -778,7 +876,7 @@ static bool build_pcg_graph(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, con
     }
     cudaGraph_t body = nullptr;
     try {
-        pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, true, true);
+        pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, true);
         for (int k = 0; k < MGLDG_K_NCLASS; ++k) G.pro_launches[k] = ctx->launches[k] - before[k];
         cudaStreamCaptureStatus st;
         cudaGraph_t cg = nullptr;
@@ -808,7 +906,7 @@ static bool build_pcg_graph(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, con
             std::memcpy(b2, ctx->launches, sizeof b2);
             MG_CHECK_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0,
                                                         cudaStreamCaptureModeThreadLocal));
-            pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, false, true);
+            pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, false);
             k_pcg_cond<<<1, 1, 0, ctx->stream>>>(m->sc, tol2, maxit, h);
             check_launch();
             cudaGraph_t bg = nullptr;
@@ -901,7 +999,7 @@ static void pcg_dev(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const doubl
                 continue;
             }
         }
-        pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, i % 50 == 0, false);
+        pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, i % 50 == 0);
         MG_CHECK_CUDA(cudaMemcpyAsync(m->h_sc, m->sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, ctx->stream));
         sync(ctx);
         ++i;
@@ -933,7 +1031,7 @@ mgldg_mg::~mgldg_mg() {
         delete L.Tt;
     }
     dfree(Cinv);
-    dfree(r); dfree(d); dfree(q); dfree(s); dfree(hist); dfree(dhi); dfree(dlo);
+    dfree(r); dfree(d); dfree(q); dfree(hist); dfree(dhi); dfree(dlo);
     dfree(host_b); dfree(host_x);
     dfree(tail_count);
     dfree(sc);
@@ -1268,7 +1366,7 @@ extern "C" int mgldg_pcg(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const 
 // The existing entry point allocates four work vectors, a history buffer and
 // pinned scalars on every call; this one uses the fixed scratch array below
 // instead and calls no allocating routine (with kernel profiling off, the
-// default).  The array is carved into r, d, q, s (kCgMaxN doubles each), the
+// default).  The array is carved into r, d, q (kCgMaxN doubles each, and as many spare), the
 // reduction partials, the residual history and the scalar block.
 namespace {
 constexpr int64_t kCgMaxN = 131072;    // largest system: 131,072 unknowns
@@ -1322,8 +1420,8 @@ extern "C" int mgldg_cg_noalloc_dev(mgldg_ctx* ctx, const mgldg_bsr* A, const do
     double* r = base;
     double* d = base + kCgMaxN;
     double* q = base + 2 * kCgMaxN;
-    double* s = base + 3 * kCgMaxN;
     double* part = base + 4 * kCgMaxN;
+    double* prr = part + kCgParts / 2;   // r.r partials (every grid has at most kCgParts / 2 CTAs)
     double* hist = part + kCgParts;
     PcgScalars* sc = reinterpret_cast<PcgScalars*>(base + kCgScalarOff);
     // the scratch keeps the previous call's contents: start the scalars at zero
@@ -1355,36 +1453,33 @@ extern "C" int mgldg_cg_noalloc_dev(mgldg_ctx* ctx, const mgldg_bsr* A, const do
             k_pcg_alpha<<<1, 256, 0, ctx->stream>>>(sc, part, np);
         }
         check_launch();
-        if (i % 50 == 0) {
+        const bool replace = i % 50 == 0;
+        int nrr = grid_vec;
+        if (replace) {
             {
                 Launch L(ctx, MGLDG_K_VECTOR);
-                k_pcg_update<<<grid_vec, 256, 0, ctx->stream>>>(n, sc, d, q, x, r, 0, part);
+                k_pcg_xupdate<<<grid_vec, 256, 0, ctx->stream>>>(n, sc, d, x);
             }
             check_launch();
-            spmv<double>(ctx, A, -1.0, x, 1.0, b, r, r, part, &np);
+            spmv<double>(ctx, A, -1.0, x, 1.0, b, r, r, prr, &nrr);
         } else {
             {
                 Launch L(ctx, MGLDG_K_VECTOR);
-                k_pcg_update<<<grid_vec, 256, 0, ctx->stream>>>(n, sc, d, q, x, r, 1, part);
+                k_pcg_update<<<grid_vec, 256, 0, ctx->stream>>>(n, sc, q, r, nullptr, prr);
             }
             check_launch();
-            np = grid_vec;
         }
+        // identity preconditioner: s = r
+        dot_partials<double>(ctx, (int)n, r, r, part, &np);
         {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_pcg_rr<<<1, 256, 0, ctx->stream>>>(sc, part, np, hist, i);
-        }
-        check_launch();
-        MG_CHECK_CUDA(cudaMemcpyAsync(s, r, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-        dot_partials<double>(ctx, (int)n, r, s, part, &np);
-        {
-            Launch L(ctx, MGLDG_K_VECTOR);
-            k_pcg_beta<<<1, 256, 0, ctx->stream>>>(sc, part, np);
+            k_pcg_beta<<<1, 256, 0, ctx->stream>>>(sc, prr, nrr, part, np, hist);
         }
         check_launch();
         {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_pcg_dir<<<grid_vec, 256, 0, ctx->stream>>>(n, sc, s, d);
+            k_pcg_dir<double><<<grid_vec, 256, 0, ctx->stream>>>(n, sc, r, d, x, replace ? 0 : 1,
+                                                                  (uintptr_t)x % 16 == 0, nullptr, nullptr);
         }
         check_launch();
         MG_CHECK_CUDA(cudaMemcpyAsync(&h, sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, ctx->stream));

@@ -72,7 +72,7 @@ struct mgldg_mg {
     double* Cinv = nullptr;   // dense inverse of the coarsest matrix
     int nc = 0;
     // pcg work space
-    double *r = nullptr, *d = nullptr, *q = nullptr, *s = nullptr, *hist = nullptr;
+    double *r = nullptr, *d = nullptr, *q = nullptr, *hist = nullptr;
     float *dhi = nullptr, *dlo = nullptr;   // d as a float pair (mixed forms, double-float q = A d)
     int64_t pcg_n = 0;
     int pcg_maxit = 0;

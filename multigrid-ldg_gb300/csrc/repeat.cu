@@ -17,8 +17,7 @@
 // Mapping: the rows are sorted by class (same sequence of table entries) and
 // a warp's rows belong to one class, so a block value read once from shared
 // memory serves all of them.  16 x 16 blocks: two lanes per row, one per
-// column half, E = 1, 2 or 4 rows per lane pair; smaller blocks: one lane per
-// row.  The sums run in the general kernels' order (16 x 16: the two column
+// column half, E = 1 or 2 rows per lane pair; smaller blocks: one lane per row.  The sums run in the general kernels' order (16 x 16: the two column
 // halves in block order, then their sum; smaller blocks: one sum per column
 // over the blocks, then the columns), and a skipped product is one with a
 // zero block entry, so for finite vectors the results are the general
@@ -313,7 +312,7 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
     // whole groups.  Chunks of 4,096 consecutive rows keep a warp's gathers
     // within one stretch of the vectors; with many classes one chunk wastes
     // fewer slots. ----
-    const int gs = b != 16 ? 32 : (n >= 131072 ? 64 : (n >= 32768 ? 32 : 16));
+    const int gs = b != 16 || n >= 32768 ? 32 : 16;
     const int chunk = ncls <= 32 ? 4096 : n;
     std::vector<int> rows, gcls;
     {
@@ -373,6 +372,13 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
         else k_rep_tables<16><<<nu, 256, 0, ctx->stream>>>(A->val, dint, dint + nu, dint + 2 * nu, Dinv, v);
     }
     check_launch();
+    std::vector<unsigned> mask(nu);
+    download(ctx, mask.data(), t->mask, nu);
+    sync(ctx);
+    for (int c = 0; c < ncls; ++c) {
+        int* d = &cls[(size_t)c * kRepCls];
+        for (int q = 0; q < d[0]; ++q) d[4 + kRepMaxNb + q] = (int)mask[d[4 + q]];
+    }
     MG_CHECK_CUDA(cudaMemcpyAsync(t->blk, slot_of, (size_t)A->nnzb * sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
     if (nslots) {
         std::vector<int> cols((size_t)kRepMaxNb * nslots);
@@ -501,23 +507,49 @@ __device__ __forceinline__ void pair_sum(const T (&p)[16], int half, T (&s)[8]) 
     }
 }
 
-// p[e] += the lane's column half of (A x)_i for its E rows (slots slot + 16 e)
+// p[e] += the lane's column half of (A x)_i for its E rows (slots slot + 16 e).
+// The gathers of block k + 1 and the column indices of block k + 2 are in
+// flight while block k is applied (their latency, three loads in a row,
+// otherwise bounds the kernel: 65,536 rows, E = 2, 19.6 us at 73 % of the
+// warps' time in it).
 template <class T, int E, bool F16>
 __device__ __forceinline__ void acc16(const RepArgs<T>& a, const T* simg, const int* cls, int slot, int half,
                                       T (&p)[E][16]) {
     using I = Img<T, 16>;
     const int nb = __ldg(cls);
+    const int* cp = a.cols + slot;
+    const T* xh = a.x + 8 * half;
+    int col[E];
+    T xn[E][8];
+#pragma unroll
+    for (int e = 0; e < E; ++e) ldg<8>(xh + (size_t)__ldg(cp + 16 * e) * 16, xn[e]);
+#pragma unroll
+    for (int e = 0; e < E; ++e) col[e] = nb > 1 ? __ldg(cp + a.nslots + 16 * e) : 0;
     int id = __ldg(cls + 4);
+    unsigned m = (unsigned)__ldg(cls + 4 + kRepMaxNb);
 #pragma unroll 1
     for (int k = 0; k < nb; ++k) {
         T xv[E][8];
 #pragma unroll
         for (int e = 0; e < E; ++e)
-            ldg<8>(a.x + (size_t)__ldg(a.cols + (size_t)k * a.nslots + slot + 16 * e) * 16 + 8 * half, xv[e]);
-        const unsigned m = __ldg(a.mask + id), rm = m & 0xffffu, cm = m >> 16;
-        const T* ab = simg + id * I::SIZE;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) xv[e][c] = xn[e][c];
+        const int idk = id;
+        const unsigned rm = m & 0xffffu, cm = m >> 16;
+        if (k + 1 < nb) {
+#pragma unroll
+            for (int e = 0; e < E; ++e) ldg<8>(xh + (size_t)col[e] * 16, xn[e]);
+            id = __ldg(cls + 5 + k);
+            m = (unsigned)__ldg(cls + 5 + kRepMaxNb + k);
+        }
+        if (k + 2 < nb) {
+            const int* cq = cp + (size_t)(k + 2) * a.nslots;
+#pragma unroll
+            for (int e = 0; e < E; ++e) col[e] = __ldg(cq + 16 * e);
+        }
+        const T* ab = simg + idk * I::SIZE;
         if (F16 || __popc(rm) <= __popc(cm)) {
-            const T sc = F16 ? (T)__ldg(a.scale + id) : T(0);
+            const T sc = F16 ? (T)__ldg(a.scale + idk) : T(0);
 #pragma unroll
             for (int r = 0; r < 16; ++r)
                 if ((rm >> r) & 1u) {
@@ -550,7 +582,6 @@ __device__ __forceinline__ void acc16(const RepArgs<T>& a, const T* simg, const 
                         for (int r = 0; r < 16; ++r) p[e][r] = fma_(av[r], xv[e][c], p[e][r]);
                 }
         }
-        if (k + 1 < nb) id = __ldg(cls + 5 + k);
     }
 }
 
@@ -749,7 +780,11 @@ struct RepDfArgs {
 };
 
 // q = A d in double-float arithmetic, 16 x 16 blocks, two lanes per row: a
-// float-pair sum per row and column half, their FP64 sum, the partial d.q
+// float-pair sum per row and column half, the two pairs added with a two-sum,
+// q and the partial d.q in FP64.  Bound by the FP32 pipes (11 operations per
+// product; the zero block rows and columns are skipped), then by the FP64
+// ones: adding the halves as float pairs and widening without conversions
+// leaves two FP64 operations per entry instead of eight.
 __global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
     using I = Img<float, 16>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -763,18 +798,36 @@ __global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
         const int slot = w * 16 + (lane >> 1);
         const int* cls = a.cls + (size_t)__ldg(a.gcls + w) * kRepCls;
         const int nb = __ldg(cls);
-        float sh[16], sl[16];
+        const int* cp = a.cols + slot;
+        float sh[16], sl[16], nh[8], nl[8];
 #pragma unroll
         for (int r = 0; r < 16; ++r) sh[r] = sl[r] = 0.f;
+        {
+            const size_t xo = (size_t)__ldg(cp) * 16 + 8 * half;
+            ldg<8>(a.xh + xo, nh);
+            ldg<8>(a.xl + xo, nl);
+        }
+        int col = nb > 1 ? __ldg(cp + a.nslots) : 0;
+        int id = __ldg(cls + 4);
+        unsigned m = (unsigned)__ldg(cls + 4 + kRepMaxNb);
 #pragma unroll 1
         for (int k = 0; k < nb; ++k) {
-            const int id = __ldg(cls + 4 + k);
-            const unsigned m = __ldg(a.mask + id), rm = m & 0xffffu, cm = m >> 16;
-            const size_t xo = (size_t)__ldg(a.cols + (size_t)k * a.nslots + slot) * 16 + 8 * half;
             float xh[8], xl[8];
-            ldg<8>(a.xh + xo, xh);
-            ldg<8>(a.xl + xo, xl);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                xh[c] = nh[c];
+                xl[c] = nl[c];
+            }
+            const unsigned rm = m & 0xffffu, cm = m >> 16;
             const int bo = id * I::SIZE;
+            if (k + 1 < nb) {
+                const size_t xo = (size_t)col * 16 + 8 * half;
+                ldg<8>(a.xh + xo, nh);
+                ldg<8>(a.xl + xo, nl);
+                id = __ldg(cls + 5 + k);
+                m = (unsigned)__ldg(cls + 5 + kRepMaxNb + k);
+            }
+            if (k + 2 < nb) col = __ldg(cp + (size_t)(k + 2) * a.nslots);
             if (__popc(rm) <= __popc(cm)) {
 #pragma unroll
                 for (int r = 0; r < 16; ++r)
@@ -799,19 +852,22 @@ __global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
                     }
             }
         }
-        double v[16], qv[8];
-#pragma unroll
-        for (int r = 0; r < 16; ++r) v[r] = (double)sh[r] + (double)sl[r];
-        pair_sum(v, half, qv);
         const int row = __ldg(a.rows + slot);
-        if (row >= 0) {
-            const size_t o = (size_t)row * 16 + 8 * half;
-            double dv[8];
-            ldg<8>(a.d + o, dv);
-            st8(a.q + o, qv);
+        const size_t o = (size_t)max(row, 0) * 16 + 8 * half;
+        double dv[8], qv[8];
+        ldg<8>(a.d + o, dv);
 #pragma unroll
-            for (int r = 0; r < 8; ++r) dacc += qv[r] * dv[r];
+        for (int r = 0; r < 8; ++r) {
+            // the halves' pairs: two-sum of the high parts, the rest added
+            const float oh = __shfl_xor_sync(0xffffffffu, half ? sh[r] : sh[r + 8], 1);
+            const float ol = __shfl_xor_sync(0xffffffffu, half ? sl[r] : sl[r + 8], 1);
+            const float mh = half ? sh[r + 8] : sh[r], ml = half ? sl[r + 8] : sl[r];
+            const float s = __fadd_rn(mh, oh), bb = __fsub_rn(s, mh);
+            const float e = __fadd_rn(__fsub_rn(mh, __fsub_rn(s, bb)), __fsub_rn(oh, bb));
+            qv[r] = widen(s) + widen(__fadd_rn(e, __fadd_rn(ml, ol)));
+            if (row >= 0) dacc += qv[r] * dv[r];
         }
+        if (row >= 0) st8(a.q + o, qv);
     }
     rep_partial(dacc, a.partials);
 }
@@ -919,12 +975,12 @@ bool rep_launch(mgldg_ctx* ctx, const RepTable* t, RepArgs<T>& a, bool f16, int 
     if (t->b == 4) return rep_launch_k(ctx, k_repc<T, 4, JACOBI>, a, smem, kclass, npart);
     if (t->b == 9) return rep_launch_k(ctx, k_repc<T, 9, JACOBI>, a, smem, kclass, npart);
     if constexpr (std::is_same<T, float>::value) {
+        // two rows per lane pair from 32,768 rows on (four measured no better:
+        // 35.7 against 32.5 us per sweep of 262,144 rows)
         if (f16) {
-            if (E == 4) return rep_launch_k(ctx, k_rep16<float, 4, JACOBI, true>, a, smem, kclass, npart);
             if (E == 2) return rep_launch_k(ctx, k_rep16<float, 2, JACOBI, true>, a, smem, kclass, npart);
             return rep_launch_k(ctx, k_rep16<float, 1, JACOBI, true>, a, smem, kclass, npart);
         }
-        if (E == 4) return rep_launch_k(ctx, k_rep16<float, 4, JACOBI, false>, a, smem, kclass, npart);
         if (E == 2) return rep_launch_k(ctx, k_rep16<float, 2, JACOBI, false>, a, smem, kclass, npart);
         return rep_launch_k(ctx, k_rep16<float, 1, JACOBI, false>, a, smem, kclass, npart);
     } else {

@@ -22,7 +22,7 @@ struct RepView {
     int nslots = 0;                // 0: too many classes for the slot kernels
     int* blk = nullptr;            // [nnzb] table entry of every stored block
     unsigned* mask = nullptr;      // [nuniq] nonzero rows | nonzero columns << 16
-    int* cls = nullptr;            // [ncls][kRepCls]: blocks per row, inverse diagonal block, -, -, entries
+    int* cls = nullptr;            // [ncls][kRepCls]: blocks per row, inverse diagonal block, -, -, entries, their masks
     int* gcls = nullptr;           // [nslots / 16] class of 16 consecutive slots
     int* rows = nullptr;           // [nslots] row, -1: padding
     int* cols = nullptr;           // [most blocks per row][nslots] block columns
@@ -39,7 +39,7 @@ struct RepTable : RepView {
     ~RepTable();
 };
 constexpr int kRepMaxNb = 12;            // longest row
-constexpr int kRepCls = kRepMaxNb + 4;   // ints per class
+constexpr int kRepCls = 2 * kRepMaxNb + 4;   // ints per class
 
 // Looks for repeated blocks in A (square blocks of 4, 9 or 16) in two steps, so that the first one's result travels with a
 // synchronisation of the caller: rep_probe queues the block hashing,

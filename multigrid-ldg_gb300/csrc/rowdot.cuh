@@ -48,6 +48,49 @@ __device__ __forceinline__ void df_fma(float& sh, float& sl, float ah, float al,
     sl = __fadd_rn(sl, __fadd_rn(e, t));
 }
 
+// ---- FP32 <-> FP64 conversions on the integer pipes ----
+// GB300 converts two values per clock and SM (the FP64 pipes), which bounded
+// the vector kernels: the direction update of 4.2 million entries took 62 us
+// with five conversions and subtractions per entry, against 27 us of HBM
+// traffic.
+
+// (double)v: the exponent is rebiased and the mantissa shifted, exact for
+// every normal value and zero; others take the conversion
+__device__ __forceinline__ double widen(float v) {
+    const unsigned u = __float_as_uint(v), e = (u >> 23) & 0xffu;
+    const int hi = (int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20)));
+    if (e - 1u < 254u) return __hiloint2double(hi, (int)(u << 29));
+    return (u << 1) == 0u ? __hiloint2double((int)u, 0) : (double)v;
+}
+__device__ __forceinline__ double widen(double v) { return v; }
+
+// (float)v, rounded to nearest even; values outside FP32's normal range (and
+// non-finite ones) take the conversion
+__device__ __forceinline__ float narrow(double v) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v), mag = u & 0x7fffffffffffffffULL;
+    if ((unsigned)(mag >> 52) - 897u >= 253u) return (float)v;
+    const unsigned long long r = (mag + 0x0fffffffULL + ((mag >> 29) & 1u)) >> 29;
+    return __uint_as_float((unsigned)(r - (896ULL << 23)) | (unsigned)(u >> 32 & 0x80000000u));
+}
+
+// v = h + l: h the nearest FP32 value (ties away from zero), l the nearest to
+// the rest; the rest is an integer below 2^29 times a power of two, so it
+// needs no FP64 operation.  Magnitudes outside 2^-60 .. 2^100 are split with
+// conversions.
+__device__ __forceinline__ void split_pair(double v, float& h, float& l) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v), mag = u & 0x7fffffffffffffffULL;
+    const unsigned e = (unsigned)(mag >> 52), sign = (unsigned)(u >> 32) & 0x80000000u;
+    if (e - 963u < 160u) {
+        const unsigned long long r = (mag + (1ULL << 28)) & ~((1ULL << 29) - 1);
+        const int rest = (int)(long long)(mag - r);
+        h = __uint_as_float((unsigned)((r >> 29) - (896ULL << 23)) | sign);
+        l = __fmul_rn((float)rest, __uint_as_float(((e - 948u) << 23) | sign));
+    } else {
+        h = (float)v;
+        l = (float)(v - (double)h);
+    }
+}
+
 // can this block shape use 128-bit loads for every lane chunk?
 template <class T, int BR, int BC>
 struct RowVec {

@@ -23,6 +23,8 @@
 
 #include "api.cuh"
 #include "mg.cuh"
+#include "repeat.cuh"
+#include "rowdot.cuh"
 
 using namespace mg;
 
@@ -629,9 +631,12 @@ static TileCfg default_cfg(int k, size_t elem) {
 
 // -------------------------------------------------------- column reductions
 // partials[blockIdx.x * k + c] = sum over this CTA's rows of a[u,c] * b[u,c]
+__device__ __forceinline__ double as_double(double v) { return v; }
+__device__ __forceinline__ double as_double(float v) { return widen(v); }
+
 template <class T>
-__global__ void __launch_bounds__(256) k_coldot(int64_t n, int k, const T* __restrict__ a, const T* __restrict__ b,
-                                               double* __restrict__ partials) {
+__global__ void __launch_bounds__(256) k_coldot(int64_t n, int k, const double* __restrict__ a,
+                                               const T* __restrict__ b, double* __restrict__ partials) {
     __shared__ double sm[256];
     const int c0 = blockIdx.y * 256;
     const int kc = min(256, k - c0);
@@ -643,16 +648,16 @@ __global__ void __launch_bounds__(256) k_coldot(int64_t n, int k, const T* __res
         const int64_t step = (int64_t)gridDim.x * rp;
         int64_t u = (int64_t)blockIdx.x * rp + ro;
         for (; u + 3 * step < n; u += 4 * step) {
-            const double p0 = (double)a[u * k + col] * (double)b[u * k + col];
-            const double p1 = (double)a[(u + step) * k + col] * (double)b[(u + step) * k + col];
-            const double p2 = (double)a[(u + 2 * step) * k + col] * (double)b[(u + 2 * step) * k + col];
-            const double p3 = (double)a[(u + 3 * step) * k + col] * (double)b[(u + 3 * step) * k + col];
+            const double p0 = a[u * k + col] * as_double(b[u * k + col]);
+            const double p1 = a[(u + step) * k + col] * as_double(b[(u + step) * k + col]);
+            const double p2 = a[(u + 2 * step) * k + col] * as_double(b[(u + 2 * step) * k + col]);
+            const double p3 = a[(u + 3 * step) * k + col] * as_double(b[(u + 3 * step) * k + col]);
             s += p0;
             s += p1;
             s += p2;
             s += p3;
         }
-        for (; u < n; u += step) s += (double)a[u * k + col] * (double)b[u * k + col];
+        for (; u < n; u += step) s += a[u * k + col] * as_double(b[u * k + col]);
     }
     sm[threadIdx.x] = s;
     __syncthreads();
@@ -668,7 +673,7 @@ static int coldot_grid(mgldg_ctx* ctx, int64_t n) {
 }
 
 template <class T>
-static void coldot(mgldg_ctx* ctx, int64_t n, int k, const T* a, const T* b, double* partials, int* np) {
+static void coldot(mgldg_ctx* ctx, int64_t n, int k, const double* a, const T* b, double* partials, int* np) {
     const int g = coldot_grid(ctx, n);
     dim3 grid(g, (k + 255) / 256);
     {
@@ -718,121 +723,267 @@ __global__ void k_bpcg_count(int k, BatchScalars sc) {
     if (threadIdx.x < 2) sc.counter[threadIdx.x] = cnt[threadIdx.x];
 }
 
-__global__ void k_bpcg_alpha(int k, BatchScalars sc, const double* partials, int np) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= k) return;
-    double a = 0;
-    if (sc.active[c]) {
-        const double dq = col_total(partials, np, k, c);
-        a = sc.delta_new[c] / dq;
-        if (!(dq > 0.0) || !isfinite(a)) {
-            sc.broken[c] = 1;
-            sc.active[c] = 0;
-            a = 0;
+// The block CG's vector work in three passes, as in the single-vector CG
+// (mg.cu): k_bpcg_update, k_coldot on the V-cycle's own output, k_bpcg_dir.
+// A thread keeps one column and walks down the rows, four rows in flight, so
+// its column's scalars stay in registers (k_coldot's layout).
+template <class F>
+__device__ __forceinline__ void column_rows(int64_t n, int k, F&& f) {
+    const int c0 = blockIdx.y * 256;
+    const int kc = min(256, k - c0);
+    const int rp = max(1, 256 / kc);
+    const int col = c0 + threadIdx.x % kc, ro = threadIdx.x / kc;
+    if (ro < rp) f(col, (int64_t)blockIdx.x * rp + ro, (int64_t)gridDim.x * rp);
+}
+
+// x += alpha d on active columns (before a residual replacement)
+__global__ void __launch_bounds__(256) k_bpcg_xupdate(int64_t n, int k, BatchScalars sc, const double* __restrict__ d,
+                                                      double* __restrict__ x) {
+    column_rows(n, k, [&](int col, int64_t u, int64_t step) {
+        if (!sc.active[col]) return;
+        const double al = sc.alpha[col];
+        for (; u < n; u += step) x[u * k + col] += al * d[u * k + col];
+    });
+}
+
+// r -= alpha q on active columns, the V-cycle's FP32 right-hand side when
+// given, and the partial column sums of r o r (k_coldot's layout)
+__global__ void __launch_bounds__(256) k_bpcg_update(int64_t n, int k, BatchScalars sc, const double* __restrict__ q,
+                                                     double* __restrict__ r, float* __restrict__ b32,
+                                                     double* __restrict__ partials) {
+    __shared__ double sm[256];
+    double s = 0;
+    column_rows(n, k, [&](int col, int64_t u, int64_t step) {
+        const double al = sc.active[col] ? sc.alpha[col] : 0.0;
+        auto one = [&](int64_t i, double rv, double qv) {
+            const double v = al != 0.0 ? rv - al * qv : rv;
+            if (al != 0.0) r[i] = v;
+            if (b32) b32[i] = narrow(v);
+            return v * v;
+        };
+        for (; u + 3 * step < n; u += 4 * step) {
+            const int64_t i0 = u * k + col, i1 = (u + step) * k + col, i2 = (u + 2 * step) * k + col,
+                          i3 = (u + 3 * step) * k + col;
+            const double r0 = r[i0], r1 = r[i1], r2 = r[i2], r3 = r[i3];
+            const double q0 = q[i0], q1 = q[i1], q2 = q[i2], q3 = q[i3];
+            s += one(i0, r0, q0);
+            s += one(i1, r1, q1);
+            s += one(i2, r2, q2);
+            s += one(i3, r3, q3);
         }
-    }
-    sc.alpha[c] = a;
-}
-
-// x += alpha d ; r -= alpha q (update_r), active columns only
-__global__ void __launch_bounds__(256) k_bpcg_update(int64_t nk, int k, BatchScalars sc, const double* __restrict__ d,
-                                                     const double* __restrict__ q, double* __restrict__ x,
-                                                     double* __restrict__ r, int update_r) {
-    const int64_t stride = (int64_t)gridDim.x * 256;
-    const int dc = (int)(stride % k);
-    int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    int c = (int)(e % k);
-    for (; e < nk; e += stride, c = (c + dc >= k) ? c + dc - k : c + dc) {
-        if (!sc.active[c]) continue;
-        const double al = sc.alpha[c];
-        x[e] += al * d[e];
-        if (update_r) r[e] -= al * q[e];
+        for (; u < n; u += step) s += one(u * k + col, r[u * k + col], q[u * k + col]);
+    });
+    const int kc = min(256, k - (int)blockIdx.y * 256), rp = max(1, 256 / kc);
+    sm[threadIdx.x] = s;
+    __syncthreads();
+    if ((int)threadIdx.x < kc) {
+        double t = 0;
+        for (int p = 0; p < rp; ++p) t += sm[p * kc + threadIdx.x];
+        partials[(size_t)blockIdx.x * k + blockIdx.y * 256 + threadIdx.x] = t;
     }
 }
 
-// it < 0: the iteration index is the device-side counter[2]
-__global__ void k_bpcg_rr(int k, BatchScalars sc, const double* partials, int np, double* hist, int maxit, int it) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= k || !sc.active[c]) return;
-    hist[(size_t)c * maxit + (it >= 0 ? it : sc.counter[2])] = sqrt(col_total(partials, np, k, c));
-}
-
-__global__ void k_bpcg_beta(int k, BatchScalars sc, const double* partials, int np) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= k) return;
-    double b = 0;
-    if (sc.active[c]) {
-        const double rs = col_total(partials, np, k, c);
-        sc.delta_old[c] = sc.delta_new[c];
-        sc.delta_new[c] = rs;
-        b = rs / sc.delta_old[c];
-        if (!isfinite(b) || rs < 0.0) {   // r.z < 0: preconditioner not positive definite
-            sc.broken[c] = 1;
-            sc.active[c] = 0;
-            b = 0;
+// x += alpha d where the column took a step and xupd, d = z + beta d on active
+// columns, d's float pair when hi is given
+template <class T>
+__global__ void __launch_bounds__(256) k_bpcg_dir(int64_t n, int k, BatchScalars sc, const T* __restrict__ z,
+                                                  double* __restrict__ d, double* __restrict__ x, int xupd,
+                                                  float* __restrict__ hi, float* __restrict__ lo) {
+    column_rows(n, k, [&](int col, int64_t u, int64_t step) {
+        const double al = xupd ? sc.alpha[col] : 0.0, be = sc.beta[col];
+        const bool act = sc.active[col] != 0;
+        if (!act && al == 0.0) return;
+        auto one = [&](int64_t i, double dv, double xv, T zv) {
+            if (al != 0.0) x[i] = xv + al * dv;
+            if (act) {
+                const double v = widen(zv) + be * dv;
+                d[i] = v;
+                if (hi) split_pair(v, hi[i], lo[i]);
+            }
+        };
+        for (; u + 3 * step < n; u += 4 * step) {
+            int64_t id[4];
+            double dv[4], xv[4];
+            T zv[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                id[e] = (u + e * step) * k + col;
+                dv[e] = d[id[e]];
+                xv[e] = al != 0.0 ? x[id[e]] : 0.0;
+                zv[e] = z[id[e]];
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) one(id[e], dv[e], xv[e], zv[e]);
         }
-    }
-    sc.beta[c] = b;
+        for (; u < n; u += step) {
+            const int64_t i = u * k + col;
+            one(i, d[i], al != 0.0 ? x[i] : 0.0, z[i]);
+        }
+    });
 }
 
-// d = s + beta d (active columns)
-__global__ void __launch_bounds__(256) k_bpcg_dir(int64_t nk, int k, BatchScalars sc, const double* __restrict__ s,
-                                                  double* __restrict__ d) {
-    const int64_t stride = (int64_t)gridDim.x * 256;
-    const int dc = (int)(stride % k);
-    int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    int c = (int)(e % k);
-    for (; e < nk; e += stride, c = (c + dc >= k) ? c + dc - k : c + dc) {
-        if (sc.active[c]) d[e] = s[e] + sc.beta[c] * d[e];
+// sums of up to two partial arrays for every column, 32 columns and 32 row
+// groups at a time (fixed order); f(c, total1, total2) runs on one thread per
+// column.  CTAs of 1024 threads, each with its own columns.
+__device__ __forceinline__ double group_sum(const double* p, int n, int k, int c, int g) {
+    double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+    int q = g;
+    for (; q + 96 < n; q += 128) {
+        a0 += p[(size_t)q * k + c];
+        a1 += p[(size_t)(q + 32) * k + c];
+        a2 += p[(size_t)(q + 64) * k + c];
+        a3 += p[(size_t)(q + 96) * k + c];
+    }
+    for (; q < n; q += 32) a0 += p[(size_t)q * k + c];
+    return (a0 + a1) + (a2 + a3);
+}
+template <class F>
+__device__ __forceinline__ void column_totals(const double* p1, int n1, const double* p2, int n2, int k, F&& f) {
+    __shared__ double s1[32][33], s2[32][33];
+    const int cl = threadIdx.x & 31, g = threadIdx.x >> 5;
+    for (int c0 = blockIdx.x * 32; c0 < k; c0 += gridDim.x * 32) {
+        const int c = c0 + cl;
+        s1[g][cl] = c < k ? group_sum(p1, n1, k, c, g) : 0.0;
+        s2[g][cl] = c < k && n2 > 0 ? group_sum(p2, n2, k, c, g) : 0.0;
+        __syncthreads();
+        if (g == 0 && c < k) {
+            double t1 = 0, t2 = 0;
+            for (int q = 0; q < 32; ++q) {
+                t1 += s1[q][cl];
+                t2 += s2[q][cl];
+            }
+            f(c, t1, t2);
+        }
+        __syncthreads();
     }
 }
 
-__global__ void k_bpcg_end(int k, BatchScalars sc, double tol2, int maxit, int it) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it < 0) it = sc.counter[2];
-    if (c >= k || !sc.active[c]) return;
-    sc.iters[c] = it + 1;
-    sc.active[c] = (it + 1 < maxit && sc.delta_new[c] > tol2 * sc.delta0[c]) ? 1 : 0;
+// (also clears the counts that k_bpcg_end adds up)
+__global__ void __launch_bounds__(1024) k_bpcg_alpha(int k, BatchScalars sc, const double* partials, int np) {
+    if (blockIdx.x == 0 && threadIdx.x < 2) sc.counter[threadIdx.x] = 0;
+    column_totals(partials, np, nullptr, 0, k, [&](int c, double dq, double) {
+        double a = 0;
+        if (sc.active[c]) {
+            a = sc.delta_new[c] / dq;
+            if (!(dq > 0.0) || !isfinite(a)) {
+                sc.broken[c] = 1;
+                sc.active[c] = 0;
+                a = 0;
+            }
+        }
+        sc.alpha[c] = a;
+    });
+}
+
+// the end of an iteration: ||r_c|| into the history, delta_new = r_c.z_c,
+// beta, the stopping test and the counts of active and broken columns.
+// it < 0: the iteration index is the device-side counter[2], which advances
+// (one CTA then).
+__global__ void __launch_bounds__(1024) k_bpcg_end(int k, BatchScalars sc, const double* prr, int nrr,
+                                                   const double* prz, int nrz, double* hist, int maxit, double tol2,
+                                                   int it) {
+    __shared__ int cnt[2];
+    const int at = it >= 0 ? it : sc.counter[2];
+    if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
+    __syncthreads();
+    column_totals(prr, nrr, prz, nrz, k, [&](int c, double rr, double rs) {
+        double b = 0;
+        if (sc.active[c]) {
+            hist[(size_t)c * maxit + at] = sqrt(rr);
+            sc.delta_old[c] = sc.delta_new[c];
+            sc.delta_new[c] = rs;
+            b = rs / sc.delta_old[c];
+            if (!isfinite(b) || rs < 0.0) {   // r.z < 0: preconditioner not positive definite
+                sc.broken[c] = 1;
+                sc.active[c] = 0;
+                b = 0;
+            } else {
+                sc.iters[c] = at + 1;
+                sc.active[c] = (at + 1 < maxit && rs > tol2 * sc.delta0[c]) ? 1 : 0;
+            }
+        }
+        sc.beta[c] = b;
+        if (sc.active[c]) atomicAdd(&cnt[0], 1);
+        if (sc.broken[c]) atomicAdd(&cnt[1], 1);
+    });
+    __syncthreads();
+    if (threadIdx.x < 2 && cnt[threadIdx.x]) atomicAdd(&sc.counter[threadIdx.x], cnt[threadIdx.x]);
+    if (threadIdx.x == 0 && it < 0) sc.counter[2] = at + 1;
 }
 
 // ---------------------------------------------------- multi-RHS coarse solve
-// one CTA per column: (b -= mean(b)); x = Cinv b, FP64 accumulation
+// mean of every column (one CTA each), subtracted in place when asked
 template <class T>
-__global__ void __launch_bounds__(256) k_bcoarse(int n, int k, T* b, T* x, const double* __restrict__ Cinv,
-                                                int mean_project, int solve) {
-    extern __shared__ double sb[];   // n doubles when solving, unused otherwise
+__global__ void __launch_bounds__(256) k_bmean(int n, int k, T* b, double* __restrict__ mean, int subtract) {
     __shared__ double red[8];
     const int c = blockIdx.x;
     double s = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double v = (double)b[(size_t)i * k + c];
-        if (solve) sb[i] = v;
-        s += v;
-    }
-    if (mean_project) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x) s += (double)b[(size_t)i * k + c];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-        __syncthreads();
-        double t = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-        const double mean = t / n;
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            const double v = (solve ? sb[i] : (double)b[(size_t)i * k + c]) - mean;
-            if (solve) sb[i] = v;
-            b[(size_t)i * k + c] = (T)v;
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    double t = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
+    const double m = t / n;
+    if (threadIdx.x == 0) mean[c] = m;
+    if (subtract)
+        for (int i = threadIdx.x; i < n; i += blockDim.x) b[(size_t)i * k + c] = (T)((double)b[(size_t)i * k + c] - m);
+}
+
+// x = Cinv (b - mean) for all columns, FP64 accumulation (mean null: 0).  A
+// CTA takes four rows and 32 V columns, its eight warps an eighth of the sum
+// each, so that b is read once for four rows and every SM has work.  One CTA
+// per column read Cinv k times with k CTAs in flight: 220 us for 576 unknowns
+// and 64 columns, against the FP64 pipes' 35.
+template <class T, int V>
+__global__ void __launch_bounds__(256) k_bcoarse_rows(int n, int k, const T* __restrict__ b, T* __restrict__ x,
+                                                      const double* __restrict__ Cinv,
+                                                      const double* __restrict__ mean) {
+    constexpr int R = 4;
+    __shared__ double part[8][R][32 * V];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row0 = blockIdx.x * R;
+    const int c = (blockIdx.y * 32 + lane) * V;
+    const int per = (n + 7) / 8, j0 = warp * per, j1 = min(n, j0 + per);
+    double acc[R][V];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[r][v] = 0;
+    if (c < k) {
+        double mv[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) mv[v] = mean ? mean[c + v] : 0.0;
+        const double* cr[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) cr[r] = Cinv + (size_t)min(row0 + r, n - 1) * n;
+#pragma unroll 4
+        for (int j = j0; j < j1; ++j) {
+            double bv[V];
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                bv[v] = as_double(__ldg(b + (size_t)j * k + c + v));
+                if (mean) bv[v] -= mv[v];
+            }
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const double a = __ldg(cr[r] + j);
+#pragma unroll
+                for (int v = 0; v < V; ++v) acc[r][v] = fma(a, bv[v], acc[r][v]);
+            }
         }
     }
-    __syncthreads();
-    if (!solve) return;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int row = w; row < n; row += nw) {
-        double a = 0;
-        for (int cc = lane; cc < n; cc += 32) a += Cinv[(size_t)row * n + cc] * sb[cc];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) x[(size_t)row * k + c] = (T)a;
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int v = 0; v < V; ++v) part[warp][r][lane * V + v] = acc[r][v];
+    __syncthreads();
+    for (int t = threadIdx.x; t < R * 32 * V; t += 256) {
+        const int r = t / (32 * V), cl = t - r * (32 * V), cc = blockIdx.y * 32 * V + cl;
+        if (row0 + r >= n || cc >= k) continue;
+        double s = 0;
+        for (int w = 0; w < 8; ++w) s += part[w][r][cl];
+        x[(size_t)(row0 + r) * k + cc] = (T)s;
     }
 }
 
@@ -855,12 +1006,11 @@ struct Batch {
     const mgldg_bsr* outer_A = nullptr;
     bool tuned = false;
     // block PCG
-    double *R = nullptr, *D = nullptr, *Q = nullptr, *S = nullptr, *hist = nullptr;
+    double *R = nullptr, *D = nullptr, *Q = nullptr, *hist = nullptr;
     float *Dhi = nullptr, *Dlo = nullptr;   // D as float pairs (mixed forms' double-float Q = A D)
     int64_t pcg_nk = 0;
     int hist_len = 0;
-    double* partials = nullptr;
-    int partials_len = 0;
+    double *partials = nullptr, *prr = nullptr, *mean = nullptr;   // column sums (two sets), coarse column means
     BatchScalars sc{};
     double* sc_mem = nullptr;
     int* sc_int = nullptr;
@@ -892,7 +1042,7 @@ void batch_free(Batch* b) {
         dfree(L.x); dfree(L.b); dfree(L.r); dfree(L.xt);
         dfree(L.x32); dfree(L.b32); dfree(L.r32); dfree(L.xt32);
     }
-    dfree(b->R); dfree(b->D); dfree(b->Q); dfree(b->S); dfree(b->hist); dfree(b->Dhi); dfree(b->Dlo);
+    dfree(b->R); dfree(b->D); dfree(b->Q); dfree(b->hist); dfree(b->Dhi); dfree(b->Dlo);
     dfree(b->partials);
     dfree(b->sc_mem);
     dfree(b->sc_int);
@@ -1011,10 +1161,15 @@ static void ensure_batch(mgldg_mg* m, int k, const mgldg_bsr* A_outer) {
         b->sc.broken = b->sc_int + 2 * k;
         b->sc.counter = b->sc_int + 3 * k;
         MG_CHECK_CUDA(cudaMallocHost(&b->h_counter, 2 * sizeof(int)));
-        b->partials_len = ctx->sm_count * 4 * k;   // coldot_grid partial rows per column
-        b->partials = dalloc<double>(b->partials_len);
+        const size_t rows = (size_t)ctx->sm_count * 4;   // coldot_grid partial rows per column
+        b->partials = dalloc<double>((2 * rows + 1) * k);
+        b->prr = b->partials + rows * k;
+        b->mean = b->prr + rows * k;
     }
     Batch* b = m->batch;
+    if (!b->tuned)
+        for (auto& L : m->L)
+            if (L.Dinv) rep_ensure_batch(ctx, const_cast<mgldg_bsr*>(L.A), L.Dinv);
     if (!b->tuned) {
         // tile widths per level operator and kernel, on the level buffers
         // (their contents are overwritten before every use)
@@ -1069,6 +1224,31 @@ static void ensure_batch(mgldg_mg* m, int k, const mgldg_bsr* A_outer) {
 }
 
 // ------------------------------------------------------- multi-RHS V-cycle
+// A level operator's product or sweep.  FP64 (bound by its pipes): from the
+// table of the operator's distinct blocks where it has one, which skips the
+// zero block columns (44,197 rows of 9 x 9, 24 columns: sweep 954 -> 764 us).
+// FP32 keeps the general kernel: rows grouped by class lose the locality of
+// their gathers (328 MB of DRAM reads against 204 MB, 135 against 108 us per
+// sweep with 64 columns).
+template <class T>
+static void level_spmm(mgldg_mg* m, const mgldg_bsr* A, const SpmmArgs<T>& a, int mode, const TileCfg& cfg, int kclass) {
+    if constexpr (std::is_same<T, double>::value) {
+        RepMM r{};
+        r.k = a.k;
+        r.X = a.X;
+        r.Yin = a.Yin;
+        r.B = a.B;
+        r.Y = a.Y;
+        r.alpha = a.alpha;
+        r.beta = a.beta;
+        r.omega = a.omega;
+        r.jacobi = mode;
+        r.xzero = a.xzero;
+        if (rep_spmm(m->ctx, A, r, kclass)) return;
+    }
+    spmm_launch<T>(m->ctx, A->br, A->bc, a, mode, cfg, kclass);
+}
+
 // n Jacobi sweeps on level l; xzero: x is zero and not materialised
 template <class T>
 static void brelax(mgldg_mg* m, int l, int n, bool xzero = false) {
@@ -1086,7 +1266,7 @@ static void brelax(mgldg_mg* m, int l, int n, bool xzero = false) {
         a.B = BL<T>::b(B);
         a.omega = (T)m->p.omega;
         a.xzero = (xzero && s == 0) ? 1 : 0;
-        spmm_launch<T>(ctx, L.A->br, L.A->bc, a, 1, B.jac, MGLDG_K_JACOBI);
+        level_spmm<T>(m, L.A, a, 1, B.jac, MGLDG_K_JACOBI);
         std::swap(BL<T>::x(B), BL<T>::xt(B));
     }
 }
@@ -1098,20 +1278,28 @@ static void bcoarse(mgldg_mg* m, int l, bool xzero) {
     mgldg_ctx* ctx = m->ctx;
     const int k = m->batch->k;
     ctx->cur_level = l;
-    if (m->p.solver == MGLDG_COARSE_RELAXATION) {
-        if (m->p.mean_project) {
-            Launch K(ctx, MGLDG_K_COARSE);
-            k_bcoarse<T><<<k, 256, 0, ctx->stream>>>((int)L.n, k, BL<T>::b(B), BL<T>::x(B), nullptr, 1, 0);
-        }
-        check_launch();
+    const bool relaxed = m->p.solver == MGLDG_COARSE_RELAXATION;
+    const double* mean = nullptr;
+    if (m->p.mean_project) {
+        Launch K(ctx, MGLDG_K_COARSE);
+        k_bmean<T><<<k, 256, 0, ctx->stream>>>((int)L.n, k, BL<T>::b(B), m->batch->mean, relaxed ? 1 : 0);
+        mean = m->batch->mean;
+    }
+    check_launch();
+    if (relaxed) {
         brelax<T>(m, l, m->p.npre, xzero);
         brelax<T>(m, l, m->p.npost);
         return;
     }
     {
+        const int n = (int)L.n;
         Launch K(ctx, MGLDG_K_COARSE);
-        k_bcoarse<T><<<k, 256, L.n * sizeof(double), ctx->stream>>>((int)L.n, k, BL<T>::b(B), BL<T>::x(B), m->Cinv,
-                                                                    m->p.mean_project, 1);
+        if (k >= 64 && k % 2 == 0)
+            k_bcoarse_rows<T, 2><<<dim3((n + 3) / 4, (k + 63) / 64), 256, 0, ctx->stream>>>(
+                n, k, BL<T>::b(B), BL<T>::x(B), m->Cinv, mean);
+        else
+            k_bcoarse_rows<T, 1><<<dim3((n + 3) / 4, (k + 31) / 32), 256, 0, ctx->stream>>>(
+                n, k, BL<T>::b(B), BL<T>::x(B), m->Cinv, mean);
     }
     check_launch();
 }
@@ -1137,7 +1325,7 @@ static void bvcycle(mgldg_mg* m, int l, bool xzero) {
         a.X = BL<T>::x(B);
         a.Yin = BL<T>::b(B);
         a.Y = BL<T>::r(B);
-        spmm_launch<T>(ctx, L.A->br, L.A->bc, a, 0, B.spmm, MGLDG_K_SPMV);
+        level_spmm<T>(m, L.A, a, 0, B.spmm, MGLDG_K_SPMV);
     }
     {
         // b_c = T^T r
@@ -1204,6 +1392,39 @@ static void bprecon(mgldg_mg* m, const double* R, double* S, bool x_is_zero) {
     }
 }
 
+// Z = V-cycle(R) from zero for the block CG, Z left in level 0's x.  The
+// mixed forms' FP32 right-hand side has been written by the caller; in FP64
+// the level reads R itself (the coarsest level of a one-level hierarchy may
+// project its right-hand side in place, so that one copies).
+static void bprecon_inplace(mgldg_mg* m) {
+    mgldg_ctx* ctx = m->ctx;
+    Batch* b = m->batch;
+    const int64_t nk = m->L[0].n * b->k;
+    BatchLevel& B = b->L[0];
+    struct LevelReset {
+        mgldg_ctx* c;
+        ~LevelReset() { c->cur_level = -1; }
+    } reset{ctx};
+    const bool z = zero_start(m, 0);
+    if (m->p.precision != MGLDG_PREC_FP64) {
+        if (!z) MG_CHECK_CUDA(cudaMemsetAsync(B.x32, 0, nk * sizeof(float), ctx->stream));
+        bvcycle<float>(m, 0, z);
+        return;
+    }
+    if (!z) MG_CHECK_CUDA(cudaMemsetAsync(B.x, 0, nk * sizeof(double), ctx->stream));
+    if (m->L.size() == 1 && m->p.mean_project) {
+        MG_CHECK_CUDA(cudaMemcpyAsync(B.b, b->R, nk * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+        bvcycle<double>(m, 0, z);
+        return;
+    }
+    struct Borrow {
+        double *&p, *own;
+        ~Borrow() { p = own; }
+    } borrow{B.b, B.b};
+    B.b = b->R;
+    bvcycle<double>(m, 0, z);
+}
+
 // ------------------------------------------- double-float outer SpMM (mixed) --
 // Q = A D for the mixed forms on the FP32 pipes: A = val32 + lo32 and D =
 // Dhi + Dlo as float pairs, each product exact in its high part (FMA error
@@ -1211,17 +1432,6 @@ static void bprecon(mgldg_mg* m, const double* R, double* S, bool x_is_zero) {
 // rounded operations (about 2^-44 relative), Q in FP64.  One warp per block
 // row, both halves of each block staged (transposed) in shared memory, the
 // lane owning V consecutive columns of the column tile.
-__device__ __forceinline__ void df_acc(float& sh, float& sl, float ah, float al, float dh, float dl) {
-    const float p = __fmul_rn(ah, dh);
-    const float pe = fmaf(ah, dh, -p);
-    const float t = fmaf(ah, dl, fmaf(al, dh, pe));
-    const float s = __fadd_rn(sh, p);
-    const float bb = __fsub_rn(s, sh);
-    const float e = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bb)), __fsub_rn(p, bb));
-    sh = s;
-    sl = __fadd_rn(sl, __fadd_rn(e, t));
-}
-
 template <int B, int V>
 __global__ void __launch_bounds__(256) k_spmm_df64(int nbr, const int* __restrict__ row_ptr,
                                                    const int* __restrict__ col_idx, const float* __restrict__ ahi,
@@ -1261,7 +1471,7 @@ __global__ void __launch_bounds__(256) k_spmm_df64(int nbr, const int* __restric
                     for (int r = 0; r < B; ++r) {
                         const float ah = sth[cc * S::BRP + r], al = stl[cc * S::BRP + r];
 #pragma unroll
-                        for (int v = 0; v < V; ++v) df_acc(sh[r][v], sl[r][v], ah, al, xh[v], xl[v]);
+                        for (int v = 0; v < V; ++v) df_fma(sh[r][v], sl[r][v], ah, al, xh[v], xl[v]);
                     }
                 }
             }
@@ -1271,38 +1481,16 @@ __global__ void __launch_bounds__(256) k_spmm_df64(int nbr, const int* __restric
 #pragma unroll
             for (int r = 0; r < B; ++r)
 #pragma unroll
-                for (int v = 0; v < V; ++v) Q[y0 + (size_t)r * k + v] = (double)sh[r][v] + (double)sl[r][v];
+                for (int v = 0; v < V; ++v) Q[y0 + (size_t)r * k + v] = widen(sh[r][v]) + widen(sl[r][v]);
         }
     }
 }
 
-// float pair of D (all columns, or the active ones after a direction update)
+// float pair of D
 __global__ void __launch_bounds__(256) k_bsplit(int64_t nk, const double* __restrict__ d, float* __restrict__ hi,
                                                 float* __restrict__ lo) {
-    for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < nk; e += (int64_t)gridDim.x * 256) {
-        const double v = d[e];
-        const float h = (float)v;
-        hi[e] = h;
-        lo[e] = (float)(v - (double)h);
-    }
-}
-
-__global__ void __launch_bounds__(256) k_bpcg_dir_split(int64_t nk, int k, BatchScalars sc, const double* __restrict__ s,
-                                                        double* __restrict__ d, float* __restrict__ hi,
-                                                        float* __restrict__ lo) {
-    const int64_t stride = (int64_t)gridDim.x * 256;
-    const int dc = (int)(stride % k);
-    int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    int c = (int)(e % k);
-    for (; e < nk; e += stride, c = (c + dc >= k) ? c + dc - k : c + dc) {
-        if (sc.active[c]) {
-            const double v = s[e] + sc.beta[c] * d[e];
-            d[e] = v;
-            const float h = (float)v;
-            hi[e] = h;
-            lo[e] = (float)(v - (double)h);
-        }
-    }
+    for (int64_t e = (int64_t)blockIdx.x * 256 + threadIdx.x; e < nk; e += (int64_t)gridDim.x * 256)
+        split_pair(d[e], hi[e], lo[e]);
 }
 
 static bool df64_batch_ok(const mgldg_mg* m, const mgldg_bsr* A) {
@@ -1332,6 +1520,7 @@ static void launch_spmm_df64(mgldg_ctx* ctx, const mgldg_bsr* A, const float* Dh
 
 static void outer_spmm_df64(mgldg_mg* m, const mgldg_bsr* A, double* Q) {
     const Batch* b = m->batch;
+    if (rep_spmm_df64(m->ctx, A, b->k, b->Dhi, b->Dlo, Q)) return;
     switch (A->br) {
         case 4: launch_spmm_df64<4>(m->ctx, A, b->Dhi, b->Dlo, b->k, Q); return;
         case 6: launch_spmm_df64<6>(m->ctx, A, b->Dhi, b->Dlo, b->k, Q); return;
@@ -1350,15 +1539,15 @@ static void outer_spmm(mgldg_mg* m, const mgldg_bsr* A, double alpha, const doub
     a.X = X;
     a.Yin = Yin;
     a.Y = Y;
-    spmm_launch<double>(m->ctx, A->br, A->bc, a, 0, m->batch->outer, MGLDG_K_SPMV);
+    level_spmm<double>(m, A, a, 0, m->batch->outer, MGLDG_K_SPMV);
 }
 
 static void ensure_bpcg(mgldg_mg* m, int64_t nk, int maxit) {
     Batch* b = m->batch;
     if (b->pcg_nk != nk) {
-        dfree(b->R); dfree(b->D); dfree(b->Q); dfree(b->S); dfree(b->Dhi); dfree(b->Dlo);
-        b->R = nullptr; b->D = nullptr; b->Q = nullptr; b->S = nullptr; b->Dhi = nullptr; b->Dlo = nullptr;
-        b->R = dalloc<double>(nk); b->D = dalloc<double>(nk); b->Q = dalloc<double>(nk); b->S = dalloc<double>(nk);
+        dfree(b->R); dfree(b->D); dfree(b->Q); dfree(b->Dhi); dfree(b->Dlo);
+        b->R = nullptr; b->D = nullptr; b->Q = nullptr; b->Dhi = nullptr; b->Dlo = nullptr;
+        b->R = dalloc<double>(nk); b->D = dalloc<double>(nk); b->Q = dalloc<double>(nk);
         if (m->p.precision != MGLDG_PREC_FP64) {
             b->Dhi = dalloc<float>(nk);
             b->Dlo = dalloc<float>(nk);
@@ -1411,6 +1600,8 @@ static void bpcg(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, int k, const d
     sync(ctx);
     take_batch_errors(m);
     int i = 0;
+    const dim3 gcol(coldot_grid(ctx, n), (k + 255) / 256);
+    const bool mixed = m->p.precision != MGLDG_PREC_FP64;
     while (b->h_counter[0] > 0) {
         // Q = A D ; alpha = delta / colsum(D o Q)
         if (df) outer_spmm_df64(m, A, b->Q);
@@ -1418,42 +1609,44 @@ static void bpcg(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, int k, const d
         coldot<double>(ctx, n, k, b->D, b->Q, b->partials, &np);
         {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_bpcg_alpha<<<gk, 128, 0, ctx->stream>>>(k, sc, b->partials, np);
+            k_bpcg_alpha<<<(k + 31) / 32, 1024, 0, ctx->stream>>>(k, sc, b->partials, np);
         }
         check_launch();
+        // R -= alpha Q (or X += alpha D, R = B - A X), its column norms and
+        // the V-cycle's right-hand side
         const bool replace = i % 50 == 0;
-        {
+        float* b32 = mixed ? b->L[0].b32 : nullptr;
+        int nrr = (int)gcol.x;
+        if (replace) {
+            {
+                Launch L(ctx, MGLDG_K_VECTOR);
+                k_bpcg_xupdate<<<gcol, 256, 0, ctx->stream>>>(n, k, sc, b->D, X);
+            }
+            check_launch();
+            outer_spmm(m, A, -1.0, X, 1.0, B, b->R);
+            coldot<double>(ctx, n, k, b->R, b->R, b->prr, &nrr);
+            if (b32) bconvert<double, float>(ctx, nk, b->R, b32);
+        } else {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_bpcg_update<<<gvec, 256, 0, ctx->stream>>>(nk, k, sc, b->D, b->Q, X, b->R, replace ? 0 : 1);
+            k_bpcg_update<<<gcol, 256, 0, ctx->stream>>>(n, k, sc, b->Q, b->R, b32, b->prr);
         }
         check_launch();
-        if (replace) outer_spmm(m, A, -1.0, X, 1.0, B, b->R);
-        coldot<double>(ctx, n, k, b->R, b->R, b->partials, &np);
+        // Z = M(R), left in the level's X ; delta_new = colsum(R o Z) ; beta ;
+        // X += alpha D ; D = Z + beta D
+        bprecon_inplace(m);
+        if (mixed) coldot<float>(ctx, n, k, b->R, b->L[0].x32, b->partials, &np);
+        else coldot<double>(ctx, n, k, b->R, b->L[0].x, b->partials, &np);
         {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_bpcg_rr<<<gk, 128, 0, ctx->stream>>>(k, sc, b->partials, np, b->hist, maxit, i);
-        }
-        check_launch();
-        // S = M(R) ; delta_new = colsum(R o S) ; beta ; D = S + beta D
-        bprecon(m, b->R, b->S, true);
-        coldot<double>(ctx, n, k, b->R, b->S, b->partials, &np);
-        {
-            Launch L(ctx, MGLDG_K_VECTOR);
-            k_bpcg_beta<<<gk, 128, 0, ctx->stream>>>(k, sc, b->partials, np);
-        }
-        check_launch();
-        {
-            Launch L(ctx, MGLDG_K_VECTOR);
-            if (df) k_bpcg_dir_split<<<gvec, 256, 0, ctx->stream>>>(nk, k, sc, b->S, b->D, b->Dhi, b->Dlo);
-            else k_bpcg_dir<<<gvec, 256, 0, ctx->stream>>>(nk, k, sc, b->S, b->D);
+            k_bpcg_end<<<(k + 31) / 32, 1024, 0, ctx->stream>>>(k, sc, b->prr, nrr, b->partials, np, b->hist, maxit,
+                                                               tol2, i);
         }
         {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_bpcg_end<<<gk, 128, 0, ctx->stream>>>(k, sc, tol2, maxit, i);
-        }
-        {
-            Launch L(ctx, MGLDG_K_VECTOR);
-            k_bpcg_count<<<1, 256, 0, ctx->stream>>>(k, sc);
+            const int xupd = replace ? 0 : 1;
+            float *hi = df ? b->Dhi : nullptr, *lo = df ? b->Dlo : nullptr;
+            if (mixed) k_bpcg_dir<float><<<gcol, 256, 0, ctx->stream>>>(n, k, sc, b->L[0].x32, b->D, X, xupd, hi, lo);
+            else k_bpcg_dir<double><<<gcol, 256, 0, ctx->stream>>>(n, k, sc, b->L[0].x, b->D, X, xupd, hi, lo);
         }
         check_launch();
         MG_CHECK_CUDA(cudaMemcpyAsync(b->h_counter, sc.counter, 2 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -1493,7 +1686,7 @@ struct SegWork {
     int64_t n = 0;
     int gx = 0;
     int64_t* off = nullptr;
-    double *R = nullptr, *D = nullptr, *Q = nullptr, *S = nullptr, *hist = nullptr, *partials = nullptr;
+    double *R = nullptr, *D = nullptr, *Q = nullptr, *hist = nullptr, *partials = nullptr, *prr = nullptr;
     int hist_len = 0;
     BatchScalars sc{};
     double* sc_mem = nullptr;
@@ -1515,7 +1708,7 @@ void seg_free(SegWork* w) {
     if (!w) return;
     if (w->exec) cudaGraphExecDestroy(w->exec);
     dfree(w->off);
-    dfree(w->R); dfree(w->D); dfree(w->Q); dfree(w->S); dfree(w->hist); dfree(w->partials);
+    dfree(w->R); dfree(w->D); dfree(w->Q); dfree(w->hist); dfree(w->partials);
     dfree(w->sc_mem);
     dfree(w->sc_int);
     if (w->h_counter) cudaFreeHost(w->h_counter);
@@ -1523,14 +1716,15 @@ void seg_free(SegWork* w) {
 }
 
 // partials[blockIdx.x * nseg + s] = this CTA's part of segment s of a.b
+template <class T>
 __global__ void __launch_bounds__(256) k_segdot(const int64_t* __restrict__ off, int nseg, const double* __restrict__ a,
-                                               const double* __restrict__ b, double* __restrict__ partials) {
+                                               const T* __restrict__ b, double* __restrict__ partials) {
     __shared__ double red[8];
     const int s = blockIdx.y;
     const int64_t lo = off[s], hi = off[s + 1];
     double acc = 0;
     for (int64_t i = lo + (int64_t)blockIdx.x * 256 + threadIdx.x; i < hi; i += (int64_t)gridDim.x * 256)
-        acc += a[i] * b[i];
+        acc += a[i] * as_double(b[i]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -1542,29 +1736,64 @@ __global__ void __launch_bounds__(256) k_segdot(const int64_t* __restrict__ off,
     }
 }
 
-// x += alpha_s d ; (r -= alpha_s q) on active segments
-__global__ void __launch_bounds__(256) k_segupdate(const int64_t* __restrict__ off, BatchScalars sc,
-                                                  const double* __restrict__ d, const double* __restrict__ q,
-                                                  double* __restrict__ x, double* __restrict__ r, int update_r) {
+// x += alpha_s d on active segments (before a residual replacement)
+__global__ void __launch_bounds__(256) k_segxupdate(const int64_t* __restrict__ off, BatchScalars sc,
+                                                   const double* __restrict__ d, double* __restrict__ x) {
     const int s = blockIdx.y;
     if (!sc.active[s]) return;
     const double al = sc.alpha[s];
     const int64_t lo = off[s], hi = off[s + 1];
-    for (int64_t i = lo + (int64_t)blockIdx.x * 256 + threadIdx.x; i < hi; i += (int64_t)gridDim.x * 256) {
+    for (int64_t i = lo + (int64_t)blockIdx.x * 256 + threadIdx.x; i < hi; i += (int64_t)gridDim.x * 256)
         x[i] += al * d[i];
-        if (update_r) r[i] -= al * q[i];
+}
+
+// r -= alpha_s q on active segments, the V-cycle's FP32 right-hand side when
+// given, and the partial r.r (k_segdot's layout)
+__global__ void __launch_bounds__(256) k_segupdate(const int64_t* __restrict__ off, int nseg, BatchScalars sc,
+                                                  const double* __restrict__ q, double* __restrict__ r,
+                                                  float* __restrict__ b32, double* __restrict__ partials) {
+    __shared__ double red[8];
+    const int s = blockIdx.y;
+    const bool act = sc.active[s] != 0;
+    const double al = act ? sc.alpha[s] : 0.0;
+    const int64_t lo = off[s], hi = off[s + 1];
+    double acc = 0;
+    for (int64_t i = lo + (int64_t)blockIdx.x * 256 + threadIdx.x; i < hi; i += (int64_t)gridDim.x * 256) {
+        double v = r[i];
+        if (act) {
+            v -= al * q[i];
+            r[i] = v;
+        }
+        if (b32) b32[i] = narrow(v);
+        acc += v * v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0;
+        for (int w = 0; w < 8; ++w) t += red[w];
+        partials[(size_t)blockIdx.x * nseg + s] = t;
     }
 }
 
-// d = s + beta_s d on active segments
+// x += alpha_s d where the segment took a step and xupd, d = z + beta_s d on
+// active segments
+template <class T>
 __global__ void __launch_bounds__(256) k_segdir(const int64_t* __restrict__ off, BatchScalars sc,
-                                               const double* __restrict__ sv, double* __restrict__ d) {
+                                               const T* __restrict__ z, double* __restrict__ d,
+                                               double* __restrict__ x, int xupd) {
     const int s = blockIdx.y;
-    if (!sc.active[s]) return;
-    const double be = sc.beta[s];
+    const bool act = sc.active[s] != 0;
+    const double al = xupd ? sc.alpha[s] : 0.0, be = sc.beta[s];
+    if (!act && al == 0.0) return;
     const int64_t lo = off[s], hi = off[s + 1];
-    for (int64_t i = lo + (int64_t)blockIdx.x * 256 + threadIdx.x; i < hi; i += (int64_t)gridDim.x * 256)
-        d[i] = sv[i] + be * d[i];
+    for (int64_t i = lo + (int64_t)blockIdx.x * 256 + threadIdx.x; i < hi; i += (int64_t)gridDim.x * 256) {
+        const double dv = d[i];
+        if (al != 0.0) x[i] += al * dv;
+        if (act) d[i] = widen(z[i]) + be * dv;
+    }
 }
 
 static SegWork* ensure_seg(mgldg_mg* m, const std::vector<int64_t>& off, int maxit) {
@@ -1585,8 +1814,9 @@ static SegWork* ensure_seg(mgldg_mg* m, const std::vector<int64_t>& off, int max
         for (int s = 0; s < nseg; ++s) maxlen = std::max<int64_t>(maxlen, off[s + 1] - off[s]);
         w->gx = (int)std::max<int64_t>(1, std::min<int64_t>((maxlen + 2047) / 2048, 4 * ctx->sm_count / std::max(1, nseg) + 1));
         w->off = dalloc<int64_t>(nseg + 1);
-        w->R = dalloc<double>(n); w->D = dalloc<double>(n); w->Q = dalloc<double>(n); w->S = dalloc<double>(n);
-        w->partials = dalloc<double>((size_t)w->gx * nseg);
+        w->R = dalloc<double>(n); w->D = dalloc<double>(n); w->Q = dalloc<double>(n);
+        w->partials = dalloc<double>(2 * (size_t)w->gx * nseg);
+        w->prr = w->partials + (size_t)w->gx * nseg;
         w->sc_mem = dalloc<double>(5 * (size_t)nseg);
         w->sc_int = dalloc<int>(3 * (size_t)nseg + 3);
         w->sc.delta_new = w->sc_mem;
@@ -1615,8 +1845,6 @@ static SegWork* ensure_seg(mgldg_mg* m, const std::vector<int64_t>& off, int max
     return w;
 }
 
-__global__ void k_seg_advance(BatchScalars sc) { sc.counter[2] += 1; }
-
 // while-loop condition of a block of segmented iterations: some segment is
 // still active and the next iteration is not a residual-replacement one
 __global__ void k_seg_cond(BatchScalars sc, cudaGraphConditionalHandle h) {
@@ -1626,55 +1854,53 @@ __global__ void k_seg_cond(BatchScalars sc, cudaGraphConditionalHandle h) {
 // one iteration of every active segment's pcg (krylov.h:43-61); `it` < 0:
 // the iteration index is the device-side counter (graph capture)
 static void seg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, SegWork* w, const double* b, double* x,
-                          double tol2, int maxit, bool replace, int it, bool eager) {
+                          double tol2, int maxit, bool replace, int it) {
     const int nseg = w->nseg;
     BatchScalars sc = w->sc;
     const dim3 grid(w->gx, nseg);
-    const int gk = (nseg + 127) / 128;
-    auto segdot = [&](const double* a, const double* c) {
+    LevelData& L0 = m->L[0];
+    const bool mixed = m->p.precision != MGLDG_PREC_FP64;
+    float* b32 = mixed ? L0.b32 : nullptr;
+    auto segdot = [&](const double* a, const double* c, double* part) {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_segdot<<<grid, 256, 0, ctx->stream>>>(w->off, nseg, a, c, w->partials);
+        k_segdot<double><<<grid, 256, 0, ctx->stream>>>(w->off, nseg, a, c, part);
     };
     spmv<double>(ctx, A, 1.0, w->D, 0.0, nullptr, w->Q);
-    segdot(w->D, w->Q);
+    segdot(w->D, w->Q, w->partials);
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_bpcg_alpha<<<gk, 128, 0, ctx->stream>>>(nseg, sc, w->partials, w->gx);
-    }
-    {
-        Launch L(ctx, MGLDG_K_VECTOR);
-        k_segupdate<<<grid, 256, 0, ctx->stream>>>(w->off, sc, w->D, w->Q, x, w->R, replace ? 0 : 1);
+        k_bpcg_alpha<<<(nseg + 31) / 32, 1024, 0, ctx->stream>>>(nseg, sc, w->partials, w->gx);
     }
     check_launch();
-    if (replace) spmv<double>(ctx, A, -1.0, x, 1.0, b, w->R);
-    segdot(w->R, w->R);
-    {
+    if (replace) {
+        {
+            Launch L(ctx, MGLDG_K_VECTOR);
+            k_segxupdate<<<grid, 256, 0, ctx->stream>>>(w->off, sc, w->D, x);
+        }
+        check_launch();
+        spmv<double>(ctx, A, -1.0, x, 1.0, b, w->R);
+        segdot(w->R, w->R, w->prr);
+        if (b32) bconvert<double, float>(ctx, w->n, w->R, b32);
+    } else {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_bpcg_rr<<<gk, 128, 0, ctx->stream>>>(nseg, sc, w->partials, w->gx, w->hist, maxit, it);
+        k_segupdate<<<grid, 256, 0, ctx->stream>>>(w->off, nseg, sc, w->Q, w->R, b32, w->prr);
     }
     check_launch();
-    if (eager) mg_precon_eager(m, w->R, w->S);
-    else mg_precon(m, w->R, w->S);
-    segdot(w->R, w->S);
+    mg_precon_inplace(m, w->R);
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_bpcg_beta<<<gk, 128, 0, ctx->stream>>>(nseg, sc, w->partials, w->gx);
+        if (mixed) k_segdot<float><<<grid, 256, 0, ctx->stream>>>(w->off, nseg, w->R, L0.x32, w->partials);
+        else k_segdot<double><<<grid, 256, 0, ctx->stream>>>(w->off, nseg, w->R, L0.x, w->partials);
     }
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_segdir<<<grid, 256, 0, ctx->stream>>>(w->off, sc, w->S, w->D);
+        k_bpcg_end<<<1, 1024, 0, ctx->stream>>>(nseg, sc, w->prr, w->gx, w->partials, w->gx, w->hist, maxit, tol2, it);
     }
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_bpcg_end<<<gk, 128, 0, ctx->stream>>>(nseg, sc, tol2, maxit, it);
-    }
-    {
-        Launch L(ctx, MGLDG_K_VECTOR);
-        k_bpcg_count<<<1, 256, 0, ctx->stream>>>(nseg, sc);
-    }
-    {
-        Launch L(ctx, MGLDG_K_VECTOR);
-        k_seg_advance<<<1, 1, 0, ctx->stream>>>(sc);
+        const int xupd = replace ? 0 : 1;
+        if (mixed) k_segdir<float><<<grid, 256, 0, ctx->stream>>>(w->off, sc, L0.x32, w->D, x, xupd);
+        else k_segdir<double><<<grid, 256, 0, ctx->stream>>>(w->off, sc, L0.x, w->D, x, xupd);
     }
     check_launch();
 }
@@ -1697,7 +1923,7 @@ static bool build_seg_graph(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, Seg
         return false;
     }
     try {
-        seg_iteration(ctx, m, A, w, b, x, tol2, maxit, true, -1, true);
+        seg_iteration(ctx, m, A, w, b, x, tol2, maxit, true, -1);
         for (int k = 0; k < MGLDG_K_NCLASS; ++k) w->pro_launches[k] = ctx->launches[k] - before[k];
         cudaStreamCaptureStatus st;
         cudaGraph_t cg = nullptr;
@@ -1725,7 +1951,7 @@ static bool build_seg_graph(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, Seg
             std::memcpy(b2, ctx->launches, sizeof b2);
             MG_CHECK_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0,
                                                         cudaStreamCaptureModeThreadLocal));
-            seg_iteration(ctx, m, A, w, b, x, tol2, maxit, false, -1, true);
+            seg_iteration(ctx, m, A, w, b, x, tol2, maxit, false, -1);
             k_seg_cond<<<1, 1, 0, ctx->stream>>>(w->sc, h);
             check_launch();
             cudaGraph_t bg = nullptr;
@@ -1767,7 +1993,7 @@ static void segpcg(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const std::v
     mg_precon(m, w->R, w->D);
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_segdot<<<grid, 256, 0, ctx->stream>>>(w->off, nseg, w->R, w->D, w->partials);
+        k_segdot<double><<<grid, 256, 0, ctx->stream>>>(w->off, nseg, w->R, w->D, w->partials);
     }
     check_launch();
     {
@@ -1808,7 +2034,7 @@ static void segpcg(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const std::v
                 continue;
             }
         }
-        seg_iteration(ctx, m, A, w, b, x, tol2, maxit, i % 50 == 0, i, false);
+        seg_iteration(ctx, m, A, w, b, x, tol2, maxit, i % 50 == 0, i);
         MG_CHECK_CUDA(cudaMemcpyAsync(w->h_counter, sc.counter, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         sync(ctx);
         ++i;

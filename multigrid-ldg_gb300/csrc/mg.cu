@@ -754,18 +754,13 @@ static void precon(mgldg_mg* m, const double* r, double* s, double* part = nullp
 }
 
 void mg_precon(mgldg_mg* m, const double* r, double* s) { precon(m, r, s); }
-void mg_precon_eager(mgldg_mg* m, const double* r, double* s) {
-    if (m->L.empty()) precon(m, r, s);
-    else vcycle_dev(m, r, s, true);
-}
 void mg_take_errors(mgldg_mg* m) { take_errors(m); }
 
 // z = V-cycle(r) from x = 0 for the CG, without copies of the FP64 vectors:
 // in the mixed forms the level's FP32 right-hand side has been written by the
 // caller, in FP64 the level reads r itself (unless the one-level hierarchy
 // projects its right-hand side in place); the result stays in the level's x.
-// partial r.z goes to part (grid CTAs).
-static void cg_precon(mgldg_mg* m, double* r, double* part, int grid) {
+void mg_precon_inplace(mgldg_mg* m, double* r) {
     mgldg_ctx* ctx = m->ctx;
     LevelData& L = m->L[0];
     struct LevelReset {
@@ -776,24 +771,30 @@ static void cg_precon(mgldg_mg* m, double* r, double* part, int grid) {
     if (m->p.precision != MGLDG_PREC_FP64) {
         if (!z) MG_CHECK_CUDA(cudaMemsetAsync(L.x32, 0, L.n * sizeof(float), ctx->stream));
         vcycle<float>(m, 0, z);
-        Launch K(ctx, MGLDG_K_VECTOR);
-        k_out_part<float><<<grid, 256, 0, ctx->stream>>>(L.n, L.x32, r, part);
-    } else {
-        if (!z) MG_CHECK_CUDA(cudaMemsetAsync(L.x, 0, L.n * sizeof(double), ctx->stream));
-        if (m->L.size() == 1 && m->p.mean_project) {
-            MG_CHECK_CUDA(cudaMemcpyAsync(L.bb, r, L.n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
-            vcycle<double>(m, 0, z);
-        } else {
-            struct Borrow {
-                double *&p, *own;
-                ~Borrow() { p = own; }
-            } borrow{L.bb, L.bb};
-            L.bb = r;
-            vcycle<double>(m, 0, z);
-        }
-        Launch K(ctx, MGLDG_K_VECTOR);
-        k_out_part<double><<<grid, 256, 0, ctx->stream>>>(L.n, L.x, r, part);
+        return;
     }
+    if (!z) MG_CHECK_CUDA(cudaMemsetAsync(L.x, 0, L.n * sizeof(double), ctx->stream));
+    if (m->L.size() == 1 && m->p.mean_project) {
+        MG_CHECK_CUDA(cudaMemcpyAsync(L.bb, r, L.n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+        vcycle<double>(m, 0, z);
+        return;
+    }
+    struct Borrow {
+        double *&p, *own;
+        ~Borrow() { p = own; }
+    } borrow{L.bb, L.bb};
+    L.bb = r;
+    vcycle<double>(m, 0, z);
+}
+
+// partial sums of r.z, z the level's x after mg_precon_inplace
+static void cg_precon(mgldg_mg* m, double* r, double* part, int grid) {
+    mgldg_ctx* ctx = m->ctx;
+    LevelData& L = m->L[0];
+    mg_precon_inplace(m, r);
+    Launch K(ctx, MGLDG_K_VECTOR);
+    if (m->p.precision != MGLDG_PREC_FP64) k_out_part<float><<<grid, 256, 0, ctx->stream>>>(L.n, L.x32, r, part);
+    else k_out_part<double><<<grid, 256, 0, ctx->stream>>>(L.n, L.x, r, part);
     check_launch();
 }
 

@@ -49,8 +49,10 @@ void seg_free(SegWork* w);
 // one preconditioner application s = V-cycle(r) from x = 0 (graph replay
 // when possible) and the collection of device-side error reports (mg.cu)
 void mg_precon(mgldg_mg* m, const double* r, double* s);
-// the same with every launch issued directly (for capture into a graph)
-void mg_precon_eager(mgldg_mg* m, const double* r, double* s);
+// z = V-cycle(r) from x = 0 with every launch issued directly (for capture
+// into a graph), z left in level 0's x (x32 in the mixed forms, whose FP32
+// right-hand side b32 the caller has written)
+void mg_precon_inplace(mgldg_mg* m, double* r);
 void mg_take_errors(mgldg_mg* m);
 // true when level i's V-cycle starts from x = 0 with a Jacobi sweep that
 // reads neither x nor the operator, so x need not be zeroed (mg.cu)

@@ -189,6 +189,14 @@ __global__ void __launch_bounds__(256) k_rep_tables(const double* __restrict__ v
         fill_image<float, B>(t.i32 + at * I4::SIZE, D, false, 0);
         fill_image<float, B>(t.i16 + at * I4::SIZE, D, false, 0);
     }
+    if constexpr (B == 16) {
+        for (int e = threadIdx.x; e < 256; e += blockDim.x) {
+            const double v = a[(e % 16) * 16 + e / 16] + 0.0;
+            t.c64[(size_t)u * 256 + e] = v;
+            t.c32[(size_t)u * 256 + e] = (float)v;
+            t.clo[(size_t)u * 256 + e] = (float)(v - (double)(float)v);
+        }
+    }
     if (threadIdx.x == 0) {
         t.mask[u] = rm | (cm << 16);
         t.s16[u] = (float)s;
@@ -204,13 +212,13 @@ __global__ void __launch_bounds__(256) k_rep_tables(const double* __restrict__ v
 // FP32 65,536 rows 9.7 / 11.0, 16,384 rows 8.1 / 7.4.
 static int rep_min_rows(int b) { return b == 16 ? 8192 : (b == 9 ? 16384 : 32768); }
 
-static bool rep_shape(const mgldg_bsr* A) {
+static bool rep_shape(const mgldg_bsr* A, int min_rows) {
     return A->br == A->bc && A->nbr == A->nbc && !A->blk && (A->br == 4 || A->br == 9 || A->br == 16) &&
-           A->nbr >= rep_min_rows(A->br) && A->nnzb < (1LL << 31);
+           A->nbr >= min_rows && A->nnzb < (1LL << 31);
 }
 
-bool rep_probe(mgldg_ctx* ctx, const mgldg_bsr* A, RepProbe& p) {
-    if (!rep_shape(A) || A->rep) return false;
+bool rep_probe(mgldg_ctx* ctx, const mgldg_bsr* A, RepProbe& p, bool batch) {
+    if (A->rep || !rep_shape(A, batch ? kRepMmRows : rep_min_rows(A->br))) return false;
     const size_t bytes = 16 + kHash * sizeof(HashSlot) + (size_t)A->nnzb * sizeof(int);
     p.mem = dalloc<char>(bytes);
     int* head = (int*)p.mem;
@@ -227,7 +235,7 @@ bool rep_probe(mgldg_ctx* ctx, const mgldg_bsr* A, RepProbe& p) {
     return true;
 }
 
-void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
+void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p, int gs_want) {
     // the caller has synchronised: p.head is valid.  A table pays when a
     // block is used several times.
     const int nu = p.head[0];
@@ -312,7 +320,7 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
     // whole groups.  Chunks of 4,096 consecutive rows keep a warp's gathers
     // within one stretch of the vectors; with many classes one chunk wastes
     // fewer slots. ----
-    const int gs = b != 16 || n >= 32768 ? 32 : 16;
+    const int gs = gs_want ? gs_want : (b != 16 || n >= 32768 ? 32 : 16), gu = std::min(gs, 16);
     const int chunk = ncls <= 32 ? 4096 : n;
     std::vector<int> rows, gcls;
     {
@@ -325,7 +333,7 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
             for (int c = 0; c < ncls; ++c) {
                 pos[c] = (int)at;
                 const size_t w = ((size_t)cnt[c] + gs - 1) / gs * gs;
-                gcls.insert(gcls.end(), w / 16, c);
+                gcls.insert(gcls.end(), w / gu, c);
                 at += w;
             }
             rows.resize(at, -1);
@@ -341,6 +349,7 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
     t->nuniq = nu;
     t->ncls = ncls;
     t->gs = gs;
+    t->gu = gu;
     t->nslots = nslots;
     // the classes name their inverse diagonal block by its place in the image
     std::vector<int> didx(nu, -1);
@@ -351,13 +360,17 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
     const size_t nimg = (size_t)nu + t->ndiag;
     const size_t v8 = (size_t)(b == 16 ? Img<double, 16>::SIZE : b * ld) * nimg;
     const size_t v4 = (size_t)(b == 16 ? Img<float, 16>::SIZE : b * ld) * nimg;
-    t->pool = dalloc<char>(v8 * 8 + 3 * v4 * 4 + (size_t)nu * 8);
-    MG_CHECK_CUDA(cudaMemsetAsync(t->pool, 0, v8 * 8 + 3 * v4 * 4, ctx->stream));
+    const size_t vc = b == 16 ? (size_t)nu * 256 : 0;   // smaller blocks' images are by columns
+    t->pool = dalloc<char>((v8 + vc) * 8 + (3 * v4 + 2 * vc) * 4 + (size_t)nu * 8);
+    MG_CHECK_CUDA(cudaMemsetAsync(t->pool, 0, (v8 + vc) * 8 + (3 * v4 + 2 * vc) * 4, ctx->stream));
     t->i64 = (double*)t->pool;
-    t->i32 = (float*)(t->i64 + v8);
+    t->c64 = vc ? t->i64 + v8 : t->i64;
+    t->i32 = (float*)(t->i64 + v8 + vc);
     t->ilo = t->i32 + v4;
     t->i16 = t->ilo + v4;
-    t->s16 = t->i16 + v4;
+    t->c32 = vc ? t->i16 + v4 : t->i32;
+    t->clo = vc ? t->c32 + vc : t->ilo;
+    t->s16 = t->i16 + v4 + 2 * vc;
     t->mask = (unsigned*)(t->s16 + nu);
     t->blk = dalloc<int>(A->nnzb);
     int* dint = (int*)slots;   // the hash slots are done with: three index lists go there
@@ -404,6 +417,15 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p) {
     }
     sync(ctx);
     A->rep = t.release();
+}
+
+bool rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv) {
+    if (A->rep) return A->rep->nslots != 0;
+    RepProbe p;
+    if (!rep_probe(ctx, A, p, true)) return false;
+    sync(ctx);
+    rep_finish(ctx, A, Dinv, p, 4);
+    return A->rep && A->rep->nslots != 0;
 }
 
 // ---------------------------------------------------------------- kernels --
@@ -990,7 +1012,7 @@ bool rep_launch(mgldg_ctx* ctx, const RepTable* t, RepArgs<T>& a, bool f16, int 
 
 }  // namespace
 
-static bool rep_used(const RepTable* t) { return t && t->nslots; }
+static bool rep_used(const RepTable* t) { return t && t->nslots && t->nbr >= rep_min_rows(t->b); }
 
 template <class T>
 bool rep_spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const T* yin, T* y, const T* dotv,

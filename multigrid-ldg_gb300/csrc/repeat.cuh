@@ -18,17 +18,21 @@ namespace mg {
 // 8 (the two column halves of a line pair then lie in different banks).
 struct RepView {
     int b = 0, ld = 0, nbr = 0, nuniq = 0, ndiag = 0, ncls = 0;
-    int gs = 16;                   // slots per group, every group one class
+    int gs = 16, gu = 16;          // slots per group, every group one class; slots per gcls entry
     int nslots = 0;                // 0: too many classes for the slot kernels
     int* blk = nullptr;            // [nnzb] table entry of every stored block
     unsigned* mask = nullptr;      // [nuniq] nonzero rows | nonzero columns << 16
     int* cls = nullptr;            // [ncls][kRepCls]: blocks per row, inverse diagonal block, -, -, entries, their masks
-    int* gcls = nullptr;           // [nslots / 16] class of 16 consecutive slots
+    int* gcls = nullptr;           // [nslots / gu] class of gu consecutive slots
     int* rows = nullptr;           // [nslots] row, -1: padding
     int* cols = nullptr;           // [most blocks per row][nslots] block columns
     double* i64 = nullptr;         // FP64 image
     float *i32 = nullptr, *ilo = nullptr;   // FP32 image and the blocks' low halves (val = i32 + ilo)
     float *i16 = nullptr, *s16 = nullptr;   // block-scaled FP16 values (all by rows), their scales
+    // the nuniq blocks by columns (b lines of ld values, no gap between the
+    // halves), for the multi-vector kernels
+    double* c64 = nullptr;
+    float *c32 = nullptr, *clo = nullptr;
 };
 struct RepTable : RepView {
     void* pool = nullptr;          // owns the value tables and mask
@@ -55,8 +59,27 @@ struct RepProbe {
     RepProbe& operator=(const RepProbe&) = delete;
     ~RepProbe();
 };
-bool rep_probe(mgldg_ctx* ctx, const mgldg_bsr* A, RepProbe& p);
-void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p);
+bool rep_probe(mgldg_ctx* ctx, const mgldg_bsr* A, RepProbe& p, bool batch = false);
+// gs: slots per group (0: the single-vector kernels' choice)
+void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p, int gs = 0);
+
+// the table for multi-vector products (levels from kRepMmRows rows on, also
+// those too small for the single-vector kernels); false: none
+bool rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv);
+constexpr int kRepMmRows = 2048;
+
+// FP64 Y = alpha A X + beta Yin, or (Jacobi) Y = X + omega Dinv (B - A X), on
+// row-major multi-vectors of k columns (spmm_rep.cu); false: no table
+struct RepMM {
+    int k;
+    const double *X, *Yin, *B;
+    double* Y;
+    double alpha, beta, omega;
+    int jacobi, xzero;
+};
+bool rep_spmm(mgldg_ctx* ctx, const mgldg_bsr* A, const RepMM& m, int kclass);
+// Q = A D in double-float arithmetic, D as float pairs
+bool rep_spmm_df64(mgldg_ctx* ctx, const mgldg_bsr* A, int k, const float* Dhi, const float* Dlo, double* Q);
 
 // y = alpha A x + beta yin with the dot epilogue of spmv; false: no table
 template <class T>

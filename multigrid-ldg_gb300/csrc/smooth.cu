@@ -465,8 +465,8 @@ __global__ void __launch_bounds__(WPB * 32, 2)
 // holds t_r = b_r - (A x_in)_r and applies row r of Dinv with t's entries
 // shuffled within the group.  The row loop is warp-uniform so every lane
 // takes part in the shuffles and the shared-memory reduction.
-template <class T, class VT, int B, int MAXB>
-__global__ void __launch_bounds__(256)
+template <class T, class VT, int B, int MAXB, int MINB>
+__global__ void __launch_bounds__(256, MINB)
     k_jacobi_rows(int n, const int* __restrict__ row_ptr, const int* __restrict__ col_idx, const VT* __restrict__ val,
                   const float* __restrict__ scl, const T* __restrict__ Dinv, const T* __restrict__ b,
                   const T* __restrict__ xin, T* __restrict__ xout, T omega, bool xzero) {
@@ -509,13 +509,19 @@ __global__ void __launch_bounds__(256)
 template <class T, int B, class VT = T>
 static void launch_jacobi_rows(mgldg_ctx* ctx, const mgldg_bsr* A, const VT* vals, const T* Dinv, const T* b,
                                const T* xin, T* xout, T omega, bool xzero, const float* scl = nullptr) {
-    constexpr int MAXB = (sizeof(T) == 4 || B <= 4) ? 4 : 2;
+    // FP32 blocks of 6, 9 and 10: blocks in flight given up for four CTAs an SM:
+    // 39.9 -> 33.1 us at 6 x 6, 175k rows; 28.5 -> 27.4 at 9 x 9, 40.0k rows;
+    // 35.5 -> 29.6 at 10 x 10, 43.5k rows.  FP64 stays with the registers the
+    // compiler takes (9 x 9: 93 us against 97, 10 x 10: 94 against 103).
+    constexpr bool F4 = sizeof(T) == 4 && (B == 6 || B == 9 || B == 10);
+    constexpr int MINB = F4 ? 4 : 0;
+    constexpr int MAXB = F4 ? (B == 10 ? 2 : 3) : ((sizeof(T) == 4 || B <= 4) ? 4 : 2);
     const int rows_per_cta = 8 * Rows<B>::G;
     const int grid = std::max(1, std::min((A->nbr + rows_per_cta - 1) / rows_per_cta, ctx->sm_count * 8));
     {
         Launch L(ctx, MGLDG_K_JACOBI);
-        k_jacobi_rows<T, VT, B, MAXB><<<grid, 256, 0, ctx->stream>>>(A->nbr, A->row_ptr, A->col_idx, vals, scl, Dinv,
-                                                                     b, xin, xout, omega, xzero);
+        k_jacobi_rows<T, VT, B, MAXB, MINB><<<grid, 256, 0, ctx->stream>>>(A->nbr, A->row_ptr, A->col_idx, vals, scl,
+                                                                           Dinv, b, xin, xout, omega, xzero);
     }
     check_launch();
 }

@@ -188,11 +188,7 @@ __global__ void __launch_bounds__(256, 2) k_vtail(const __grid_constant__ TailAr
         for (int i = threadIdx.x; i < n; i += blockDim.x) sb[i] = (double)__ldcg(v.b + i);
         __syncthreads();
         for (int row = gw; row < n; row += nw) {
-            const double* cr = a.Cinv + (size_t)row * n;
-            double s = 0;
-            for (int c = lane; c < n; c += 32) s += __ldg(cr + c) * sb[c];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            const double s = coarse_row(a.Cinv, sb, n, row, lane);
             if (lane == 0) __stcg(v.x + row, (float)s);
         }
         MG_TAIL_SYNC

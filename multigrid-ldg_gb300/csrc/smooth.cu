@@ -11,11 +11,11 @@
 // therefore depends only on its earlier neighbours; rows are grouped into
 // level sets (level(i) = 1 + max level of its earlier neighbours) and the
 // rows of one level are independent.  One persistent cooperative launch
-// covers a sweep: warps take rows in level order (static round-robin), read
+// covers a pass of consecutive sweeps: warps take rows in level order, read
 // the later neighbours (their old values are stable until row i publishes,
-// because each of them waits for row i), then wait on a per-row completion
-// flag of each earlier neighbour, finish the row and publish it with a
-// release store.  Every wait is bounded (about one second of %globaltimer);
+// because each of them waits for row i), wait for the earlier neighbours'
+// published values, finish the row and publish it; blocks of up to 16 in tiles
+// of rows per CTA (k_gs_tiles), 25 and 27 row by row (k_gs_pass).  Every wait is bounded (about one second of %globaltimer);
 // on expiry the kernel records an error word, every other waiter gives up,
 // and the host returns MGLDG_ERR_TIMEOUT with the context still usable.
 // The sweep counter lives in device memory and is advanced by the last CTA
@@ -135,9 +135,8 @@ __device__ __forceinline__ bool read_row(const unsigned long long* xp, int j, un
             }
         }
         if (__all_sync(0xffffffffu, ok)) return true;
-        ++it;
-        if (it == 1) t0 = globaltimer_ns();
-        if ((it & 15u) == 0) {
+        if ((++it & 15u) == 0) {
+            if (it == 16) t0 = globaltimer_ns();
             bool stop = *(volatile unsigned*)&sync->err != 0;
             if (!stop && (int64_t)(globaltimer_ns() - t0) > timeout_ns) {
                 atomicOr(&sync->err, 1u);
@@ -188,9 +187,8 @@ __device__ __forceinline__ bool poll_rows(const unsigned long long* xp, const in
             }
         pending = still;
         if (!pending) return true;
-        ++it;
-        if (it == 1) t0 = globaltimer_ns();
-        if ((it & 15u) == 0) {
+        if ((++it & 15u) == 0) {
+            if (it == 16) t0 = globaltimer_ns();
             bool stop = *(volatile unsigned*)&sync->err != 0;
             if (!stop && (int64_t)(globaltimer_ns() - t0) > timeout_ns) {
                 atomicOr(&sync->err, 1u);
@@ -413,6 +411,415 @@ __global__ void __launch_bounds__(WPB * 32)
     }
 }
 
+// ------------------------------------------------- GS pass, tiles of rows --
+// The same pass for blocks of up to 16 with most of its dependency chain
+// inside SMs.  A pass is a chain of level sets (511 for one sweep of a
+// 256 x 256 grid); through L2 each of its steps costs a store's way there and
+// a poll's way back, about 1,900 cycles with the arithmetic.  Here kGsTile
+// consecutive rows of one sweep -- a compact patch in the space-filling orders
+// of the meshes -- go to one CTA, which also publishes its rows in a ring in
+// shared memory; a row waits there for its own CTA's rows and only for the
+// others in L2.  A step inside a CTA takes 770 cycles in FP32 (16 x 16
+// blocks), 1,400 in FP64 (9 x 9; ten dependent FP64 operations).
+//
+// A CTA's items are dealt to its warps in level order, so every wait is for
+// an item that an earlier or concurrent warp holds.  What a row needs besides
+// its neighbours' values is copied to shared memory while the warp's previous
+// row waits (item records three items ahead, columns two, blocks one): loading
+// it row by row held a warp for 5,000 cycles, longer than the steps it has to
+// spare.  Keeping the blocks in registers instead made the code long straight
+// lines per neighbour slot (26.6 ms for the 256 x 256 mixed solve below).
+//
+// 256 x 256, 16 x 16 blocks FP32, two sweeps: 514 -> 344 us; 64 x 64, 9 x 9
+// FP64: 223 -> 153 us; 15.7k triangles, 6 x 6 FP32: 447 -> 223 us.  Solve of
+// the 256 x 256 grid 33.0 -> 23.5 ms.
+//
+// Two consecutive rows may be of different tiles and a tile's rows of
+// different levels: the ring's slots carry the item's number in the CTA, and a
+// reader that finds its slot taken by a later item reads the row from L2.
+constexpr unsigned kGsRing = 64;
+
+// Rows that go to one CTA: 4 x 4 patches, whose diagonals have a row for each
+// of the SM's warp schedulers (8 x 8: 858 us instead of 449 for the 256 x 256
+// pass; 2 x 2: 382 against 344).  FP64 blocks of 16 are bound by the SM's FP64
+// pipes, which a patch's rows share: 2 x 2 (219 us against 233 for 64 x 64).
+template <class T, int B>
+constexpr int kGsTile = sizeof(T) == 8 && B == 16 ? 4 : 16;
+
+__device__ __forceinline__ void lds_pair(const unsigned long long* p, unsigned long long& a, unsigned long long& b) {
+    asm volatile("ld.relaxed.cta.shared.v2.b64 {%0, %1}, [%2];"
+                 : "=l"(a), "=l"(b)
+                 : "r"((unsigned)__cvta_generic_to_shared(p))
+                 : "memory");
+}
+__device__ __forceinline__ unsigned long long lds_word(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.cta.shared.b64 %0, [%1];" : "=l"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+    return v;
+}
+__device__ __forceinline__ void sts_word(unsigned long long* p, unsigned long long v) {
+    asm volatile("st.relaxed.cta.shared.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "l"(v) : "memory");
+}
+
+// The lane's CH entries, starting at c0, of a row published in shared memory
+// with `tag`; polls until they carry it.  Warp-uniform result: 0 read, 1 the
+// slot has passed to a later row (the value is in global memory), 2 gave up.
+template <class T, int B, int CH>
+__device__ __forceinline__ int poll_local(const unsigned long long* row, int c0, unsigned tag, T (&xv)[CH],
+                                          GsSync* sync, int64_t timeout_ns) {
+    constexpr int WPV = Packed<T>::WPV, NW = CH * WPV;
+    constexpr bool FULL = WL<B, B>::S * CH == B;
+    const unsigned long long* p = row + c0 * WPV;
+    uint64_t t0 = 0;
+    unsigned it = 0;
+    while (true) {
+        unsigned long long u[NW];
+        if constexpr (NW % 2 == 0) {
+#pragma unroll
+            for (int w = 0; w < NW; w += 2) lds_pair(p + w, u[w], u[w + 1]);
+        } else {
+#pragma unroll
+            for (int w = 0; w < NW; ++w) u[w] = lds_word(p + w);
+        }
+        unsigned diff[2] = {0u, 0u};
+#pragma unroll
+        for (int w = 0; w < NW; ++w)
+            if (FULL || c0 + w / WPV < B) diff[w & 1] |= (unsigned)(u[w] >> 32) ^ tag;
+        if (__all_sync(0xffffffffu, (diff[0] | diff[1]) == 0)) {
+#pragma unroll
+            for (int c = 0; c < CH; ++c) {
+                if constexpr (sizeof(T) == 4) xv[c] = __uint_as_float((unsigned)u[c]);
+                else xv[c] = __hiloint2double((int)(unsigned)u[2 * c], (int)(unsigned)u[2 * c + 1]);
+            }
+            return 0;
+        }
+        const bool later = (FULL || c0 < B) && (int)((unsigned)(u[0] >> 32) - tag) > 0;
+        if (__any_sync(0xffffffffu, later)) return 1;
+        if ((++it & 255u) == 0) {
+            if (it == 256u) t0 = globaltimer_ns();
+            bool stop = *(volatile unsigned*)&sync->err != 0;
+            if (!stop && (int64_t)(globaltimer_ns() - t0) > timeout_ns) {
+                atomicOr(&sync->err, 1u);
+                stop = true;
+            }
+            if (__any_sync(0xffffffffu, stop)) return 2;
+        }
+    }
+}
+
+// Copies nbytes from global to shared memory by one warp (asynchronous, CP
+// bytes per lane and step; both sides CP-aligned).
+template <int CP>
+__device__ __forceinline__ void warp_copy(void* dst, const void* src, int nbytes, int lane) {
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const char* g = reinterpret_cast<const char*>(src);
+    for (int o = lane * CP; o < nbytes; o += 32 * CP) {
+        if constexpr (CP == 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + o), "l"(g + o) : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d + o), "l"(g + o), "n"(CP) : "memory");
+    }
+}
+
+// Sizes of the tile kernel: blocks of a row kept in shared memory (two rows
+// per warp, the one in work and the next), warps per CTA.
+template <class T, int B>
+struct GsTile {
+    using L = WL<B, B>;
+    static constexpr int BB = B * B;
+    static constexpr int WPV = Packed<T>::WPV, W = B * WPV;
+    static constexpr int XL = L::S * L::CH;                        // entries of a staged row
+    static constexpr int LDW = (XL * WPV + 1) / 2 * 2;             // words of a ring row
+    static constexpr int MAXB = B == 16 ? 5 : 8;
+    static constexpr int NR = 4;                                   // rows gathered at a time
+    static constexpr int KW = (NR * W + 31) / 32;
+    static constexpr int BUF = ((MAXB + 1) * BB * (int)sizeof(T) + 15) / 16 * 16;
+    static constexpr int STAGE = (NR * XL * (int)sizeof(T) + 15) / 16 * 16;
+    static constexpr int PER_WARP = 2 * BUF + STAGE;
+    static constexpr int RING = (int)kGsRing * LDW * 8;
+    static constexpr int WPB = RING + 16 * PER_WARP <= 220 * 1024 ? 16 : (RING + 12 * PER_WARP <= 220 * 1024 ? 12 : 8);
+    static constexpr int SMEM = RING + WPB * PER_WARP;
+    static constexpr int CP = BB * (int)sizeof(T) % 16 == 0 ? 16 : (BB * (int)sizeof(T) % 8 == 0 ? 8 : 4);
+};
+
+// Gathers nr <= NR rows into the warp's stage: row q is jl's lane t_q (byte q
+// of tp; 0xff: row i itself).  plain: from the vector x; else from the packed
+// rows, once every word carries an epoch at or after tgt.  Warp-uniform
+// result: false if the wait ran out or another waiter gave up.
+template <class T, int B>
+__device__ __forceinline__ bool gather_rows(const unsigned long long* xp, const T* x, bool plain, unsigned tgt,
+                                            unsigned tp, int nr, int i, int jl, T* stage, GsSync* sync,
+                                            int64_t timeout_ns, int lane) {
+    using G = GsTile<T, B>;
+    constexpr int KW = G::KW, W = G::W, WPV = G::WPV;
+    size_t at[KW];
+    unsigned v[KW];
+#pragma unroll
+    for (int k = 0; k < KW; ++k) {
+        const int w = lane + 32 * k, q = w / W;
+        const int t = (int)((tp >> (8 * (q & 3))) & 0xffu);
+        const int j = __shfl_sync(0xffffffffu, jl, t & 31);
+        at[k] = (size_t)(t == 0xff ? i : j) * W + (w - q * W);
+        v[k] = 0;
+    }
+    const int n = nr * W;
+    if (plain) {
+        // hi and lo halves of an FP64 entry are in the packed order
+#pragma unroll
+        for (int k = 0; k < KW; ++k)
+            if (lane + 32 * k < n) v[k] = __ldcg(reinterpret_cast<const unsigned*>(x) + (WPV == 2 ? at[k] ^ 1u : at[k]));
+    } else {
+        uint64_t t0 = 0;
+        unsigned it = 0;
+        while (true) {
+            bool ok = true;
+            unsigned long long u[KW];
+#pragma unroll
+            for (int k = 0; k < KW; ++k) u[k] = lane + 32 * k < n ? ld_relaxed_u64(xp + at[k]) : (unsigned long long)tgt << 32;
+#pragma unroll
+            for (int k = 0; k < KW; ++k) {
+                v[k] = (unsigned)u[k];
+                ok = ok && (int)((unsigned)(u[k] >> 32) - tgt) >= 0;
+            }
+            if (__all_sync(0xffffffffu, ok)) break;
+            if ((++it & 15u) == 0) {
+                if (it == 16u) t0 = globaltimer_ns();
+                bool stop = *(volatile unsigned*)&sync->err != 0;
+                if (!stop && (int64_t)(globaltimer_ns() - t0) > timeout_ns) {
+                    atomicOr(&sync->err, 1u);
+                    stop = true;
+                }
+                if (__any_sync(0xffffffffu, stop)) return false;
+            }
+        }
+    }
+    __syncwarp();
+    unsigned* st = reinterpret_cast<unsigned*>(stage);
+#pragma unroll
+    for (int k = 0; k < KW; ++k) {
+        const int w = lane + 32 * k, q = w / W, e = w - q * W;
+        if (w < n) st[q * (G::XL * WPV) + (WPV == 2 ? e ^ 1 : e)] = v[k];
+    }
+    __syncwarp();
+    return true;
+}
+
+// the lane's part of a block: columns c0 .. of row rr (zero past the last)
+template <class T, int B>
+__device__ __forceinline__ void block_part(const T* a, int rr, int c0, T (&v)[WL<B, B>::CH]) {
+    constexpr int CH = WL<B, B>::CH;
+    constexpr bool FULL = WL<B, B>::S * CH == B;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) v[c] = FULL || c0 + c < B ? a[rr * B + c0 + c] : T(0);
+}
+
+template <class T, int B>
+__global__ void __launch_bounds__(GsTile<T, B>::WPB * 32, 1)
+    k_gs_tiles(const int* __restrict__ cta_ptr, const int4* __restrict__ items, const int* __restrict__ ltag,
+               int64_t nnzb, int nsw, const int* __restrict__ col_idx, const T* __restrict__ val,
+               const T* __restrict__ Dinv, const T* __restrict__ b, T* x, unsigned long long* xp,
+               const int* __restrict__ xptr, const int* __restrict__ xidx, GsSync* sync, T omega, int reverse,
+               int64_t timeout_ns) {
+    using G = GsTile<T, B>;
+    using L = WL<B, B>;
+    constexpr int CH = L::CH, BB = G::BB, WPV = G::WPV, WPB = G::WPB;
+    constexpr bool FULL = L::S * CH == B;
+    constexpr unsigned ALL = 0xffffffffu;
+    extern __shared__ __align__(16) unsigned char smem[];
+    unsigned long long* ring = reinterpret_cast<unsigned long long*>(smem);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned char* mine = smem + G::RING + warp * G::PER_WARP;
+    T* stage = reinterpret_cast<T*>(mine + 2 * G::BUF);
+    const int r = lane / L::S, sl = lane - r * L::S;
+    const bool active = B * L::S == 32 || r < B;
+    const bool first = active && sl == 0;
+    const int rr = active ? r : 0;
+    const int c0 = sl * CH;
+    for (int q = threadIdx.x; q < (int)kGsRing * G::LDW; q += WPB * 32) ring[q] = 0;
+    for (int q = lane; q < G::NR * G::XL; q += 32) stage[q] = T(0);
+    const unsigned base = __ldcg(&sync->epoch);
+    __syncthreads();
+    const int w0 = __ldg(cta_ptr + blockIdx.x), w1 = __ldg(cta_ptr + blockIdx.x + 1);
+    // records are loaded three items ahead, columns two, blocks one
+    const int4 none = make_int4(-1, 0, 0, 0);
+    auto record = [&](int w) { return w < w1 ? __ldg(items + w) : none; };
+    auto columns = [&](const int4& it, int& jl, int& tl) {
+        jl = lane < it.z ? __ldg(col_idx + it.y + lane) : -1;
+        tl = lane < it.z ? __ldg(ltag + (it.x & 7) * nnzb + it.y + lane) : 0;
+    };
+    T bn = 0, xn0 = 0;
+    auto blocks = [&](const int4& it, int buf) {
+        if (it.x < 0) return;
+        T* d = reinterpret_cast<T*>(mine + buf * G::BUF);
+        const int i = it.x >> 3;
+        warp_copy<G::CP>(d, Dinv + (size_t)i * BB, BB * (int)sizeof(T), lane);
+        warp_copy<G::CP>(d + BB, val + (size_t)it.y * BB, min(it.z, G::MAXB) * BB * (int)sizeof(T), lane);
+    };
+    auto vectors = [&](const int4& it) {
+        bn = xn0 = 0;
+        if (first && it.x >= 0) {
+            const size_t o = (size_t)(it.x >> 3) * B + r;
+            bn = __ldg(b + o);
+            if ((it.x & 7) == 0) xn0 = __ldcg(x + o);
+        }
+    };
+    int4 it = record(w0 + warp), it1 = record(w0 + warp + WPB), it2 = record(w0 + warp + 2 * WPB);
+    int jl, tl, jl1, tl1;
+    columns(it, jl, tl);
+    columns(it1, jl1, tl1);
+    blocks(it, 0);
+    vectors(it);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    int pb = 0;
+    for (int w = w0 + warp; w < w1; w += WPB, pb ^= 1) {
+        const int i = it.x >> 3, s = it.x & 7, k0 = it.y, nk = it.z;
+        const unsigned tgt_new = base + (unsigned)s + 1u;   // this sweep's values
+        const unsigned tgt_old = base + (unsigned)s;        // the previous sweep's values
+        T acc = bn, xi = xn0;
+        __syncwarp();
+        blocks(it1, pb ^ 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        vectors(it1);
+        int jl2, tl2;
+        columns(it2, jl2, tl2);
+        const int4 it3 = record(w + 3 * WPB);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const T* buf = reinterpret_cast<const T*>(mine + pb * G::BUF);
+        // ---- work that does not depend on the pass's progress ----
+        T dch[CH];
+#pragma unroll
+        for (int c = 0; c < CH; ++c) dch[c] = active && (FULL || c0 + c < B) ? buf[rr * B + c0 + c] : T(0);
+        const unsigned nb = __ballot_sync(ALL, lane < nk && jl != i);
+        const unsigned early = __ballot_sync(ALL, reverse ? jl > i : jl < i) & nb;
+        unsigned own = __ballot_sync(ALL, tl != 0) & early;
+        bool failed = false;
+        // the blocks of the rows in sel times their values at version tgt,
+        // up to NR rows per L2 round trip, in column order
+        auto others = [&](unsigned sel, bool self, bool plain, unsigned tgt) {
+            while ((sel || self) && !failed) {
+                unsigned tp = 0;
+                int nr = 0;
+                if (self) {
+                    tp = 0xffu;
+                    nr = 1;
+                }
+                while (nr < G::NR && sel) {
+                    tp |= (unsigned)(__ffs(sel) - 1) << (8 * nr++);
+                    sel &= sel - 1;
+                }
+                if (!gather_rows<T, B>(xp, x, plain, tgt, tp, nr, i, jl, stage, sync, timeout_ns, lane)) {
+                    failed = true;
+                    return;
+                }
+#pragma unroll 1
+                for (int q = 0; q < nr; ++q) {
+                    const int t = (int)((tp >> (8 * q)) & 0xffu);
+                    if (t == 0xff) {
+                        if (first) xi = stage[r];
+                        continue;
+                    }
+                    T av[CH];
+                    if (t < G::MAXB) block_part<T, B>(buf + (t + 1) * BB, rr, c0, av);
+                    else block_part<T, B>(val + (size_t)(k0 + t) * BB, rr, c0, av);
+#pragma unroll
+                    for (int c = 0; c < CH; ++c) acc = fma(-av[c], stage[q * G::XL + c0 + c], acc);
+                }
+                self = false;
+            }
+        };
+        // neighbours of the symmetrised pattern outside the row's own
+        // pattern: waited for without reading
+        if (it.w) {
+            const int e0 = __ldg(xptr + i), e1 = __ldg(xptr + i + 1);
+            for (int q = e0; q < e1 && !failed; ++q) {
+                const int j = __ldg(xidx + q);
+                const bool earlier = reverse ? (j > i) : (j < i);
+                if (!earlier && s == 0) continue;
+                if (!gather_rows<T, B>(xp, x, false, earlier ? tgt_new : tgt_old, 0u, 1, i, j, stage, sync, timeout_ns,
+                                       lane))
+                    failed = true;
+            }
+        }
+        // blocks past the 32 columns held by the lanes, one at a time
+        for (int t = 32; t < nk && !failed; ++t) {
+            const int j = __ldg(col_idx + k0 + t);
+            if (j == i) continue;
+            const bool earlier = reverse ? (j > i) : (j < i);
+            if (!gather_rows<T, B>(xp, x, !earlier && s == 0, earlier ? tgt_new : tgt_old, 0u, 1, i, j, stage, sync,
+                                   timeout_ns, lane)) {
+                failed = true;
+                break;
+            }
+            T av[CH];
+            block_part<T, B>(val + (size_t)(k0 + t) * BB, rr, c0, av);
+#pragma unroll
+            for (int c = 0; c < CH; ++c) acc = fma(-av[c], stage[c0 + c], acc);
+        }
+        // later neighbours and the row itself (the previous sweep's values),
+        // then the earlier neighbours of other CTAs, then this CTA's
+        others(nb & ~early, s > 0, s == 0, tgt_old);
+        const T xs = (T(1) - omega) * xi;
+        others(early & ~own, false, false, tgt_new);
+#pragma unroll 1
+        while (own && !failed) {
+            const int t = __ffs(own) - 1;
+            own &= own - 1;
+            const unsigned tag = (unsigned)__shfl_sync(ALL, tl, t);
+            T av[CH], xv[CH];
+            if (t < G::MAXB) block_part<T, B>(buf + (t + 1) * BB, rr, c0, av);
+            else block_part<T, B>(val + (size_t)(k0 + t) * BB, rr, c0, av);
+            const int st = poll_local<T, B, CH>(ring + ((tag - 1u) & (kGsRing - 1u)) * G::LDW, c0, tag, xv, sync,
+                                                timeout_ns);
+            if (st == 0) {
+#pragma unroll
+                for (int c = 0; c < CH; ++c) acc = fma(-av[c], xv[c], acc);
+            } else if (st == 1) {
+                others(1u << t, false, false, tgt_new);
+            } else {
+                failed = true;
+            }
+        }
+        if (failed) break;
+        // x_i + omega (Dinv_i t - x_i), t = b_i - sum_{j != i} A_ij x_j
+        const T tt = seg_sum<L::S>(acc);
+        T y = 0;
+#pragma unroll
+        for (int c = 0; c < CH; ++c) {
+            const T tc = __shfl_sync(ALL, tt, ((c0 + c) * L::S) & 31);
+            y = fma(dch[c], FULL || c0 + c < B ? tc : T(0), y);
+        }
+        const T xn = fma(omega, seg_sum<L::S>(y), xs);
+        if (first) {
+            const unsigned seq = (unsigned)(w - w0);
+            unsigned long long* so = ring + (seq & (kGsRing - 1u)) * G::LDW + r * WPV;
+            const unsigned long long hi = (unsigned long long)(seq + 1u) << 32;
+            if constexpr (sizeof(T) == 4) {
+                sts_word(so, hi | __float_as_uint(xn));
+            } else {
+                sts_word(so, hi | (unsigned)__double2hiint(xn));
+                sts_word(so + 1, hi | (unsigned)__double2loint(xn));
+            }
+            publish<T>(xp, (size_t)i * B + r, xn, tgt_new);
+            if (s == nsw - 1) x[(size_t)i * B + r] = xn;
+        }
+        it = it1; it1 = it2; it2 = it3;
+        jl = jl1; tl = tl1; jl1 = jl2; tl1 = tl2;
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    // the last CTA to finish advances the epoch past this pass
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned prev = atomicAdd(&sync->done, 1u);
+        if (prev == gridDim.x - 1) {
+            sync->done = 0;
+            __threadfence();
+            atomicExch(&sync->epoch, base + (unsigned)nsw);
+        }
+    }
+}
+
 // ------------------------------------------------------------ Jacobi sweep --
 // x_out_i = x_in_i + omega * Dinv_i (b_i - sum_j A_ij x_in_j)
 //
@@ -601,12 +1008,14 @@ void sched_build(mgldg_ctx* ctx, const mgldg_bsr* A, Sched& S) {
     symmetrised_neighbours(n, A->h_row_ptr.data(), A->h_col_idx.data(), S.nb);
     // neighbours j of i with A_ji stored but not A_ij: waited for, not read
     std::vector<int> xp_(n + 1, 0), xi;
+    S.xcount.assign(n, 0);
     for (int i = 0; i < n; ++i) {
         const int* c0 = A->h_col_idx.data() + A->h_row_ptr[i];
         const int* c1 = A->h_col_idx.data() + A->h_row_ptr[i + 1];
         for (int j : S.nb[i])
             if (std::find(c0, c1, j) == c1) xi.push_back(j);
         xp_[i + 1] = (int)xi.size();
+        S.xcount[i] = xp_[i + 1] - xp_[i];
     }
     S.xptr = dalloc<int>(n + 1);
     S.xidx = dalloc<int>(std::max<size_t>(1, xi.size()));
@@ -623,22 +1032,25 @@ void sched_build(mgldg_ctx* ctx, const mgldg_bsr* A, Sched& S) {
 static int gs_pass_levels_host(int n, const std::vector<std::vector<int>>& nb, int dir, int nsw, std::vector<int>& lev) {
     lev.assign((size_t)nsw * n, 0);
     int maxlev = -1;
-    for (int s = 0; s < nsw; ++s)
+    for (int s = 0; s < nsw; ++s) {
+        int* cur = lev.data() + (size_t)s * n;
+        const int* old = s > 0 ? cur - n : nullptr;
         for (int t = 0; t < n; ++t) {
             const int i = dir == 0 ? t : n - 1 - t;
-            int l = s > 0 ? lev[(size_t)(s - 1) * n + i] + 1 : 0;
+            int l = old ? old[i] + 1 : 0;
             for (int j : nb[i]) {
                 const bool earlier = dir == 0 ? (j < i) : (j > i);
-                if (earlier) l = std::max(l, lev[(size_t)s * n + j] + 1);
-                else if (s > 0) l = std::max(l, lev[(size_t)(s - 1) * n + j] + 1);
+                if (earlier) l = std::max(l, cur[j] + 1);
+                else if (old) l = std::max(l, old[j] + 1);
             }
-            lev[(size_t)s * n + i] = l;
+            cur[i] = l;
             maxlev = std::max(maxlev, l);
         }
+    }
     return maxlev + 1;
 }
 
-static void pass_build(mgldg_ctx* ctx, Sched& S, int dir, int nsw, GsPass& P) {
+static void pass_build(mgldg_ctx* ctx, Sched& S, int dir, int nsw, int grid, int tile, GsPass& P) {
     const int n = S.n;
     MG_REQUIRE(n < (1 << 28) && nsw >= 1 && nsw <= 7, MGLDG_ERR_UNSUPPORTED, "Gauss-Seidel pass too large");
     std::vector<int> lev;
@@ -655,21 +1067,74 @@ static void pass_build(mgldg_ctx* ctx, Sched& S, int dir, int nsw, GsPass& P) {
         }
     P.nsw = nsw;
     P.dir = dir;
+    P.grid = grid;
+    P.tile = tile;
     P.nitems = nsw * n;
     P.depth = n ? maxlev + 1 : 0;
+    if (grid > 0) {
+        // groups of consecutive rows, one sweep each, go to the CTAs in the
+        // order in which the pass reaches them
+        const int shift = __builtin_ctz((unsigned)tile), ng = (n + tile - 1) >> shift;   // a power of two
+        std::vector<int> owner((size_t)nsw * ng, -1), cnt2(grid + 1, 0);
+        struct Loc { int cta, seq; };
+        std::vector<Loc> loc((size_t)nsw * n);
+        int next = 0;
+        for (int it : items) {
+            const int i = it >> 3, s = it & 7;
+            int& o = owner[(size_t)s * ng + (i >> shift)];
+            if (o < 0) {
+                o = next;
+                next = next + 1 < grid ? next + 1 : 0;
+            }
+            loc[(size_t)s * n + i] = {o, ++cnt2[o + 1]};
+        }
+        for (int c = 0; c < grid; ++c) cnt2[c + 1] += cnt2[c];
+        const int *rp = S.A->h_row_ptr.data(), *ci = S.A->h_col_idx.data();
+        // one array: records, tags per (sweep, block), items per CTA
+        const size_t nrec = std::max<size_t>(1, items.size()), ntag = (size_t)nsw * rp[n];
+        std::vector<int> tab(4 * nrec + ntag + grid + 1, 0);
+        int* ltag = tab.data() + 4 * nrec;
+        for (int s = 0; s < nsw; ++s, ltag += rp[n]) {
+            const Loc* ls = loc.data() + (size_t)s * n;
+            for (int i = 0; i < n; ++i) {
+                const Loc l = ls[i];
+                int* rec = tab.data() + 4 * (size_t)(cnt2[l.cta] + l.seq - 1);
+                rec[0] = (i << 3) | s;
+                rec[1] = rp[i];
+                rec[2] = rp[i + 1] - rp[i];
+                rec[3] = S.xcount[i] ? 1 : 0;
+                for (int k = rp[i]; k < rp[i + 1]; ++k) {
+                    const int j = ci[k];
+                    if ((dir == 0 ? j < i : j > i) && ls[j].cta == l.cta) ltag[k] = ls[j].seq;
+                }
+            }
+        }
+        std::copy(cnt2.begin(), cnt2.end(), tab.end() - (grid + 1));
+        P.items = dalloc<int>(tab.size());
+        upload(ctx, P.items, tab.data(), tab.size());
+        P.rec = reinterpret_cast<int4*>(P.items);
+        P.ltag = P.items + 4 * nrec;
+        P.cta_ptr = P.ltag + ntag;
+        sync(ctx);
+        return;
+    }
     P.items = dalloc<int>(std::max<size_t>(1, items.size()));
     upload(ctx, P.items, items.data(), items.size());
     sync(ctx);
 }
 
-static GsPass& get_pass(mgldg_ctx* ctx, Sched& S, int dir, int nsw) {
+static void pass_free(GsPass& P) {
+    dfree(P.items);
+}
+
+static GsPass& get_pass(mgldg_ctx* ctx, Sched& S, int dir, int nsw, int grid, int tile) {
     for (auto& P : S.passes)
-        if (P.dir == dir && P.nsw == nsw) return P;
+        if (P.dir == dir && P.nsw == nsw && P.grid == grid && P.tile == tile) return P;
     GsPass P;
     try {
-        pass_build(ctx, S, dir, nsw, P);
+        pass_build(ctx, S, dir, nsw, grid, tile, P);
     } catch (...) {
-        dfree(P.items);
+        pass_free(P);
         throw;
     }
     S.passes.push_back(P);
@@ -677,7 +1142,7 @@ static GsPass& get_pass(mgldg_ctx* ctx, Sched& S, int dir, int nsw) {
 }
 
 void sched_free(Sched& S) {
-    for (auto& P : S.passes) dfree(P.items);
+    for (auto& P : S.passes) pass_free(P);
     S.passes.clear();
     dfree(S.xptr);
     dfree(S.xidx);
@@ -704,13 +1169,8 @@ int gs_take_error(mgldg_ctx* ctx, Sched& S) {
     return 0;
 }
 
-template <class T, int B>
-static void launch_gs(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, const T* Dinv, const T* b, T* x, Sched& S,
-                      T omega, bool reverse, int nsw) {
-    constexpr int WPB = 4;
-    constexpr int MAXE = B <= 10 ? 8 : (B <= 16 ? 4 : 1);
-    auto kern = k_gs_pass<T, B, WPB, MAXE>;
-    const int words = B * Packed<T>::WPV;
+// the published rows of a schedule, `words` 64-bit words each
+static void packed_rows(mgldg_ctx* ctx, Sched& S, int words) {
     if (!S.xp || S.words_per_row != words) {
         dfree(S.xp);
         S.xp = nullptr;
@@ -721,7 +1181,48 @@ static void launch_gs(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, const T
         // epochs restart below every word
         MG_CHECK_CUDA(cudaMemsetAsync(S.sync, 0, sizeof(GsSync), ctx->stream));
     }
-    GsPass& P = get_pass(ctx, S, reverse ? 1 : 0, nsw);
+}
+
+template <class T, int B>
+static void launch_gs_tiles(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, const T* Dinv, const T* b, T* x,
+                            Sched& S, T omega, bool reverse, int nsw) {
+    using G = GsTile<T, B>;
+    constexpr int WPB = G::WPB, tile = kGsTile<T, B>;
+    packed_rows(ctx, S, G::W);
+    auto kern = k_gs_tiles<T, B>;
+    MG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM));
+    int per_sm = 0;
+    MG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WPB * 32, G::SMEM));
+    MG_REQUIRE(per_sm > 0, MGLDG_ERR_CUDA, "Gauss-Seidel kernel does not fit on an SM");
+    const int64_t groups = (int64_t)nsw * ((S.n + tile - 1) / tile);
+    const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(groups, (int64_t)per_sm * ctx->sm_count));
+    GsPass& P = get_pass(ctx, S, reverse ? 1 : 0, nsw, grid, tile);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(WPB * 32);
+    cfg.dynamicSmemBytes = G::SMEM;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;   // all CTAs co-resident
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    {
+        Launch L(ctx, MGLDG_K_GS);
+        MG_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const int*)P.cta_ptr, (const int4*)P.rec, (const int*)P.ltag,
+                                         (int64_t)A->h_row_ptr.back(), nsw, (const int*)A->col_idx, vals, Dinv, b, x, S.xp, (const int*)S.xptr, (const int*)S.xidx, S.sync, omega,
+                                         (int)reverse, S.timeout_ns));
+    }
+}
+
+template <class T, int B>
+static void launch_gs(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, const T* Dinv, const T* b, T* x, Sched& S,
+                      T omega, bool reverse, int nsw) {
+    constexpr int WPB = 4;
+    constexpr int MAXE = 1;
+    auto kern = k_gs_pass<T, B, WPB, MAXE>;
+    packed_rows(ctx, S, B * Packed<T>::WPV);
+    GsPass& P = get_pass(ctx, S, reverse ? 1 : 0, nsw, 0, 0);
     int per_sm = 0;
     MG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WPB * 32, 0));
     MG_REQUIRE(per_sm > 0, MGLDG_ERR_CUDA, "Gauss-Seidel kernel does not fit on an SM");
@@ -752,14 +1253,14 @@ void gs_sweeps(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, const T* Dinv,
     while (nsw > 0) {
         const int k = std::min(nsw, 4);
         switch (A->br) {
-            case 1: launch_gs<T, 1>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
-            case 3: launch_gs<T, 3>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
-            case 4: launch_gs<T, 4>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
-            case 6: launch_gs<T, 6>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
-            case 8: launch_gs<T, 8>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
-            case 9: launch_gs<T, 9>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
-            case 10: launch_gs<T, 10>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
-            case 16: launch_gs<T, 16>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
+            case 1: launch_gs_tiles<T, 1>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
+            case 3: launch_gs_tiles<T, 3>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
+            case 4: launch_gs_tiles<T, 4>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
+            case 6: launch_gs_tiles<T, 6>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
+            case 8: launch_gs_tiles<T, 8>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
+            case 9: launch_gs_tiles<T, 9>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
+            case 10: launch_gs_tiles<T, 10>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
+            case 16: launch_gs_tiles<T, 16>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
             case 25: launch_gs<T, 25>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
             case 27: launch_gs<T, 27>(ctx, A, vals, Dinv, b, x, S, omega, reverse, k); break;
             default: throw Error(MGLDG_ERR_UNSUPPORTED, "Gauss-Seidel: unsupported block size");
@@ -878,19 +1379,30 @@ extern "C" int mgldg_selftest_wait_timeout(mgldg_ctx* ctx, int64_t timeout_ns, i
         dinv = dalloc<double>(2); b = dalloc<double>(2); x = dalloc<double>(2);
         upload(ctx, dinv, dv, 2); upload(ctx, b, dv, 2); upload(ctx, x, zero, 2);
         sched_build(ctx, A, S);
-        GsPass P;
-        const int item = (1 << 3) | 0;
-        P.nsw = 1;
-        P.dir = 0;
-        P.nitems = 1;
-        P.depth = 1;
-        P.items = dalloc<int>(1);
-        upload(ctx, P.items, &item, 1);
-        S.passes.push_back(P);
         S.timeout_ns = timeout_ns;
-        gs_sweeps<double>(ctx, A, A->val, dinv, b, x, S, 1.0, false, 1);
-        sync(ctx);
-        *status = gs_take_error(ctx, S) ? MGLDG_ERR_TIMEOUT : MGLDG_OK;
+        *status = MGLDG_ERR_TIMEOUT;
+        // row 0 is never run: row 1 waits for it as another CTA's row (in
+        // global memory), then as its own CTA's (in shared memory)
+        for (int owner = -1; owner <= 0; ++owner) {
+            S.passes.emplace_back();
+            GsPass& P = S.passes.back();
+            const int tab[10] = {(1 << 3) | 0, 2, 2, 0, /* tags */ 0, 0, owner + 1, 0, /* items */ 0, 1};
+            P.nsw = 1;
+            P.nitems = 1;
+            P.depth = 1;
+            P.grid = 1;
+            P.tile = kGsTile<double, 1>;
+            P.items = dalloc<int>(10);
+            P.rec = reinterpret_cast<int4*>(P.items);
+            P.ltag = P.items + 4;
+            P.cta_ptr = P.items + 8;
+            upload(ctx, P.items, tab, 10);
+            gs_sweeps<double>(ctx, A, A->val, dinv, b, x, S, 1.0, false, 1);
+            sync(ctx);
+            if (!gs_take_error(ctx, S)) *status = MGLDG_OK;
+            pass_free(P);
+            S.passes.pop_back();
+        }
         // the context must still work: a plain SpMV
         spmv<double>(ctx, A, 1.0, b, 0.0, nullptr, x);
         sync(ctx);

@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) k_rep_tables(const double* __restrict__ v
     }
     __syncthreads();
     // small blocks are always read by columns
-    const bool cols = B != 16 || __popc(rm) > __popc(cm);
+    const bool cols = B != 16 || __popc(rm) >= __popc(cm);
     using I8 = Img<double, B>;
     using I4 = Img<float, B>;
     fill_image<double, B>(t.i64 + (size_t)u * I8::SIZE, a, cols, 0);
@@ -570,7 +570,7 @@ __device__ __forceinline__ void acc16(const RepArgs<T>& a, const T* simg, const 
             for (int e = 0; e < E; ++e) col[e] = __ldg(cq + 16 * e);
         }
         const T* ab = simg + idk * I::SIZE;
-        if (F16 || __popc(rm) <= __popc(cm)) {
+        if (F16 || __popc(rm) < __popc(cm)) {
             const T sc = F16 ? (T)__ldg(a.scale + idk) : T(0);
 #pragma unroll
             for (int r = 0; r < 16; ++r)
@@ -803,11 +803,14 @@ struct RepDfArgs {
 
 // q = A d in double-float arithmetic, 16 x 16 blocks, two lanes per row: a
 // float-pair sum per row and column half, the two pairs added as in FP64
-// (PairSum), q and the partial d.q in FP64.  Bound by the FP32 pipes (11 operations per
-// product; the zero block rows and columns are skipped), then by the FP64
-// ones: adding the halves as float pairs and widening without conversions
-// leaves three FP64 operations per entry instead of eight.
-__global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
+// (PairSum), q and the partial d.q in FP64.  Blocks read by columns take two
+// rows at a time (packed FP32 operations).  Bound by the FP32 pipes (11
+// operations per product, zero block rows and columns skipped; 46 % busy) and
+// the FP64 ones (three operations per entry; adding the halves as float pairs
+// and widening without conversions took away five more; 30 %).  262,144 rows:
+// 122 us with four CTAs an SM and x loaded a block ahead, 110 us with five and
+// without.
+__global__ void __launch_bounds__(128, 5) k_rep16_df64(const RepDfArgs a) {
     using I = Img<float, 16>;
     extern __shared__ __align__(16) unsigned char smraw[];
     float* sh_ = reinterpret_cast<float*>(smraw);
@@ -821,44 +824,38 @@ __global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
         const int* cls = a.cls + (size_t)__ldg(a.gcls + w) * kRepCls;
         const int nb = __ldg(cls);
         const int* cp = a.cols + slot;
-        float sh[16], sl[16], nh[8], nl[8];
+        unsigned long long sh[8], sl[8];   // rows 2 r, 2 r + 1
 #pragma unroll
-        for (int r = 0; r < 16; ++r) sh[r] = sl[r] = 0.f;
-        {
-            const size_t xo = (size_t)__ldg(cp) * 16 + 8 * half;
-            ldg<8>(a.xh + xo, nh);
-            ldg<8>(a.xl + xo, nl);
-        }
-        int col = nb > 1 ? __ldg(cp + a.nslots) : 0;
+        for (int r = 0; r < 8; ++r) sh[r] = sl[r] = 0ULL;
+        int col = __ldg(cp);
         int id = __ldg(cls + 4);
         unsigned m = (unsigned)__ldg(cls + 4 + kRepMaxNb);
 #pragma unroll 1
         for (int k = 0; k < nb; ++k) {
             float xh[8], xl[8];
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-                xh[c] = nh[c];
-                xl[c] = nl[c];
-            }
+            const size_t xo = (size_t)col * 16 + 8 * half;
+            ldg<8>(a.xh + xo, xh);
+            ldg<8>(a.xl + xo, xl);
             const unsigned rm = m & 0xffffu, cm = m >> 16;
             const int bo = id * I::SIZE;
             if (k + 1 < nb) {
-                const size_t xo = (size_t)col * 16 + 8 * half;
-                ldg<8>(a.xh + xo, nh);
-                ldg<8>(a.xl + xo, nl);
+                col = __ldg(cp + (size_t)(k + 1) * a.nslots);
                 id = __ldg(cls + 5 + k);
                 m = (unsigned)__ldg(cls + 5 + kRepMaxNb + k);
             }
-            if (k + 2 < nb) col = __ldg(cp + (size_t)(k + 2) * a.nslots);
-            if (__popc(rm) <= __popc(cm)) {
+            if (__popc(rm) < __popc(cm)) {
 #pragma unroll
                 for (int r = 0; r < 16; ++r)
                     if ((rm >> r) & 1u) {
                         float ah[8], al[8];
                         lds<8>(sh_ + bo + I::line(r) + 8 * half, ah);
                         lds<8>(sl_ + bo + I::line(r) + 8 * half, al);
+                        float2 h = unpack2(sh[r / 2]), l = unpack2(sl[r / 2]);
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) df_fma(sh[r], sl[r], ah[c], al[c], xh[c], xl[c]);
+                        for (int c = 0; c < 8; ++c)
+                            df_fma(r & 1 ? h.y : h.x, r & 1 ? l.y : l.x, ah[c], al[c], xh[c], xl[c]);
+                        sh[r / 2] = pack2(h.x, h.y);
+                        sl[r / 2] = pack2(l.x, l.y);
                     }
             } else {
                 const unsigned any = cm | (cm >> 8);
@@ -869,8 +866,12 @@ __global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
                         float ah[16], al[16];
                         lds<16>(sh_ + co + c * 16, ah);
                         lds<16>(sl_ + co + c * 16, al);
+                        const unsigned long long d2 = pack2(xh[c], xh[c]), n2 = pack2(-xh[c], -xh[c]),
+                                                 e2 = pack2(xl[c], xl[c]);
 #pragma unroll
-                        for (int r = 0; r < 16; ++r) df_fma(sh[r], sl[r], ah[r], al[r], xh[c], xl[c]);
+                        for (int r = 0; r < 8; ++r)
+                            df_fma2(sh[r], sl[r], pack2(ah[2 * r], ah[2 * r + 1]), pack2(al[2 * r], al[2 * r + 1]), d2,
+                                    n2, e2);
                     }
             }
         }
@@ -880,9 +881,13 @@ __global__ void __launch_bounds__(128) k_rep16_df64(const RepDfArgs a) {
         ldg<8>(a.d + o, dv);
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
-            const float oh = __shfl_xor_sync(0xffffffffu, half ? sh[r] : sh[r + 8], 1);
-            const float ol = __shfl_xor_sync(0xffffffffu, half ? sl[r] : sl[r + 8], 1);
-            const float mh = half ? sh[r + 8] : sh[r], ml = half ? sl[r + 8] : sl[r];
+            const float2 h0 = unpack2(sh[r / 2]), h1 = unpack2(sh[r / 2 + 4]);
+            const float2 l0 = unpack2(sl[r / 2]), l1 = unpack2(sl[r / 2 + 4]);
+            const float ha = r & 1 ? h0.y : h0.x, hb = r & 1 ? h1.y : h1.x;
+            const float la = r & 1 ? l0.y : l0.x, lb = r & 1 ? l1.y : l1.x;
+            const float oh = __shfl_xor_sync(0xffffffffu, half ? ha : hb, 1);
+            const float ol = __shfl_xor_sync(0xffffffffu, half ? la : lb, 1);
+            const float mh = half ? hb : ha, ml = half ? lb : la;
             PairSum v{mh, ml};
             v.add(oh, ol);
             qv[r] = v.value();

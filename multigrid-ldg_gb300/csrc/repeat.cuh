@@ -12,7 +12,7 @@ namespace mg {
 // to a group, so that a warp applies one block to many rows at once.
 //
 // Images: the value tables as the kernels hold them in shared memory, first
-// the nuniq blocks (by rows, or by columns where fewer columns than rows hold
+// the nuniq blocks (by columns, or by rows where fewer rows than columns hold
 // nonzeros), then the ndiag distinct inverse diagonal blocks (by rows); a
 // block is b lines of ld values, for b = 16 with 16 bytes between lines 7 and
 // 8 (the two column halves of a line pair then lie in different banks).

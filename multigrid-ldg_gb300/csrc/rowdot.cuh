@@ -76,12 +76,12 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-// (nah = -ah: the product enters the two-sum with its sign turned, so nothing
+// (ndh = -dh: the product enters the two-sum with its sign turned, so nothing
 // is negated per product)
 __device__ __forceinline__ void df_fma2(unsigned long long& sh, unsigned long long& sl, unsigned long long ah,
-                                        unsigned long long nah, unsigned long long al, unsigned long long dh,
+                                        unsigned long long al, unsigned long long dh, unsigned long long ndh,
                                         unsigned long long dl) {
-    const unsigned long long np = mul2(nah, dh);
+    const unsigned long long np = mul2(ah, ndh);
     const unsigned long long t = fma2(ah, dl, fma2(al, dh, fma2(ah, dh, np)));
     const unsigned long long s = sub2(sh, np);
     const unsigned long long bb = sub2(s, sh);

@@ -249,11 +249,10 @@ __global__ void __launch_bounds__(128) k_spmm_rep_df64(MMArgs<float> a, const fl
 #pragma unroll
                         for (int r = 0; r < NP; ++r) {
                             const u64 a2 = pack2(ah[2 * r], ah[2 * r + 1]), b2 = pack2(al[2 * r], al[2 * r + 1]);
-                            const u64 n2 = a2 ^ 0x8000000080000000ULL;
 #pragma unroll
                             for (int v = 0; v < V; ++v)
-                                df_fma2(sh[r][v], sl[r][v], a2, n2, b2, pack2(xh[d][v], xh[d][v]),
-                                        pack2(xl[d][v], xl[d][v]));
+                                df_fma2(sh[r][v], sl[r][v], a2, b2, pack2(xh[d][v], xh[d][v]),
+                                        pack2(-xh[d][v], -xh[d][v]), pack2(xl[d][v], xl[d][v]));
                         }
                     }
             }

@@ -9,7 +9,7 @@
 // shared memory, a product moves its vectors and indices only, and all-zero
 // block rows (or columns) are skipped.  Level 0 of 512 x 512 Q3, event times
 // before and after: FP32 sweeps (three full, one from x = 0) 213 -> 36 us on
-// average, FP32 residual 240 -> 34 us, double-float product 410 -> 147 us;
+// average, FP32 residual 240 -> 34 us, double-float product 410 -> 110 us;
 // 256 x 256 Q3 FP64 sweeps 174 -> 105 us, residual 185 -> 90 us.  What is
 // left: vector traffic and shared-memory reads (FP32), the FP64 pipes (FP64
 // and the conversions of the double-float product).
@@ -17,7 +17,8 @@
 // Mapping: the rows are sorted by class (same sequence of table entries) and
 // a warp's rows belong to one class, so a block value read once from shared
 // memory serves all of them.  16 x 16 blocks: two lanes per row, one per
-// column half, E = 1 or 2 rows per lane pair; smaller blocks: one lane per row.  The sums run in the general kernels' order (16 x 16: the two column
+// column half, E = 1 or 2 rows per lane pair; smaller blocks: one lane per
+// row.  The sums run in the general kernels' order (16 x 16: the two column
 // halves in block order, then their sum; smaller blocks: one sum per column
 // over the blocks, then the columns), and a skipped product is one with a
 // zero block entry, so for finite vectors the results are the general

@@ -15,7 +15,8 @@
 // the later neighbours (their old values are stable until row i publishes,
 // because each of them waits for row i), wait for the earlier neighbours'
 // published values, finish the row and publish it; blocks of up to 16 in tiles
-// of rows per CTA (k_gs_tiles), 25 and 27 row by row (k_gs_pass).  Every wait is bounded (about one second of %globaltimer);
+// of rows per CTA (k_gs_tiles), 25 and 27 row by row (k_gs_pass).  Every wait
+// is bounded (about one second of %globaltimer);
 // on expiry the kernel records an error word, every other waiter gives up,
 // and the host returns MGLDG_ERR_TIMEOUT with the context still usable.
 // The sweep counter lives in device memory and is advanced by the last CTA

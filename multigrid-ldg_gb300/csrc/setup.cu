@@ -16,6 +16,8 @@
 #include <chrono>
 #include <numeric>
 
+#include <cooperative_groups.h>
+
 #include "api.cuh"
 #include "plan.cuh"
 
@@ -474,60 +476,103 @@ __global__ void k_identity_right(int n, double* aug) {
         for (int c = threadIdx.x; c < n; c += blockDim.x) aug[(size_t)r * 2 * n + n + c] = (r == c) ? 1.0 : 0.0;
 }
 
-// Gauss-Jordan on [A | I] with partial pivoting; one CTA of 1024 threads.
-__global__ void __launch_bounds__(1024) k_gauss_jordan(int n, double* aug, int* status) {
-    __shared__ double sv[32];
-    __shared__ int si[32];
-    __shared__ int piv;
-    __shared__ double pinv;
-    const int w2 = 2 * n;
+// Gauss-Jordan with partial pivoting, the matrix in the shared memory of one
+// cluster: CTA q holds columns q, q + 8, ...  Step k is bound by its latency:
+// the owner of column k picks the pivot row and writes it and the factors to
+// every CTA, one cluster barrier, then each CTA eliminates its columns.  The
+// inverse is built in place: once row k has been a pivot row, slot k holds the
+// column of the inverse that row k's unit vector has become (perm), so a step
+// touches n columns of [A | I], not 2 n; every entry gets the operations that
+// the elimination of [A | I] gives it.  The
+// coarsest level of a 64 x 64 Q2 hierarchy (144 unknowns, allocations and all):
+// 2.1 -> 0.6 ms against a pair of launches per pivot.  Up to kGjMaxN the matrix
+// fits the shared memory of eight SMs; beyond it the pairs of launches below
+// run over all SMs.
+constexpr int kGjCtas = 8;
+constexpr int kGjMaxN = 448;   // 8 x 211 KB
+
+__host__ __device__ constexpr int gj_ld(int n) { return ((n + kGjCtas - 1) / kGjCtas) | 1; }
+static size_t gj_smem(int n) { return ((size_t)n * gj_ld(n) + 2 * (size_t)n + 2) * sizeof(double) + ((size_t)n + 2) * sizeof(int); }
+
+__global__ void __cluster_dims__(kGjCtas, 1, 1) __launch_bounds__(1024)
+    k_gauss_jordan(int n, const double* __restrict__ aug, const int* __restrict__ absent, double* __restrict__ out,
+                   int* status) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int q = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ncol = (n + kGjCtas - 1) / kGjCtas, ld = gj_ld(n);
+    extern __shared__ __align__(16) double gj_s[];
+    double* S = gj_s;                     // [n][ld]
+    double* F = S + (size_t)n * ld;       // factors of two steps in turn, [2][n]
+    double* pinvs = F + 2 * n;            // [2]
+    int* perm = (int*)(pinvs + 2);        // [n]
+    int* pivs = perm + n;                 // [2]
+    // a thread's column and first row; the last 1024 % ncol threads have none
+    const int step = 1024 / ncol, lc = tid % ncol, r0 = tid / ncol;
+    const bool mine = r0 < step && lc * kGjCtas + q < n;
+    if (mine)
+        for (int r = r0; r < n; r += step) S[(size_t)r * ld + lc] = aug[(size_t)r * 2 * n + lc * kGjCtas + q];
+    for (int r = tid; r < n; r += 1024) perm[r] = r;
+    cluster.sync();
     for (int k = 0; k < n; ++k) {
-        double v = -1.0;
-        int idx = n;
-        for (int r = k + threadIdx.x; r < n; r += blockDim.x) {
-            double a = fabs(aug[(size_t)r * w2 + k]);
-            if (a > v) { v = a; idx = r; }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-            int i2 = __shfl_xor_sync(0xffffffffu, idx, o);
-            if (v2 > v || (v2 == v && i2 < idx)) { v = v2; idx = i2; }
-        }
-        if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = v; si[threadIdx.x >> 5] = idx; }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double bv = -1.0;
-            int bi = n;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w)
-                if (sv[w] > bv || (sv[w] == bv && si[w] < bi)) { bv = sv[w]; bi = si[w]; }
-            if (!(bv > 0.0) || !isfinite(bv) || bi >= n) { *status = 1; bi = k; }
-            piv = bi;
-        }
-        __syncthreads();
-        const int p = piv;
-        if (p != k)
-            for (int c = threadIdx.x; c < w2; c += blockDim.x) {
-                double t = aug[(size_t)k * w2 + c];
-                aug[(size_t)k * w2 + c] = aug[(size_t)p * w2 + c];
-                aug[(size_t)p * w2 + c] = t;
+        const int buf = k & 1, lk = k / kGjCtas;
+        const bool owner = q == k % kGjCtas;
+        if (owner && warp < kGjCtas) {
+            // every warp finds the pivot for itself and tells one CTA
+            double v = -1.0;
+            int idx = n;
+            for (int r = k + lane; r < n; r += 32) {
+                const double a = fabs(S[(size_t)r * ld + lk]);
+                if (a > v) { v = a; idx = r; }
             }
-        __syncthreads();
-        if (threadIdx.x == 0) pinv = 1.0 / aug[(size_t)k * w2 + k];
-        __syncthreads();
-        for (int c = threadIdx.x; c < w2; c += blockDim.x) aug[(size_t)k * w2 + c] *= pinv;
-        __syncthreads();
-        // eliminate column k from every other row; the factors are read from
-        // column k before it is overwritten (column k is done last)
-        for (int q = threadIdx.x; q < n * w2; q += blockDim.x) {
-            int r = q / w2, c = q - r * w2;
-            if (r == k || c == k) continue;
-            aug[q] -= aug[(size_t)r * w2 + k] * aug[(size_t)k * w2 + c];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
+                const int i2 = __shfl_xor_sync(0xffffffffu, idx, o);
+                if (v2 > v || (v2 == v && i2 < idx)) { v = v2; idx = i2; }
+            }
+            if (!(v > 0.0) || !isfinite(v) || idx >= n) {
+                idx = k;
+                if (lane == 0) *status = 1;
+            }
+            double* f = cluster.map_shared_rank(F, warp) + (size_t)buf * n;
+            const double ak = S[(size_t)k * ld + lk];
+            for (int r = lane; r < n; r += 32) f[r] = r == k ? 0.0 : (r == idx ? ak : S[(size_t)r * ld + lk]);
+            if (lane == 0) {
+                cluster.map_shared_rank(pinvs, warp)[buf] = 1.0 / S[(size_t)idx * ld + lk];
+                cluster.map_shared_rank(pivs, warp)[buf] = idx;
+            }
+        }
+        cluster.sync();
+        const int p = pivs[buf];
+        const double pinv = pinvs[buf];
+        const double* f = F + (size_t)buf * n;
+        const bool slot = owner && lc == lk;   // column k's place goes to the inverse
+        double pk = 0, old = 0;
+        if (mine) {
+            pk = slot ? pinv : S[(size_t)p * ld + lc] * pinv;
+            old = S[(size_t)k * ld + lc];
         }
         __syncthreads();
-        for (int r = threadIdx.x; r < n; r += blockDim.x)
-            if (r != k) aug[(size_t)r * w2 + k] = 0.0;
+        if (mine)
+            for (int r = r0; r < n; r += step) {
+                double* e = S + (size_t)r * ld + lc;
+                const double fr = f[r];
+                if (r == k) *e = pk;
+                else if (fr != 0.0 || r == p || slot)
+                    *e = fma(-fr, pk, slot ? 0.0 : (r == p ? old : *e));
+            }
+        if (tid == 0) {
+            const int t = perm[k];
+            perm[k] = perm[p];
+            perm[p] = t;
+        }
         __syncthreads();
+    }
+    if (mine) {
+        const int c = perm[lc * kGjCtas + q];
+        for (int r = r0; r < n; r += step)
+            out[(size_t)r * n + c] = (absent[r] || absent[c]) ? 0.0 : S[(size_t)r * ld + lc];
     }
 }
 // The same elimination for larger n, one pivot column per pair of launches:
@@ -634,16 +679,18 @@ void dense_spd_inverse(mgldg_ctx* ctx, const mgldg_bsr* A, double* out_inv) {
         }
         {
             Launch L(ctx, MGLDG_K_SETUP);
-            k_identity_right<<<std::min(n, 1024), 256, 0, ctx->stream>>>(n, aug);
-        }
-        {
-            Launch L(ctx, MGLDG_K_SETUP);
             k_mark_absent<<<(n + 7) / 8, 256, 0, ctx->stream>>>(n, aug, absent);
         }
-        if (n <= 128) {
+        if (n <= kGjMaxN) {
+            const size_t smem = gj_smem(n);
+            MG_CHECK_CUDA(cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
             Launch L(ctx, MGLDG_K_SETUP);
-            k_gauss_jordan<<<1, 1024, 0, ctx->stream>>>(n, aug, dstatus);
+            k_gauss_jordan<<<kGjCtas, 1024, smem, ctx->stream>>>(n, aug, absent, out_inv, dstatus);
         } else {
+            {
+                Launch L(ctx, MGLDG_K_SETUP);
+                k_identity_right<<<std::min(n, 1024), 256, 0, ctx->stream>>>(n, aug);
+            }
             double* f = dalloc<double>(n);
             try {
                 const dim3 grid((unsigned)std::min(8, (2 * n + 255) / 256), (unsigned)std::min(n, ctx->sm_count * 8));
@@ -661,10 +708,10 @@ void dense_spd_inverse(mgldg_ctx* ctx, const mgldg_bsr* A, double* out_inv) {
             }
             sync(ctx);
             dfree(f);
-        }
-        {
-            Launch L(ctx, MGLDG_K_SETUP);
-            k_extract_right<<<std::min(n, 1024), 256, 0, ctx->stream>>>(n, aug, absent, out_inv);
+            {
+                Launch L(ctx, MGLDG_K_SETUP);
+                k_extract_right<<<std::min(n, 1024), 256, 0, ctx->stream>>>(n, aug, absent, out_inv);
+            }
         }
         check_launch();
         int h = 0;

@@ -199,7 +199,11 @@ def level_bytes(mg, nlev, s, f16=False):
     Jacobi sweep from x = 0 (the first of each V-cycle level: inverse diagonal
     blocks, b and x_out only), one SpMV.  f16: the level operator is read from
     its block-scaled FP16 copy (2 bytes per entry + one 4-byte scale per
-    block; inverse diagonal blocks and vectors in FP32, s = 4)."""
+    block; inverse diagonal blocks and vectors in FP32, s = 4).  The uniform
+    grid's operators have 17 distinct blocks; from TABLE_ROWS block rows on,
+    Jacobi sweeps and products keep them on chip and move indices and vectors
+    only."""
+    TABLE_ROWS = {4: 32768, 9: 16384, 16: 8192}
     out = []
     for l in range(nlev):
         nbr, nbc, br, bc, nnzb = mg.level_op(l, 4).info()
@@ -211,7 +215,10 @@ def level_bytes(mg, nlev, s, f16=False):
         jac = av + nbr * b2 * s + idx + 3 * n * s
         jac0 = nbr * b2 * s + 2 * n * s
         spmv = av + idx + 3 * n * s
-        out.append(dict(gs=gs, jacobi=jac, jacobi0=jac0, spmv=spmv, nbr=nbr, nnzb=nnzb, b=br))
+        table = br == bc and nbr >= TABLE_ROWS.get(br, nbr + 1)
+        if table:
+            jac, jac0, spmv = idx + 3 * n * s, 4 * nbr + 2 * n * s, idx + 3 * n * s
+        out.append(dict(gs=gs, jacobi=jac, jacobi0=jac0, spmv=spmv, nbr=nbr, nnzb=nnzb, b=br, table=table))
     return out
 
 
@@ -856,12 +863,8 @@ def run_gpu(args, ws, rank, local):
     # few us each and their event times include launch gaps).  Algorithmic
     # bytes per launch come from the level's actual matrix; time from CUDA
     # events on the library's stream in the profiled pass of the same steps.
-    # traffic: dram__bytes_read.sum + dram__bytes_write.sum of the same kernel
-    # from one ncu capture at 256x256 Q3 (DRAM bytes / algorithmic bytes, the
-    # ratio below), scaled to this launch by its algorithmic bytes.
-    NCU_TRAFFIC_RATIO = {("mixed_jacobi", "jacobi"): 418.508032 / 415.756292,
-                         ("mixed16_jacobi", "jacobi"): 254.26816 / 249.815044}
-
+    # Kernels that hold the operator's distinct blocks in shared memory are
+    # bound by the FP64 pipes or by latency on chip, not by HBM.
     def kernel_roof(form, cls, key):
         _, _, prec = FORMS[form]
         prof_f, per_level_f = profs[form]
@@ -877,14 +880,11 @@ def run_gpu(args, ws, rank, local):
             nsw = WL["npre"] + WL["npost"]
             bytes0 = ((nsw - 1) * lb[0]["jacobi"] + lb[0]["jacobi0"]) / nsw
         achieved = bytes0 * n0 / (ms0 * 1e-3) / 1e9
-        r = {"bound": "hbm", "form": form, "kernel": cls, "level": 0, "achieved": achieved, "peak": hbm,
+        bound = "hbm" if key == "gs" or not lb[0]["table"] else ("fp64 pipes" if prec == 0 else "latency (L1, L2)")
+        r = {"bound": bound, "form": form, "kernel": cls, "level": 0, "achieved": achieved, "peak": hbm,
              "unit": "GB/s", "frac": achieved / hbm, "traffic": None, "peak_kind": peak_kind, "launches": n0,
              "avg_launch_ms": ms0 / n0, "algorithmic_bytes_per_launch": bytes0,
              "all_levels": {"launches": prof_f[cls][0], "ms": prof_f[cls][1]}}
-        ratio = NCU_TRAFFIC_RATIO.get((form, key))
-        if ratio:
-            r["traffic"] = bytes0 * ratio
-            r["traffic_source"] = "ncu at 256x256 Q3, scaled by block rows"
         return r
 
     _, _, prec_h = FORMS[headline]

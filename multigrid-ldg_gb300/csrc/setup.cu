@@ -483,11 +483,11 @@ __global__ void k_identity_right(int n, double* aug) {
 // inverse is built in place: once row k has been a pivot row, slot k holds the
 // column of the inverse that row k's unit vector has become (perm), so a step
 // touches n columns of [A | I], not 2 n; every entry gets the operations that
-// the elimination of [A | I] gives it.  The
-// coarsest level of a 64 x 64 Q2 hierarchy (144 unknowns, allocations and all):
-// 2.1 -> 0.6 ms against a pair of launches per pivot.  Up to kGjMaxN the matrix
-// fits the shared memory of eight SMs; beyond it the pairs of launches below
-// run over all SMs.
+// the elimination of [A | I] gives it.  Coarsest levels, allocations and all:
+// 64 unknowns 0.6 -> 0.2 ms (one CTA on global memory before), 144 unknowns 2.1
+// -> 0.6, 256 unknowns 3.7 -> 1.9 (a pair of launches per pivot before).  Up to
+// kGjMaxN the matrix fits the shared memory of eight SMs; beyond it the pairs
+// of launches below run over all SMs.
 constexpr int kGjCtas = 8;
 constexpr int kGjMaxN = 448;   // 8 x 211 KB
 

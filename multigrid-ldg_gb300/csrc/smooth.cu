@@ -437,8 +437,11 @@ __global__ void __launch_bounds__(WPB * 32)
 //
 // Two consecutive rows may be of different tiles and a tile's rows of
 // different levels: the ring's slots carry the item's number in the CTA, and a
-// reader that finds its slot taken by a later item reads the row from L2.
-constexpr unsigned kGsRing = 64;
+// reader that finds its slot taken by a later item reads the row from L2.  The
+// ring's length is a multiple of the warp count, so that all items of a slot
+// belong to one warp and are written in order: an older item's tag put over a
+// newer one would leave the newer one's readers waiting.
+constexpr int kGsRing = 64;   // most slots
 
 // Rows that go to one CTA: 4 x 4 patches, whose diagonals have a row for each
 // of the SM's warp schedulers (8 x 8: 858 us instead of 449 for the 256 x 256
@@ -537,8 +540,11 @@ struct GsTile {
     static constexpr int BUF = ((MAXB + 1) * BB * (int)sizeof(T) + 15) / 16 * 16;
     static constexpr int STAGE = (NR * XL * (int)sizeof(T) + 15) / 16 * 16;
     static constexpr int PER_WARP = 2 * BUF + STAGE;
-    static constexpr int RING = (int)kGsRing * LDW * 8;
-    static constexpr int WPB = RING + 16 * PER_WARP <= 220 * 1024 ? 16 : (RING + 12 * PER_WARP <= 220 * 1024 ? 12 : 8);
+    static constexpr int RMAX = kGsRing * LDW * 8;
+    static constexpr int WPB = RMAX + 16 * PER_WARP <= 220 * 1024 ? 16 : (RMAX + 12 * PER_WARP <= 220 * 1024 ? 12 : 8);
+    static constexpr unsigned SLOTS = kGsRing / WPB * WPB;
+    static_assert(SLOTS > 0 && SLOTS % WPB == 0, "one warp per ring slot");
+    static constexpr int RING = (int)SLOTS * LDW * 8;
     static constexpr int SMEM = RING + WPB * PER_WARP;
     static constexpr int CP = BB * (int)sizeof(T) % 16 == 0 ? 16 : (BB * (int)sizeof(T) % 8 == 0 ? 8 : 4);
 };
@@ -636,7 +642,7 @@ __global__ void __launch_bounds__(GsTile<T, B>::WPB * 32, 1)
     const bool first = active && sl == 0;
     const int rr = active ? r : 0;
     const int c0 = sl * CH;
-    for (int q = threadIdx.x; q < (int)kGsRing * G::LDW; q += WPB * 32) ring[q] = 0;
+    for (int q = threadIdx.x; q < (int)G::SLOTS * G::LDW; q += WPB * 32) ring[q] = 0;
     for (int q = lane; q < G::NR * G::XL; q += 32) stage[q] = T(0);
     const unsigned base = __ldcg(&sync->epoch);
     __syncthreads();
@@ -770,7 +776,7 @@ __global__ void __launch_bounds__(GsTile<T, B>::WPB * 32, 1)
             T av[CH], xv[CH];
             if (t < G::MAXB) block_part<T, B>(buf + (t + 1) * BB, rr, c0, av);
             else block_part<T, B>(val + (size_t)(k0 + t) * BB, rr, c0, av);
-            const int st = poll_local<T, B, CH>(ring + ((tag - 1u) & (kGsRing - 1u)) * G::LDW, c0, tag, xv, sync,
+            const int st = poll_local<T, B, CH>(ring + ((tag - 1u) % G::SLOTS) * G::LDW, c0, tag, xv, sync,
                                                 timeout_ns);
             if (st == 0) {
 #pragma unroll
@@ -793,7 +799,7 @@ __global__ void __launch_bounds__(GsTile<T, B>::WPB * 32, 1)
         const T xn = fma(omega, seg_sum<L::S>(y), xs);
         if (first) {
             const unsigned seq = (unsigned)(w - w0);
-            unsigned long long* so = ring + (seq & (kGsRing - 1u)) * G::LDW + r * WPV;
+            unsigned long long* so = ring + (seq % G::SLOTS) * G::LDW + r * WPV;
             const unsigned long long hi = (unsigned long long)(seq + 1u) << 32;
             if constexpr (sizeof(T) == 4) {
                 sts_word(so, hi | __float_as_uint(xn));

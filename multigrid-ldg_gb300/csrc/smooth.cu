@@ -622,7 +622,7 @@ __device__ __forceinline__ void block_part(const T* a, int rr, int c0, T (&v)[WL
 
 template <class T, int B>
 __global__ void __launch_bounds__(GsTile<T, B>::WPB * 32, 1)
-    k_gs_tiles(const int* __restrict__ cta_ptr, const int4* __restrict__ items, const int* __restrict__ ltag,
+    k_gs_tiles(const int* __restrict__ cta_ptr, const int4* __restrict__ items, const signed char* __restrict__ ltag,
                int64_t nnzb, int nsw, const int* __restrict__ col_idx, const T* __restrict__ val,
                const T* __restrict__ Dinv, const T* __restrict__ b, T* x, unsigned long long* xp,
                const int* __restrict__ xptr, const int* __restrict__ xidx, GsSync* sync, T omega, int reverse,
@@ -652,7 +652,7 @@ __global__ void __launch_bounds__(GsTile<T, B>::WPB * 32, 1)
     auto record = [&](int w) { return w < w1 ? __ldg(items + w) : none; };
     auto columns = [&](const int4& it, int& jl, int& tl) {
         jl = lane < it.z ? __ldg(col_idx + it.y + lane) : -1;
-        tl = lane < it.z ? __ldg(ltag + (it.x & 7) * nnzb + it.y + lane) : 0;
+        tl = lane < it.z ? (int)__ldg(ltag + (it.x & 7) * nnzb + it.y + lane) : 0;
     };
     T bn = 0, xn0 = 0;
     auto blocks = [&](const int4& it, int buf) {
@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(GsTile<T, B>::WPB * 32, 1)
         while (own && !failed) {
             const int t = __ffs(own) - 1;
             own &= own - 1;
-            const unsigned tag = (unsigned)__shfl_sync(ALL, tl, t);
+            const unsigned tag = (unsigned)(w - w0 + 1 - __shfl_sync(ALL, tl, t));
             T av[CH], xv[CH];
             if (t < G::MAXB) block_part<T, B>(buf + (t + 1) * BB, rr, c0, av);
             else block_part<T, B>(val + (size_t)(k0 + t) * BB, rr, c0, av);
@@ -993,18 +993,39 @@ void gs_levels_host(int n, const int* row_ptr, const int* col_idx, int dir, std:
     nlev = n ? maxlev + 1 : 0;
 }
 
-static void symmetrised_neighbours(int n, const int* row_ptr, const int* col_idx, std::vector<std::vector<int>>& nb) {
-    nb.assign(n, {});
+// neighbours of every row in the symmetrised pattern, row i's at idx[ptr[i]] ..
+// idx[ptr[i + 1] - 1] in ascending order: its own columns merged with the rows
+// that have it as a column (one pass over the pattern each)
+static void symmetrised_neighbours(int n, const int* row_ptr, const int* col_idx, std::vector<int>& ptr,
+                                   std::vector<int>& idx) {
+    std::vector<int> tp(n + 1, 0);
+    auto other = [&](int i, int j) { return j != i && j >= 0 && j < n; };
+    int64_t nnz = 0;
     for (int i = 0; i < n; ++i)
-        for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k) {
-            const int j = col_idx[k];
-            if (j == i || j < 0 || j >= n) continue;
-            nb[i].push_back(j);
-            nb[j].push_back(i);
+        for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k)
+            if (other(i, col_idx[k])) tp[col_idx[k] + 1]++, ++nnz;
+    for (int i = 0; i < n; ++i) tp[i + 1] += tp[i];
+    std::vector<int> ti(nnz), at(tp.begin(), tp.end() - 1);
+    for (int i = 0; i < n; ++i)
+        for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k)
+            if (other(i, col_idx[k])) ti[at[col_idx[k]]++] = i;
+    ptr.assign(n + 1, 0);
+    idx.clear();
+    idx.reserve(nnz + nnz / 8);
+    std::vector<int> own;
+    for (int i = 0; i < n; ++i) {
+        own.clear();
+        for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k)
+            if (other(i, col_idx[k])) own.push_back(col_idx[k]);
+        if (!std::is_sorted(own.begin(), own.end())) std::sort(own.begin(), own.end());
+        const int *p = own.data(), *pe = p + own.size(), *q = ti.data() + tp[i], *qe = ti.data() + tp[i + 1];
+        int last = -1;
+        while (p < pe || q < qe) {
+            const int j = q == qe || (p < pe && *p <= *q) ? *p++ : *q++;
+            if (j != last) idx.push_back(j);
+            last = j;
         }
-    for (auto& v : nb) {
-        std::sort(v.begin(), v.end());
-        v.erase(std::unique(v.begin(), v.end()), v.end());
+        ptr[i + 1] = (int)idx.size();
     }
 }
 
@@ -1012,17 +1033,15 @@ void sched_build(mgldg_ctx* ctx, const mgldg_bsr* A, Sched& S) {
     const int n = A->nbr;
     S.n = n;
     S.A = A;
-    symmetrised_neighbours(n, A->h_row_ptr.data(), A->h_col_idx.data(), S.nb);
+    symmetrised_neighbours(n, A->h_row_ptr.data(), A->h_col_idx.data(), S.nbp, S.nbi);
     // neighbours j of i with A_ji stored but not A_ij: waited for, not read
     std::vector<int> xp_(n + 1, 0), xi;
-    S.xcount.assign(n, 0);
     for (int i = 0; i < n; ++i) {
         const int* c0 = A->h_col_idx.data() + A->h_row_ptr[i];
         const int* c1 = A->h_col_idx.data() + A->h_row_ptr[i + 1];
-        for (int j : S.nb[i])
-            if (std::find(c0, c1, j) == c1) xi.push_back(j);
+        for (int q = S.nbp[i]; q < S.nbp[i + 1]; ++q)
+            if (std::find(c0, c1, S.nbi[q]) == c1) xi.push_back(S.nbi[q]);
         xp_[i + 1] = (int)xi.size();
-        S.xcount[i] = xp_[i + 1] - xp_[i];
     }
     S.xptr = dalloc<int>(n + 1);
     S.xidx = dalloc<int>(std::max<size_t>(1, xi.size()));
@@ -1036,7 +1055,8 @@ void sched_build(mgldg_ctx* ctx, const mgldg_bsr* A, Sched& S) {
 // Level sets of nsw consecutive sweeps: (s, i) follows (s, j) for earlier
 // neighbours j, (s - 1, j) for later neighbours j and (s - 1, i).
 // lev[s * n + i] is the level of (s, i); returns the number of levels.
-static int gs_pass_levels_host(int n, const std::vector<std::vector<int>>& nb, int dir, int nsw, std::vector<int>& lev) {
+static int gs_pass_levels_host(int n, const std::vector<int>& nbp, const std::vector<int>& nbi, int dir, int nsw,
+                               std::vector<int>& lev) {
     lev.assign((size_t)nsw * n, 0);
     int maxlev = -1;
     for (int s = 0; s < nsw; ++s) {
@@ -1045,7 +1065,8 @@ static int gs_pass_levels_host(int n, const std::vector<std::vector<int>>& nb, i
         for (int t = 0; t < n; ++t) {
             const int i = dir == 0 ? t : n - 1 - t;
             int l = old ? old[i] + 1 : 0;
-            for (int j : nb[i]) {
+            for (int q = nbp[i]; q < nbp[i + 1]; ++q) {
+                const int j = nbi[q];
                 const bool earlier = dir == 0 ? (j < i) : (j > i);
                 if (earlier) l = std::max(l, cur[j] + 1);
                 else if (old) l = std::max(l, old[j] + 1);
@@ -1057,11 +1078,35 @@ static int gs_pass_levels_host(int n, const std::vector<std::vector<int>>& nb, i
     return maxlev + 1;
 }
 
-static void pass_build(mgldg_ctx* ctx, Sched& S, int dir, int nsw, int grid, int tile, GsPass& P) {
+// records and tags of a tile pass, one thread per (sweep, row): loc is the
+// item's number in its CTA's list, owner the CTA of a (sweep, tile)
+__global__ void __launch_bounds__(256) k_gs_plan(int n, int nsw, int shift, int ng, int reverse, int slots,
+                                                 int64_t nnzb, const int* __restrict__ row_ptr,
+                                                 const int* __restrict__ col_idx, const int* __restrict__ xptr,
+                                                 const int* __restrict__ cta_ptr, const int* __restrict__ owner,
+                                                 const int* __restrict__ loc, int4* __restrict__ rec,
+                                                 signed char* __restrict__ ltag) {
+    const int64_t total = (int64_t)nsw * n;
+    for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < total; t += (int64_t)gridDim.x * 256) {
+        const int s = (int)(t / n), i = (int)(t - (int64_t)s * n);
+        const int *os = owner + (size_t)s * ng, *ls = loc + (size_t)s * n;
+        const int o = __ldg(os + (i >> shift)), seq = __ldg(ls + i);
+        const int k0 = __ldg(row_ptr + i), k1 = __ldg(row_ptr + i + 1);
+        rec[(size_t)__ldg(cta_ptr + o) + seq] = make_int4((i << 3) | s, k0, k1 - k0, __ldg(xptr + i + 1) > __ldg(xptr + i));
+        for (int k = k0; k < k1; ++k) {
+            const int j = __ldg(col_idx + k);
+            int d = 0;
+            if ((reverse ? j > i : j < i) && __ldg(os + (j >> shift)) == o) d = seq - __ldg(ls + j);
+            ltag[s * nnzb + k] = (signed char)(d > 0 && d <= slots ? d : 0);
+        }
+    }
+}
+
+static void pass_build(mgldg_ctx* ctx, Sched& S, int dir, int nsw, int grid, int tile, int slots, GsPass& P) {
     const int n = S.n;
     MG_REQUIRE(n < (1 << 28) && nsw >= 1 && nsw <= 7, MGLDG_ERR_UNSUPPORTED, "Gauss-Seidel pass too large");
     std::vector<int> lev;
-    const int maxlev = gs_pass_levels_host(n, S.nb, dir, nsw, lev) - 1;
+    const int maxlev = gs_pass_levels_host(n, S.nbp, S.nbi, dir, nsw, lev) - 1;
     // counting sort by level; inside a level by sweep, then in sweep order
     std::vector<int> cnt(maxlev + 2, 0);
     for (int l : lev) cnt[l + 1]++;
@@ -1078,13 +1123,19 @@ static void pass_build(mgldg_ctx* ctx, Sched& S, int dir, int nsw, int grid, int
     P.tile = tile;
     P.nitems = nsw * n;
     P.depth = n ? maxlev + 1 : 0;
+    P.slots = slots;
     if (grid > 0) {
         // groups of consecutive rows, one sweep each, go to the CTAs in the
-        // order in which the pass reaches them
+        // order in which the pass reaches them; the records and tags follow
+        // from that on the GPU (first V-cycle of a hierarchy with 16,384 rows of
+        // 4 x 4, FP32: 1.04 ms with them made and uploaded here, 0.61 ms)
         const int shift = __builtin_ctz((unsigned)tile), ng = (n + tile - 1) >> shift;   // a power of two
-        std::vector<int> owner((size_t)nsw * ng, -1), cnt2(grid + 1, 0);
-        struct Loc { int cta, seq; };
-        std::vector<Loc> loc((size_t)nsw * n);
+        const size_t nrec = std::max<size_t>(1, items.size()), nown = (size_t)nsw * ng;
+        const size_t ntag = (size_t)nsw * S.A->h_row_ptr[n];
+        // first items of the CTAs, owners, numbers in the CTAs' lists
+        std::vector<int> tab(grid + 1 + nown + items.size(), 0);
+        int *cta = tab.data(), *owner = cta + grid + 1, *loc = owner + nown;
+        std::fill(owner, owner + nown, -1);
         int next = 0;
         for (int it : items) {
             const int i = it >> 3, s = it & 7;
@@ -1093,35 +1144,22 @@ static void pass_build(mgldg_ctx* ctx, Sched& S, int dir, int nsw, int grid, int
                 o = next;
                 next = next + 1 < grid ? next + 1 : 0;
             }
-            loc[(size_t)s * n + i] = {o, ++cnt2[o + 1]};
+            loc[(size_t)s * n + i] = cta[o + 1]++;
         }
-        for (int c = 0; c < grid; ++c) cnt2[c + 1] += cnt2[c];
-        const int *rp = S.A->h_row_ptr.data(), *ci = S.A->h_col_idx.data();
-        // one array: records, tags per (sweep, block), items per CTA
-        const size_t nrec = std::max<size_t>(1, items.size()), ntag = (size_t)nsw * rp[n];
-        std::vector<int> tab(4 * nrec + ntag + grid + 1, 0);
-        int* ltag = tab.data() + 4 * nrec;
-        for (int s = 0; s < nsw; ++s, ltag += rp[n]) {
-            const Loc* ls = loc.data() + (size_t)s * n;
-            for (int i = 0; i < n; ++i) {
-                const Loc l = ls[i];
-                int* rec = tab.data() + 4 * (size_t)(cnt2[l.cta] + l.seq - 1);
-                rec[0] = (i << 3) | s;
-                rec[1] = rp[i];
-                rec[2] = rp[i + 1] - rp[i];
-                rec[3] = S.xcount[i] ? 1 : 0;
-                for (int k = rp[i]; k < rp[i + 1]; ++k) {
-                    const int j = ci[k];
-                    if ((dir == 0 ? j < i : j > i) && ls[j].cta == l.cta) ltag[k] = ls[j].seq;
-                }
-            }
-        }
-        std::copy(cnt2.begin(), cnt2.end(), tab.end() - (grid + 1));
-        P.items = dalloc<int>(tab.size());
-        upload(ctx, P.items, tab.data(), tab.size());
+        for (int c = 0; c < grid; ++c) cta[c + 1] += cta[c];
+        P.items = dalloc<int>(4 * nrec + tab.size() + (ntag + 3) / 4);
         P.rec = reinterpret_cast<int4*>(P.items);
-        P.ltag = P.items + 4 * nrec;
-        P.cta_ptr = P.ltag + ntag;
+        P.cta_ptr = P.items + 4 * nrec;
+        P.ltag = reinterpret_cast<signed char*>(P.cta_ptr + tab.size());
+        upload(ctx, P.cta_ptr, tab.data(), tab.size());
+        if (n) {
+            const int g = (int)std::min<int64_t>(((int64_t)nsw * n + 255) / 256, ctx->sm_count * 16);
+            Launch L(ctx, MGLDG_K_SETUP);
+            k_gs_plan<<<g, 256, 0, ctx->stream>>>(n, nsw, shift, ng, dir, slots, (int64_t)S.A->h_row_ptr[n],
+                                                  S.A->row_ptr, S.A->col_idx, S.xptr, P.cta_ptr, P.cta_ptr + grid + 1,
+                                                  P.cta_ptr + grid + 1 + nown, P.rec, P.ltag);
+        }
+        check_launch();
         sync(ctx);
         return;
     }
@@ -1134,12 +1172,13 @@ static void pass_free(GsPass& P) {
     dfree(P.items);
 }
 
-static GsPass& get_pass(mgldg_ctx* ctx, Sched& S, int dir, int nsw, int grid, int tile) {
+static GsPass& get_pass(mgldg_ctx* ctx, Sched& S, int dir, int nsw, int grid, int tile, int slots) {
     for (auto& P : S.passes)
-        if (P.dir == dir && P.nsw == nsw && P.grid == grid && P.tile == tile) return P;
+        if (P.dir == dir && P.nsw == nsw && P.grid == grid && P.tile == tile && P.slots == slots)
+            return P;
     GsPass P;
     try {
-        pass_build(ctx, S, dir, nsw, grid, tile, P);
+        pass_build(ctx, S, dir, nsw, grid, tile, slots, P);
     } catch (...) {
         pass_free(P);
         throw;
@@ -1203,7 +1242,7 @@ static void launch_gs_tiles(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, c
     MG_REQUIRE(per_sm > 0, MGLDG_ERR_CUDA, "Gauss-Seidel kernel does not fit on an SM");
     const int64_t groups = (int64_t)nsw * ((S.n + tile - 1) / tile);
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(groups, (int64_t)per_sm * ctx->sm_count));
-    GsPass& P = get_pass(ctx, S, reverse ? 1 : 0, nsw, grid, tile);
+    GsPass& P = get_pass(ctx, S, reverse ? 1 : 0, nsw, grid, tile, (int)G::SLOTS);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(WPB * 32);
@@ -1216,9 +1255,10 @@ static void launch_gs_tiles(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, c
     cfg.numAttrs = 1;
     {
         Launch L(ctx, MGLDG_K_GS);
-        MG_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const int*)P.cta_ptr, (const int4*)P.rec, (const int*)P.ltag,
-                                         (int64_t)A->h_row_ptr.back(), nsw, (const int*)A->col_idx, vals, Dinv, b, x, S.xp, (const int*)S.xptr, (const int*)S.xidx, S.sync, omega,
-                                         (int)reverse, S.timeout_ns));
+        MG_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, (const int*)P.cta_ptr, (const int4*)P.rec,
+                                         (const signed char*)P.ltag, (int64_t)A->h_row_ptr.back(), nsw,
+                                         (const int*)A->col_idx, vals, Dinv, b, x, S.xp, (const int*)S.xptr,
+                                         (const int*)S.xidx, S.sync, omega, (int)reverse, S.timeout_ns));
     }
 }
 
@@ -1229,7 +1269,7 @@ static void launch_gs(mgldg_ctx* ctx, const mgldg_bsr* A, const T* vals, const T
     constexpr int MAXE = 1;
     auto kern = k_gs_pass<T, B, WPB, MAXE>;
     packed_rows(ctx, S, B * Packed<T>::WPV);
-    GsPass& P = get_pass(ctx, S, reverse ? 1 : 0, nsw, 0, 0);
+    GsPass& P = get_pass(ctx, S, reverse ? 1 : 0, nsw, 0, 0, 0);
     int per_sm = 0;
     MG_CHECK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, WPB * 32, 0));
     MG_REQUIRE(per_sm > 0, MGLDG_ERR_CUDA, "Gauss-Seidel kernel does not fit on an SM");
@@ -1357,10 +1397,9 @@ extern "C" int mgldg_gs_pass_levels(int nbr, const int* row_ptr, const int* col_
                                     int* level, int* nlevels) {
     if (nbr < 0 || !row_ptr || nsw < 1 || nsw > 7 || (nbr > 0 && row_ptr[nbr] > 0 && !col_idx)) return MGLDG_ERR_ARG;
     try {
-        std::vector<std::vector<int>> nb;
-        mg::symmetrised_neighbours(nbr, row_ptr, col_idx, nb);
-        std::vector<int> lev;
-        const int nl = mg::gs_pass_levels_host(nbr, nb, reverse ? 1 : 0, nsw, lev);
+        std::vector<int> nbp, nbi, lev;
+        mg::symmetrised_neighbours(nbr, row_ptr, col_idx, nbp, nbi);
+        const int nl = mg::gs_pass_levels_host(nbr, nbp, nbi, reverse ? 1 : 0, nsw, lev);
         if (level) std::copy(lev.begin(), lev.end(), level);
         if (nlevels) *nlevels = nl;
     } catch (...) {
@@ -1390,20 +1429,24 @@ extern "C" int mgldg_selftest_wait_timeout(mgldg_ctx* ctx, int64_t timeout_ns, i
         *status = MGLDG_ERR_TIMEOUT;
         // row 0 is never run: row 1 waits for it as another CTA's row (in
         // global memory), then as its own CTA's (in shared memory)
-        for (int owner = -1; owner <= 0; ++owner) {
+        // (the number of an item that its list does not have)
+        for (int tag0 = 0; tag0 >= -1; --tag0) {
             S.passes.emplace_back();
             GsPass& P = S.passes.back();
-            const int tab[10] = {(1 << 3) | 0, 2, 2, 0, /* tags */ 0, 0, owner + 1, 0, /* items */ 0, 1};
+            const signed char tag[4] = {0, 0, (signed char)tag0, 0};
+            int tab[7] = {(1 << 3) | 0, 2, 2, 0, /* items */ 0, 1, /* tags */ 0};
+            std::memcpy(tab + 6, tag, sizeof tag);
             P.nsw = 1;
             P.nitems = 1;
             P.depth = 1;
             P.grid = 1;
             P.tile = kGsTile<double, 1>;
-            P.items = dalloc<int>(10);
+            P.slots = GsTile<double, 1>::SLOTS;
+            P.items = dalloc<int>(7);
             P.rec = reinterpret_cast<int4*>(P.items);
-            P.ltag = P.items + 4;
-            P.cta_ptr = P.items + 8;
-            upload(ctx, P.items, tab, 10);
+            P.cta_ptr = P.items + 4;
+            P.ltag = reinterpret_cast<signed char*>(P.items + 6);
+            upload(ctx, P.items, tab, 7);
             gs_sweeps<double>(ctx, A, A->val, dinv, b, x, S, 1.0, false, 1);
             sync(ctx);
             if (!gs_take_error(ctx, S)) *status = MGLDG_OK;

@@ -17,21 +17,22 @@ struct GsSync {
 // 1 reverse), items (row << 3 | sweep) in the level order of the combined
 // dependency graph; with grid > 0 per CTA, `tile` consecutive rows to one
 struct GsPass {
-    int nsw = 0, dir = 0, nitems = 0, depth = 0, grid = 0, tile = 0;
+    int nsw = 0, dir = 0, nitems = 0, depth = 0, grid = 0, tile = 0, slots = 0;
     int* items = nullptr;     // the items, or the arrays below in one allocation
     int4* rec = nullptr;      // per CTA's item: item, first block, blocks, rows to wait for without reading?
-    int* ltag = nullptr;      // per (sweep, block): the neighbour's number in the CTA's list + 1, 0 if elsewhere
     int* cta_ptr = nullptr;   // first item of every CTA
+    // per (sweep, block): how many items earlier the neighbour is in the CTA's
+    // list, 0 if it is not among the last `slots` of them
+    signed char* ltag = nullptr;
 };
 
 // Gauss-Seidel schedule of one matrix
 struct Sched {
     int n = 0;
     const mgldg_bsr* A = nullptr;            // the pattern the passes are built from
-    std::vector<std::vector<int>> nb;        // symmetrised neighbours of every row (host)
+    std::vector<int> nbp, nbi;               // symmetrised neighbours of every row (host): offsets, rows
     int* xptr = nullptr;                     // per row: symmetrised neighbours outside its own pattern
     int* xidx = nullptr;
-    std::vector<int> xcount;                 // their number (host)
     std::vector<GsPass> passes;              // built on first use per (direction, sweeps)
     unsigned long long* xp = nullptr;        // packed published values, words_per_row per row
     int words_per_row = 0;

@@ -147,14 +147,23 @@ void launch_split(mgldg_ctx* ctx, const SplitArgs<T>& a, int kclass) {
 // each lane a block row (strided loads, 1.1 TB/s).  General / 1 / 2 / 4 / 8
 // groups per row on a 5-level ball: 5,143 rows (11.7 blocks each) 161 / 39.8 /
 // 32.8 / 34.3 / 40.4, 605 rows (14.2) 60.4 / 14.5 / 10.8 / 9.3 / 10.9; 25 x 25,
-// 20,000 rows of 5.5 blocks 270 / - / 65.5, 300 rows 24.6 / - / - / 6.5.  FP64 is
-// bound by its pipes, which the row sums of this form load further: 27 x 27
-// 605 rows 36.9 / 28.9 (4 groups) but 5,143 rows 144 / 155 (2), 25 x 25 300
-// rows 18.5 / 12.7 (4), 1,500 rows 30.6 / 40.1 (4).
+// 20,000 rows of 5.5 blocks 270 / - / 65.5, 300 rows 24.6 / - / - / 6.5.
+//
+// FP64 is bound by its pipes, which the row sums of this form load further: it
+// pays while the SMs are nearly empty, and the longer for longer rows.  One
+// V-cycle of eight sweeps, general / 4 groups, 27 x 27: 1 block per row 150 rows
+// 79 / 79, 200 rows 79 / 95, 2,000 rows 128 / 349; 4 blocks 300 rows 129 / 96,
+// 450 rows 128 / 127, 800 rows 129 / 226; 9 blocks 600 rows 210 / 183, 800 rows
+// 210 / 303; 16 blocks 600 rows 302 / 227, 800 rows 309 / 349.  25 x 25 has the
+// same lines (4 blocks 450 rows 128 / 116, 600 rows 128 / 144).
+//
 // 9 x 9 (agglomerated triangles), general / 1 / 3 / 6 / 12 groups: FP32 8,859
 // rows (13.1) 13.7 / 13.9 / 15.2 / 16.5 / 19.5, 1,995 rows (16.5) 10.9 / 12.3 /
 // 8.8 / 8.7 / 9.6; FP64 1,995 rows 21.0 / 16.7 (3), 4,000 rows 34.9 / 26.9 (3).
-// Uniform grids have five blocks per row, too few to deal out.
+// In FP64 the split has the time of two CTAs (16 rows) on an SM up to 16 rows
+// per SM, the general kernel that of one CTA (24 rows) up to 24: eight sweeps of
+// rows of 13 blocks 2,000 rows 144 / 128, 3,000 rows 145 / 161, 4,000 rows 225 /
+// 196.  Uniform grids have five blocks per row, too few to deal out.
 template <class T, bool JACOBI>
 bool split_dispatch(mgldg_ctx* ctx, const mgldg_bsr* A, SplitArgs<T>& a, int kclass) {
     if (A->br != A->bc || A->blk || A->nbr == 0) return false;
@@ -162,17 +171,20 @@ bool split_dispatch(mgldg_ctx* ctx, const mgldg_bsr* A, SplitArgs<T>& a, int kcl
     a.n = A->nbr;
     a.row_ptr = A->row_ptr;
     a.col_idx = A->col_idx;
-    if (A->br == 27 && (!f64 || A->nbr < 2048)) {
-        if (A->nbr < 2048) launch_split<T, 27, 4, 1, JACOBI>(ctx, a, kclass);
-        else launch_split<T, 27, 2, 1, JACOBI>(ctx, a, kclass);
+    const int64_t n = A->nbr, nnzb = A->nnzb;
+    if (A->br == 27 || A->br == 25) {
+        if constexpr (f64) {
+            if (!(n <= 150 || (n < 400 && nnzb >= 3 * n) || (n < 640 && nnzb >= 8 * n))) return false;
+        } else if (n >= 2048) {
+            if (A->br == 27) launch_split<T, 27, 2, 1, JACOBI>(ctx, a, kclass);
+            else launch_split<T, 25, 2, 1, JACOBI>(ctx, a, kclass);
+            return true;
+        }
+        if (A->br == 27) launch_split<T, 27, 4, 1, JACOBI>(ctx, a, kclass);
+        else launch_split<T, 25, 4, 1, JACOBI>(ctx, a, kclass);
         return true;
     }
-    if (A->br == 25 && (!f64 || A->nbr < 1024)) {
-        if (A->nbr < 2048) launch_split<T, 25, 4, 1, JACOBI>(ctx, a, kclass);
-        else launch_split<T, 25, 2, 1, JACOBI>(ctx, a, kclass);
-        return true;
-    }
-    if (A->br == 9 && A->nbr < 4096 && A->nnzb >= 8 * (int64_t)A->nbr) {
+    if (A->br == 9 && n < 4096 && nnzb >= 8 * n && (!f64 || n <= 16 * ctx->sm_count || n > 24 * ctx->sm_count)) {
         launch_split<T, 9, 3, 2, JACOBI>(ctx, a, kclass);
         return true;
     }

@@ -1081,14 +1081,13 @@ static void level_alloc(mgldg_ctx* ctx, mgldg_mg* m, LevelData& L, bool need_sch
         MG_CHECK_CUDA(cudaMemsetAsync(dstatus, 0, sizeof(int), ctx->stream));
         L.Dinv = dalloc<double>((size_t)L.ne * L.b * L.b);
         block_inverse(ctx, L.A, L.Dinv, dstatus);
-        RepProbe probe;
-        const bool probed = rep_probe(ctx, L.A, probe);
-        int h = 0;
+        int h = 0, distinct = 0;
+        const bool sampled = rep_sample(ctx, L.A, &distinct);
         download(ctx, &h, dstatus, 1);
         sync(ctx);
         MG_REQUIRE(h == 0, MGLDG_ERR_NOT_SPD, "singular diagonal block in a level matrix");
         // operators made of a few distinct blocks get their table form
-        if (probed) rep_finish(ctx, const_cast<mgldg_bsr*>(L.A), L.Dinv, probe);
+        if (sampled) rep_build(ctx, const_cast<mgldg_bsr*>(L.A), L.Dinv, distinct);
     } catch (...) {
         dfree(dstatus);
         throw;

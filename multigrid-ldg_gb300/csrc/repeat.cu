@@ -41,14 +41,13 @@ RepTable::~RepTable() {
     if (pool) cudaFree(pool);
     if (slots) cudaFree(slots);
 }
-RepProbe::~RepProbe() {
-    if (mem) cudaFree(mem);
-}
 
 // -------------------------------------------------------------- detection --
 namespace {
 constexpr int kMaxUniq = 2048;    // most distinct blocks kept
 constexpr int kHash = 8192;       // hash slots
+constexpr int kSample = 2560;     // blocks of the sample, more than kMaxUniq
+constexpr int kSampleKeys = 4096;
 struct HashSlot {
     unsigned long long key;       // block hash, 0: empty
     int first;                    // smallest block index with this hash
@@ -63,30 +62,55 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long z) {
     return z ^ (z >> 31);
 }
 
+// hash of one block's values by a warp, with -0 taken as +0 (valid in every
+// lane, never 0)
+__device__ __forceinline__ unsigned long long block_hash(const double* __restrict__ a, int bsz, int lane) {
+    unsigned long long h = 0;
+    for (int e = lane; e < bsz; e += 32) {
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(__ldg(a + e) + 0.0);
+        h += mix64(bits + 0x9e3779b97f4a7c15ULL * (unsigned long long)(e + 1));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+    return h ? h : 1ULL;
+}
+
+// Number of distinct blocks among m evenly spaced ones, one warp each: more
+// than kMaxUniq of them rule a table out.  Most operators without repeated
+// blocks end here, with no allocation and no wait of their own (hashing all of
+// them, with the table's memory, took mgldg_mg_create 0.4 ms per large level).
+__global__ void __launch_bounds__(256) k_rep_sample(int64_t nnzb, int bsz, const double* __restrict__ val, int m,
+                                                    unsigned long long* keys, int* count) {
+    const int lane = threadIdx.x & 31, t = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (t >= m) return;
+    const int64_t k = (int64_t)t * nnzb / m;
+    const unsigned long long h = block_hash(val + k * bsz, bsz, lane);
+    if (lane) return;
+    int s = (int)(h & (kSampleKeys - 1));
+    for (int probe = 0; probe < kSampleKeys; ++probe) {   // m < kSampleKeys: ends
+        const unsigned long long cur = atomicCAS(keys + s, 0ULL, h);
+        if (cur == 0ULL) atomicAdd(count, 1);
+        if (cur == 0ULL || cur == h) return;
+        s = (s + 1) & (kSampleKeys - 1);
+    }
+}
+
 __global__ void k_rep_clear(HashSlot* slots, int* head) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < kHash) slots[t] = HashSlot{0ULL, 0x7fffffff, -1};
     if (t < 2) head[t] = 0;
 }
 
-// One warp per block: hash of its values (with -0 taken as +0), entered into
-// the hash table with the smallest block index.  Once more than kMaxUniq
-// distinct hashes were met the warps stop: an operator without repeated
-// blocks costs this kernel a few microseconds.
+// One warp per block: its hash, entered into the hash table with the smallest
+// block index.  Once more than kMaxUniq distinct hashes were met the warps
+// stop.
 __global__ void __launch_bounds__(256) k_rep_hash(int64_t nnzb, int bsz, const double* __restrict__ val,
                                                   HashSlot* slots, int* head, int* __restrict__ slot_of) {
     const int lane = threadIdx.x & 31;
     for (int64_t k = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); k < nnzb; k += (int64_t)gridDim.x * 8) {
         if (*(volatile int*)&head[1]) return;
-        unsigned long long h = 0;
-        for (int e = lane; e < bsz; e += 32) {
-            const unsigned long long bits = (unsigned long long)__double_as_longlong(__ldg(val + k * bsz + e) + 0.0);
-            h += mix64(bits + 0x9e3779b97f4a7c15ULL * (unsigned long long)(e + 1));
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
+        const unsigned long long h = block_hash(val + k * bsz, bsz, lane);
         if (lane == 0) {
-            if (h == 0) h = 1;
             int s = (int)(h & (kHash - 1));
             int found = -1;
             for (int probe = 0; probe < kHash; ++probe) {
@@ -218,32 +242,47 @@ static bool rep_shape(const mgldg_bsr* A, int min_rows) {
            A->nbr >= min_rows && A->nnzb < (1LL << 31);
 }
 
-bool rep_probe(mgldg_ctx* ctx, const mgldg_bsr* A, RepProbe& p, bool batch) {
+bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int* distinct, bool batch) {
     if (A->rep || !rep_shape(A, batch ? kRepMmRows : rep_min_rows(A->br))) return false;
-    const size_t bytes = 16 + kHash * sizeof(HashSlot) + (size_t)A->nnzb * sizeof(int);
-    p.mem = dalloc<char>(bytes);
-    int* head = (int*)p.mem;
-    HashSlot* slots = (HashSlot*)((char*)p.mem + 16);
+    // keys and count in the reduction scratch
+    unsigned long long* keys = (unsigned long long*)ctx->d_partials;
+    int* count = (int*)(keys + kSampleKeys);
+    MG_REQUIRE(ctx->n_partials > kSampleKeys, MGLDG_ERR_ARG, "reduction scratch too small");
+    MG_CHECK_CUDA(cudaMemsetAsync(keys, 0, (kSampleKeys + 1) * sizeof(*keys), ctx->stream));
+    const int m = (int)std::min<int64_t>(A->nnzb, kSample);
+    {
+        Launch L(ctx, MGLDG_K_SETUP);
+        k_rep_sample<<<(m + 7) / 8, 256, 0, ctx->stream>>>(A->nnzb, (int)A->bsz(), A->val, m, keys, count);
+    }
+    check_launch();
+    download(ctx, distinct, count, 1);
+    return true;
+}
+
+void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, int gs_want) {
+    // (both hold for all blocks if they hold for a sample)
+    if (distinct > kMaxUniq || (int64_t)distinct * 4 > A->nnzb) return;
+    struct Mem {
+        char* p = nullptr;
+        ~Mem() { dfree(p); }
+    } mem;
+    mem.p = dalloc<char>(16 + kHash * sizeof(HashSlot) + (size_t)A->nnzb * sizeof(int));
+    int* head = (int*)mem.p;   // distinct blocks, overflow
+    HashSlot* slots = (HashSlot*)(mem.p + 16);
     int* slot_of = (int*)(slots + kHash);
-    k_rep_clear<<<kHash / 256, 256, 0, ctx->stream>>>(slots, head);
     const int g = (int)std::min<int64_t>((A->nnzb + 7) / 8, ctx->sm_count * 8);
+    k_rep_clear<<<kHash / 256, 256, 0, ctx->stream>>>(slots, head);
     {
         Launch L(ctx, MGLDG_K_SETUP);
         k_rep_hash<<<g, 256, 0, ctx->stream>>>(A->nnzb, (int)A->bsz(), A->val, slots, head, slot_of);
     }
     check_launch();
-    download(ctx, p.head, head, 2);
-    return true;
-}
-
-void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p, int gs_want) {
-    // the caller has synchronised: p.head is valid.  A table pays when a
-    // block is used several times.
-    const int nu = p.head[0];
-    if (!p.mem || p.head[1] || nu < 1 || (int64_t)nu * 4 > A->nnzb) return;
-    int* head = (int*)p.mem;
-    HashSlot* slots = (HashSlot*)((char*)p.mem + 16);
-    int* slot_of = (int*)(slots + kHash);
+    int hd[2] = {0, 0};
+    download(ctx, hd, head, 2);
+    sync(ctx);
+    // a table pays when a block is used several times
+    const int nu = hd[0];
+    if (hd[1] || nu < 1 || (int64_t)nu * 4 > A->nnzb) return;
     const int b = A->br, n = A->nbr, ld = (b + 3) / 4 * 4;
     std::vector<HashSlot> hs(kHash);
     download(ctx, hs.data(), slots, hs.size());
@@ -260,17 +299,16 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p, i
         first[u] = hs[order[u]].first;
     }
     upload(ctx, slots, hs.data(), hs.size());
-    const int g = (int)std::min<int64_t>((A->nnzb + 7) / 8, ctx->sm_count * 8);
     {
         Launch L(ctx, MGLDG_K_SETUP);
         k_rep_assign<<<g, 256, 0, ctx->stream>>>(A->nnzb, (int)A->bsz(), A->val, slots, head, slot_of);
     }
     check_launch();
     std::vector<int> id(A->nnzb);
-    download(ctx, p.head, head, 2);
+    download(ctx, hd, head, 2);
     download(ctx, id.data(), slot_of, id.size());
     sync(ctx);
-    if (p.head[1]) return;   // two different blocks with one hash
+    if (hd[1]) return;   // two different blocks with one hash
     // ---- row classes ----
     const int* rp = A->h_row_ptr.data();
     const int* ci = A->h_col_idx.data();
@@ -422,10 +460,10 @@ void rep_finish(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, RepProbe& p, i
 
 bool rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv) {
     if (A->rep) return A->rep->nslots != 0;
-    RepProbe p;
-    if (!rep_probe(ctx, A, p, true)) return false;
+    int distinct = 0;
+    if (!rep_sample(ctx, A, &distinct, true)) return false;
     sync(ctx);
-    rep_finish(ctx, A, Dinv, p, 4);
+    rep_build(ctx, A, Dinv, distinct, 4);
     return A->rep && A->rep->nslots != 0;
 }
 

@@ -26,7 +26,6 @@
 #include <algorithm>
 #include <memory>
 #include <type_traits>
-#include <unordered_map>
 
 #include "api.cuh"
 #include "repeat.cuh"
@@ -45,13 +44,14 @@ RepTable::~RepTable() {
 // -------------------------------------------------------------- detection --
 namespace {
 constexpr int kMaxUniq = 2048;    // most distinct blocks kept
+constexpr int kMaxCls = 4096;     // most row classes kept
 constexpr int kHash = 8192;       // hash slots
 constexpr int kSample = 2560;     // blocks of the sample, more than kMaxUniq
 constexpr int kSampleKeys = 4096;
 struct HashSlot {
-    unsigned long long key;       // block hash, 0: empty
-    int first;                    // smallest block index with this hash
-    int id;                       // table entry (second step)
+    unsigned long long key;       // hash of a block (a row), 0: empty
+    int first;                    // smallest block (row) index with this hash
+    int id;                       // table entry (class), second step
 };
 }  // namespace
 
@@ -97,8 +97,31 @@ __global__ void __launch_bounds__(256) k_rep_sample(int64_t nnzb, int bsz, const
 
 __global__ void k_rep_clear(HashSlot* slots, int* head) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < kHash) slots[t] = HashSlot{0ULL, 0x7fffffff, -1};
-    if (t < 2) head[t] = 0;
+    if (t < 2 * kHash) slots[t] = HashSlot{0ULL, 0x7fffffff, -1};
+    if (t < 4) head[t] = 0;
+}
+
+// enters hash h of item k; head: distinct hashes, set once there are more
+// than `most`.  The slot, or -1 after that.
+__device__ __forceinline__ int hash_enter(HashSlot* slots, int* head, int most, unsigned long long h, int k) {
+    int s = (int)(h & (kHash - 1));
+    for (int probe = 0; probe < kHash; ++probe) {
+        unsigned long long cur = *(volatile unsigned long long*)&slots[s].key;
+        if (cur == 0) {
+            cur = atomicCAS(&slots[s].key, 0ULL, h);
+            if (cur == 0) {
+                if (atomicAdd(&head[0], 1) >= most) *(volatile int*)&head[1] = 1;
+                cur = h;
+            }
+        }
+        if (cur == h) {
+            if (*(volatile int*)&slots[s].first > k) atomicMin(&slots[s].first, k);
+            return s;
+        }
+        if (*(volatile int*)&head[1]) break;
+        s = (s + 1) & (kHash - 1);
+    }
+    return -1;
 }
 
 // One warp per block: its hash, entered into the hash table with the smallest
@@ -111,28 +134,8 @@ __global__ void __launch_bounds__(256) k_rep_hash(int64_t nnzb, int bsz, const d
         if (*(volatile int*)&head[1]) return;
         const unsigned long long h = block_hash(val + k * bsz, bsz, lane);
         if (lane == 0) {
-            int s = (int)(h & (kHash - 1));
-            int found = -1;
-            for (int probe = 0; probe < kHash; ++probe) {
-                unsigned long long cur = *(volatile unsigned long long*)&slots[s].key;
-                if (cur == 0) {
-                    cur = atomicCAS(&slots[s].key, 0ULL, h);
-                    if (cur == 0) {
-                        if (atomicAdd(&head[0], 1) >= kMaxUniq) *(volatile int*)&head[1] = 1;
-                        cur = h;
-                    }
-                }
-                if (cur == h) {
-                    found = s;
-                    break;
-                }
-                if (*(volatile int*)&head[1]) break;
-                s = (s + 1) & (kHash - 1);
-            }
-            if (found >= 0) {
-                if (*(volatile int*)&slots[found].first > (int)k) atomicMin(&slots[found].first, (int)k);
-                slot_of[k] = found;
-            }
+            const int s = hash_enter(slots, head, kMaxUniq, h, (int)k);
+            if (s >= 0) slot_of[k] = s;
         }
     }
 }
@@ -154,6 +157,69 @@ __global__ void __launch_bounds__(256) k_rep_assign(int64_t nnzb, int bsz, const
             if (!same) head[1] = 1;
             slot_of[k] = s.id;
         }
+    }
+}
+
+// Row classes (same sequence of table entries and the diagonal one in the same
+// place), the same way: hash of every row, then every row against the class's
+// first row.  (Made row by row on the host, the tables of a hierarchy with
+// 175,006 quadtree rows of 9 x 9 took mgldg_mg_create 15 ms, now 6.)
+__global__ void __launch_bounds__(256) k_rep_row_hash(int n, const int* __restrict__ row_ptr,
+                                                      const int* __restrict__ diag, const int* __restrict__ id,
+                                                      HashSlot* slots, int* head, int* __restrict__ slot_of) {
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const int k0 = __ldg(row_ptr + i), nb = __ldg(row_ptr + i + 1) - k0, dk = __ldg(diag + i);
+        if (nb < 1 || nb > kRepMaxNb || dk < 0) {
+            head[1] = 1;
+            return;
+        }
+        unsigned long long h = mix64((unsigned long long)nb * 64 + (unsigned long long)(dk - k0));
+        for (int q = 0; q < nb; ++q) h = mix64(h + 0x9e3779b97f4a7c15ULL * (unsigned long long)(id[k0 + q] + 1));
+        const int s = hash_enter(slots, head, kMaxCls, h ? h : 1ULL, i);
+        if (s < 0) return;
+        slot_of[i] = s;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_rep_classes(int ncls, const int* __restrict__ first,
+                                                     const int* __restrict__ row_ptr, const int* __restrict__ diag,
+                                                     const int* __restrict__ id, int* __restrict__ cls) {
+    for (int t = blockIdx.x * 256 + threadIdx.x; t < ncls * kRepCls; t += gridDim.x * 256) {
+        const int c = t / kRepCls, e = t - c * kRepCls, i = first[c];
+        const int k0 = __ldg(row_ptr + i), nb = __ldg(row_ptr + i + 1) - k0;
+        int v = 0;
+        if (e == 0) v = nb;
+        else if (e == 1) v = id[__ldg(diag + i)];
+        else if (e == 2) v = __ldg(diag + i) - k0;
+        else if (e >= 4 && e < 4 + nb) v = id[k0 + e - 4];
+        cls[t] = v;
+    }
+}
+
+__global__ void __launch_bounds__(256) k_rep_row_assign(int n, const int* __restrict__ row_ptr,
+                                                        const int* __restrict__ diag, const int* __restrict__ id,
+                                                        const HashSlot* __restrict__ slots, const int* __restrict__ cls,
+                                                        int* head, int* slot_of) {
+    for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) {
+        const int c = slots[slot_of[i]].id;
+        const int k0 = __ldg(row_ptr + i), nb = __ldg(row_ptr + i + 1) - k0;
+        const int* d = cls + (size_t)c * kRepCls;
+        bool same = d[0] == nb && d[2] == __ldg(diag + i) - k0;
+        for (int q = 0; q < nb && same; ++q) same = d[4 + q] == id[k0 + q];
+        if (!same) head[1] = 1;
+        slot_of[i] = c;
+    }
+}
+
+// block columns of the slots; padding slots read what their group's first row
+// reads
+__global__ void __launch_bounds__(256) k_rep_cols(int nslots, int gs, int most, const int* __restrict__ rows,
+                                                  const int* __restrict__ row_ptr, const int* __restrict__ col_idx,
+                                                  int* __restrict__ cols) {
+    for (int s = blockIdx.x * 256 + threadIdx.x; s < nslots; s += gridDim.x * 256) {
+        const int r = rows[s], i = r >= 0 ? r : rows[s / gs * gs];
+        const int k0 = __ldg(row_ptr + i), nb = __ldg(row_ptr + i + 1) - k0;
+        for (int q = 0; q < most; ++q) cols[(size_t)q * nslots + s] = __ldg(col_idx + k0 + min(q, nb - 1));
     }
 }
 
@@ -262,99 +328,88 @@ bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int* distinct, bool batch) {
 void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, int gs_want) {
     // (both hold for all blocks if they hold for a sample)
     if (distinct > kMaxUniq || (int64_t)distinct * 4 > A->nnzb) return;
+    const int b = A->br, n = A->nbr, ld = (b + 3) / 4 * 4;
+    const int* rp = A->h_row_ptr.data();
+    if (A->nnzb > (int64_t)kRepMaxNb * n) return;
+    for (int i = 0; i < n; ++i)
+        if (rp[i + 1] - rp[i] > kRepMaxNb) return;
     struct Mem {
         char* p = nullptr;
         ~Mem() { dfree(p); }
     } mem;
-    mem.p = dalloc<char>(16 + kHash * sizeof(HashSlot) + (size_t)A->nnzb * sizeof(int));
-    int* head = (int*)mem.p;   // distinct blocks, overflow
-    HashSlot* slots = (HashSlot*)(mem.p + 16);
-    int* slot_of = (int*)(slots + kHash);
-    const int g = (int)std::min<int64_t>((A->nnzb + 7) / 8, ctx->sm_count * 8);
-    k_rep_clear<<<kHash / 256, 256, 0, ctx->stream>>>(slots, head);
+    mem.p = dalloc<char>(16 + 2 * kHash * sizeof(HashSlot) +
+                         ((size_t)A->nnzb + n + (size_t)kMaxCls * (kRepCls + 1)) * sizeof(int));
+    int* head = (int*)mem.p;   // distinct blocks, not for a table; the same of the row classes
+    HashSlot *slots = (HashSlot*)(mem.p + 16), *cslots = slots + kHash;
+    int *slot_of = (int*)(cslots + kHash), *cls_of_d = slot_of + A->nnzb, *cfirst = cls_of_d + n, *cls_d = cfirst + kMaxCls;
+    const int g = (int)std::min<int64_t>((A->nnzb + 7) / 8, ctx->sm_count * 8), gr = std::min((n + 255) / 256, ctx->sm_count * 8);
+    // slots in the order of their first blocks or rows (independent of the
+    // order in which the hashing threads arrived)
+    std::vector<HashSlot> hs(kHash);
+    auto number = [&](HashSlot* dev, std::vector<int>& first) {
+        std::vector<int> order;
+        for (int s = 0; s < kHash; ++s)
+            if (hs[s].key) order.push_back(s);
+        std::sort(order.begin(), order.end(), [&](int x, int y) { return hs[x].first < hs[y].first; });
+        for (size_t u = 0; u < order.size(); ++u) {
+            hs[order[u]].id = (int)u;
+            first.push_back(hs[order[u]].first);
+        }
+        upload(ctx, dev, hs.data(), hs.size());
+    };
+    int hd[4] = {0, 0, 0, 0};
+    k_rep_clear<<<2 * kHash / 256, 256, 0, ctx->stream>>>(slots, head);
     {
         Launch L(ctx, MGLDG_K_SETUP);
         k_rep_hash<<<g, 256, 0, ctx->stream>>>(A->nnzb, (int)A->bsz(), A->val, slots, head, slot_of);
     }
     check_launch();
-    int hd[2] = {0, 0};
-    download(ctx, hd, head, 2);
+    download(ctx, hd, head, 4);
+    download(ctx, hs.data(), slots, hs.size());
     sync(ctx);
     // a table pays when a block is used several times
     const int nu = hd[0];
     if (hd[1] || nu < 1 || (int64_t)nu * 4 > A->nnzb) return;
-    const int b = A->br, n = A->nbr, ld = (b + 3) / 4 * 4;
-    std::vector<HashSlot> hs(kHash);
-    download(ctx, hs.data(), slots, hs.size());
-    sync(ctx);
-    // table entries in the order of their first blocks (independent of the
-    // order in which the hashing warps arrived)
-    std::vector<int> order;
-    for (int s = 0; s < kHash; ++s)
-        if (hs[s].key) order.push_back(s);
-    std::sort(order.begin(), order.end(), [&](int x, int y) { return hs[x].first < hs[y].first; });
-    std::vector<int> first(nu), drow(nu, -1);
-    for (int u = 0; u < nu; ++u) {
-        hs[order[u]].id = u;
-        first[u] = hs[order[u]].first;
-    }
-    upload(ctx, slots, hs.data(), hs.size());
+    std::vector<int> first, cls_first;
+    number(slots, first);
     {
         Launch L(ctx, MGLDG_K_SETUP);
         k_rep_assign<<<g, 256, 0, ctx->stream>>>(A->nnzb, (int)A->bsz(), A->val, slots, head, slot_of);
     }
-    check_launch();
-    std::vector<int> id(A->nnzb);
-    download(ctx, hd, head, 2);
-    download(ctx, id.data(), slot_of, id.size());
-    sync(ctx);
-    if (hd[1]) return;   // two different blocks with one hash
     // ---- row classes ----
-    const int* rp = A->h_row_ptr.data();
-    const int* ci = A->h_col_idx.data();
-    std::vector<int> cls_of(n), cls;     // cls: kRepCls ints per class
-    bool ok = true;
     {
-        std::unordered_map<uint64_t, std::vector<int>> seen;
-        uint64_t last_key = 0;
-        int last = -1;
-        for (int i = 0; i < n && ok; ++i) {
-            const int k0 = rp[i], nb = rp[i + 1] - k0, dk = A->h_diag[i];
-            if (nb < 1 || nb > kRepMaxNb || dk < 0) {
-                ok = false;
-                break;
-            }
-            uint64_t key = (uint64_t)nb * 64 + (uint64_t)(dk - k0);
-            for (int q = 0; q < nb; ++q) key = key * 0x100000001b3ULL + (uint64_t)id[k0 + q] + 1;   // FNV-style
-            drow[id[dk]] = drow[id[dk]] < 0 ? i : drow[id[dk]];
-            auto same = [&](int c) {
-                const int* d = &cls[(size_t)c * kRepCls];
-                return d[0] == nb && d[1] == id[dk] && std::equal(d + 4, d + 4 + nb, id.begin() + k0);
-            };
-            int c = -1;
-            if (last >= 0 && key == last_key && same(last)) {
-                c = last;
-            } else {
-                std::vector<int>& v = seen[key];
-                for (int q : v)
-                    if (same(q)) c = q;
-                if (c < 0) {
-                    c = (int)(cls.size() / kRepCls);
-                    v.push_back(c);
-                    cls.resize(cls.size() + kRepCls, 0);
-                    int* d = &cls[(size_t)c * kRepCls];
-                    d[0] = nb;
-                    d[1] = id[dk];
-                    std::copy(id.begin() + k0, id.begin() + k0 + nb, d + 4);
-                }
-            }
-            last = c;
-            last_key = key;
-            cls_of[i] = c;
-        }
+        Launch L(ctx, MGLDG_K_SETUP);
+        k_rep_row_hash<<<gr, 256, 0, ctx->stream>>>(n, A->row_ptr, A->diag, slot_of, cslots, head + 2, cls_of_d);
     }
-    if (!ok) return;
-    const int ncls = (int)(cls.size() / kRepCls);
+    check_launch();
+    download(ctx, hd, head, 4);
+    download(ctx, hs.data(), cslots, hs.size());
+    sync(ctx);
+    if (hd[1] || hd[3]) return;   // two different blocks with one hash; too many classes
+    number(cslots, cls_first);
+    const int ncls = (int)cls_first.size();
+    upload(ctx, cfirst, cls_first.data(), ncls);
+    {
+        Launch L(ctx, MGLDG_K_SETUP);
+        k_rep_classes<<<std::min((ncls * kRepCls + 255) / 256, ctx->sm_count), 256, 0, ctx->stream>>>(
+            ncls, cfirst, A->row_ptr, A->diag, slot_of, cls_d);
+    }
+    {
+        Launch L(ctx, MGLDG_K_SETUP);
+        k_rep_row_assign<<<gr, 256, 0, ctx->stream>>>(n, A->row_ptr, A->diag, slot_of, cslots, cls_d, head, cls_of_d);
+    }
+    check_launch();
+    std::vector<int> cls_of(n), cls((size_t)ncls * kRepCls);   // cls: kRepCls ints per class
+    download(ctx, hd, head, 4);
+    download(ctx, cls.data(), cls_d, cls.size());
+    download(ctx, cls_of.data(), cls_of_d, n);
+    sync(ctx);
+    if (hd[1]) return;
+    std::vector<int> drow(nu, -1);   // a row with this diagonal block
+    for (int c = 0; c < ncls; ++c) {
+        int& d = drow[cls[(size_t)c * kRepCls + 1]];
+        if (d < 0) d = cls_first[c];
+    }
     // ---- slots: the rows of a chunk sorted by class, each class padded to
     // whole groups.  Chunks of 4,096 consecutive rows keep a warp's gathers
     // within one stretch of the vectors; with many classes one chunk wastes
@@ -433,15 +488,8 @@ void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, i
     }
     MG_CHECK_CUDA(cudaMemcpyAsync(t->blk, slot_of, (size_t)A->nnzb * sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
     if (nslots) {
-        std::vector<int> cols((size_t)kRepMaxNb * nslots);
         int most = 0;
         for (int c = 0; c < ncls; ++c) most = std::max(most, cls[(size_t)c * kRepCls]);
-        for (int s = 0; s < nslots; ++s) {
-            // padding slots read what their group's first row reads
-            const int i = rows[s] >= 0 ? rows[s] : rows[s / gs * gs];
-            const int nb = rp[i + 1] - rp[i];
-            for (int q = 0; q < most; ++q) cols[(size_t)q * nslots + s] = ci[rp[i] + std::min(q, nb - 1)];
-        }
         const size_t nc = cls.size(), ng = gcls.size();
         t->slots = dalloc<int>(nc + ng + nslots + (size_t)most * nslots + 16);
         t->cls = (int*)t->slots;
@@ -449,9 +497,14 @@ void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, i
         t->rows = t->cols + (size_t)most * nslots;
         t->gcls = t->rows + nslots;
         upload(ctx, t->cls, cls.data(), nc);
-        upload(ctx, t->cols, cols.data(), (size_t)most * nslots);
         upload(ctx, t->rows, rows.data(), nslots);
         upload(ctx, t->gcls, gcls.data(), ng);
+        {
+            Launch L(ctx, MGLDG_K_SETUP);
+            k_rep_cols<<<std::min((nslots + 255) / 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(
+                nslots, gs, most, t->rows, A->row_ptr, A->col_idx, t->cols);
+        }
+        check_launch();
         sync(ctx);   // the host arrays go out of scope
     }
     sync(ctx);

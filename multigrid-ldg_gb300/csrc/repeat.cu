@@ -36,7 +36,6 @@ using namespace mg;
 namespace mg {
 
 RepTable::~RepTable() {
-    if (blk) cudaFree(blk);
     if (pool) cudaFree(pool);
     if (slots) cudaFree(slots);
 }
@@ -435,7 +434,8 @@ void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, i
         }
     }
     // more than twice as many slots as rows: rare classes, mostly idle lanes
-    const int nslots = rows.size() > 2 * (size_t)n ? 0 : (int)rows.size();
+    if (rows.size() > 2 * (size_t)n) return;
+    const int nslots = (int)rows.size();
     std::unique_ptr<RepTable> t(new RepTable());
     t->b = b;
     t->ld = ld;
@@ -466,7 +466,6 @@ void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, i
     t->clo = vc ? t->c32 + vc : t->ilo;
     t->s16 = t->i16 + v4 + 2 * vc;
     t->mask = (unsigned*)(t->s16 + nu);
-    t->blk = dalloc<int>(A->nnzb);
     int* dint = (int*)slots;   // the hash slots are done with: three index lists go there
     upload(ctx, dint, first.data(), first.size());
     upload(ctx, dint + nu, drow.data(), drow.size());
@@ -486,38 +485,34 @@ void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, i
         int* d = &cls[(size_t)c * kRepCls];
         for (int q = 0; q < d[0]; ++q) d[4 + kRepMaxNb + q] = (int)mask[d[4 + q]];
     }
-    MG_CHECK_CUDA(cudaMemcpyAsync(t->blk, slot_of, (size_t)A->nnzb * sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
-    if (nslots) {
-        int most = 0;
-        for (int c = 0; c < ncls; ++c) most = std::max(most, cls[(size_t)c * kRepCls]);
-        const size_t nc = cls.size(), ng = gcls.size();
-        t->slots = dalloc<int>(nc + ng + nslots + (size_t)most * nslots + 16);
-        t->cls = (int*)t->slots;
-        t->cols = t->cls + nc;
-        t->rows = t->cols + (size_t)most * nslots;
-        t->gcls = t->rows + nslots;
-        upload(ctx, t->cls, cls.data(), nc);
-        upload(ctx, t->rows, rows.data(), nslots);
-        upload(ctx, t->gcls, gcls.data(), ng);
-        {
-            Launch L(ctx, MGLDG_K_SETUP);
-            k_rep_cols<<<std::min((nslots + 255) / 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(
-                nslots, gs, most, t->rows, A->row_ptr, A->col_idx, t->cols);
-        }
-        check_launch();
-        sync(ctx);   // the host arrays go out of scope
+    int most = 0;
+    for (int c = 0; c < ncls; ++c) most = std::max(most, cls[(size_t)c * kRepCls]);
+    const size_t nc = cls.size(), ng = gcls.size();
+    t->slots = dalloc<int>(nc + ng + nslots + (size_t)most * nslots + 16);
+    t->cls = (int*)t->slots;
+    t->cols = t->cls + nc;
+    t->rows = t->cols + (size_t)most * nslots;
+    t->gcls = t->rows + nslots;
+    upload(ctx, t->cls, cls.data(), nc);
+    upload(ctx, t->rows, rows.data(), nslots);
+    upload(ctx, t->gcls, gcls.data(), ng);
+    {
+        Launch L(ctx, MGLDG_K_SETUP);
+        k_rep_cols<<<std::min((nslots + 255) / 256, ctx->sm_count * 8), 256, 0, ctx->stream>>>(
+            nslots, gs, most, t->rows, A->row_ptr, A->col_idx, t->cols);
     }
-    sync(ctx);
+    check_launch();
+    sync(ctx);   // the host arrays go out of scope
     A->rep = t.release();
 }
 
 bool rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv) {
-    if (A->rep) return A->rep->nslots != 0;
+    if (A->rep) return true;
     int distinct = 0;
     if (!rep_sample(ctx, A, &distinct, true)) return false;
     sync(ctx);
     rep_build(ctx, A, Dinv, distinct, 4);
-    return A->rep && A->rep->nslots != 0;
+    return A->rep != nullptr;
 }
 
 // ---------------------------------------------------------------- kernels --
@@ -1108,7 +1103,8 @@ bool rep_launch(mgldg_ctx* ctx, const RepTable* t, RepArgs<T>& a, bool f16, int 
 
 }  // namespace
 
-static bool rep_used(const RepTable* t) { return t && t->nslots && t->nbr >= rep_min_rows(t->b); }
+// (groups of 4 slots, made for multi-vectors, are no whole warps)
+static bool rep_used(const RepTable* t) { return t && t->gs >= 16 && t->nbr >= rep_min_rows(t->b); }
 
 template <class T>
 bool rep_spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const T* yin, T* y, const T* dotv,

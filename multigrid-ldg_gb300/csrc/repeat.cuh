@@ -7,7 +7,7 @@ namespace mg {
 
 // Table form of a square block-sparse operator whose blocks repeat (grids
 // with constant coefficients: 17 distinct blocks on every uniform level).
-// A stored block k is table entry blk[k]; rows with the same sequence of
+// Rows with the same sequence of
 // table entries form a class, and the slots list the rows class by class, gs
 // to a group, so that a warp applies one block to many rows at once.
 //
@@ -19,8 +19,7 @@ namespace mg {
 struct RepView {
     int b = 0, ld = 0, nbr = 0, nuniq = 0, ndiag = 0, ncls = 0;
     int gs = 16, gu = 16;          // slots per group, every group one class; slots per gcls entry
-    int nslots = 0;                // 0: too many classes for the slot kernels
-    int* blk = nullptr;            // [nnzb] table entry of every stored block
+    int nslots = 0;
     unsigned* mask = nullptr;      // [nuniq] nonzero rows | nonzero columns << 16
     int* cls = nullptr;            // [ncls][kRepCls]: blocks per row, inverse diagonal block, -, -, entries, their masks
     int* gcls = nullptr;           // [nslots / gu] class of gu consecutive slots

@@ -317,7 +317,7 @@ void mm_dispatch(mgldg_ctx* ctx, MMArgs<double>& a, bool two, bool jacobi, int k
 
 bool rep_spmm(mgldg_ctx* ctx, const mgldg_bsr* A, const RepMM& m, int kclass) {
     const RepTable* t = A->rep;
-    if (!t || !t->nslots || t->nbr < kRepMmRows) return false;
+    if (!t || t->nbr < kRepMmRows) return false;
     MMArgs<double> a = mm_args<double>(t, m.k);
     a.X = m.X;
     a.Yin = m.Yin;
@@ -339,7 +339,7 @@ bool rep_spmm(mgldg_ctx* ctx, const mgldg_bsr* A, const RepMM& m, int kclass) {
 }
 bool rep_spmm_df64(mgldg_ctx* ctx, const mgldg_bsr* A, int k, const float* Dhi, const float* Dlo, double* Q) {
     const RepTable* t = A->rep;
-    if (!t || !t->nslots || t->nbr < kRepMmRows) return false;
+    if (!t || t->nbr < kRepMmRows) return false;
     MMArgs<float> a = mm_args<float>(t, k);
     a.X = Dhi;
     a.ngroups = t->nslots;

@@ -682,10 +682,12 @@ void dense_spd_inverse(mgldg_ctx* ctx, const mgldg_bsr* A, double* out_inv) {
             k_mark_absent<<<(n + 7) / 8, 256, 0, ctx->stream>>>(n, aug, absent);
         }
         if (n <= kGjMaxN) {
-            const size_t smem = gj_smem(n);
-            MG_CHECK_CUDA(cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            // the limit belongs to the kernel, not to the context: the same
+            // value from every host thread
+            MG_CHECK_CUDA(cudaFuncSetAttribute(k_gauss_jordan, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)gj_smem(kGjMaxN)));
             Launch L(ctx, MGLDG_K_SETUP);
-            k_gauss_jordan<<<kGjCtas, 1024, smem, ctx->stream>>>(n, aug, absent, out_inv, dstatus);
+            k_gauss_jordan<<<kGjCtas, 1024, gj_smem(n), ctx->stream>>>(n, aug, absent, out_inv, dstatus);
         } else {
             {
                 Launch L(ctx, MGLDG_K_SETUP);

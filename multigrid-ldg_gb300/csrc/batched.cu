@@ -1854,7 +1854,7 @@ __global__ void k_seg_cond(BatchScalars sc, cudaGraphConditionalHandle h) {
 // one iteration of every active segment's pcg (krylov.h:43-61); `it` < 0:
 // the iteration index is the device-side counter (graph capture)
 static void seg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, SegWork* w, const double* b, double* x,
-                          double tol2, int maxit, bool replace, int it) {
+                          double tol2, int maxit, bool replace, int it, bool eager) {
     const int nseg = w->nseg;
     BatchScalars sc = w->sc;
     const dim3 grid(w->gx, nseg);
@@ -1886,7 +1886,7 @@ static void seg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, SegWo
         k_segupdate<<<grid, 256, 0, ctx->stream>>>(w->off, nseg, sc, w->Q, w->R, b32, w->prr);
     }
     check_launch();
-    mg_precon_inplace(m, w->R);
+    mg_precon_inplace(m, w->R, eager);
     {
         Launch L(ctx, MGLDG_K_VECTOR);
         if (mixed) k_segdot<float><<<grid, 256, 0, ctx->stream>>>(w->off, nseg, w->R, L0.x32, w->partials);
@@ -1923,7 +1923,7 @@ static bool build_seg_graph(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, Seg
         return false;
     }
     try {
-        seg_iteration(ctx, m, A, w, b, x, tol2, maxit, true, -1);
+        seg_iteration(ctx, m, A, w, b, x, tol2, maxit, true, -1, true);
         for (int k = 0; k < MGLDG_K_NCLASS; ++k) w->pro_launches[k] = ctx->launches[k] - before[k];
         cudaStreamCaptureStatus st;
         cudaGraph_t cg = nullptr;
@@ -1951,7 +1951,7 @@ static bool build_seg_graph(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, Seg
             std::memcpy(b2, ctx->launches, sizeof b2);
             MG_CHECK_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0,
                                                         cudaStreamCaptureModeThreadLocal));
-            seg_iteration(ctx, m, A, w, b, x, tol2, maxit, false, -1);
+            seg_iteration(ctx, m, A, w, b, x, tol2, maxit, false, -1, true);
             k_seg_cond<<<1, 1, 0, ctx->stream>>>(w->sc, h);
             check_launch();
             cudaGraph_t bg = nullptr;
@@ -2034,7 +2034,7 @@ static void segpcg(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const std::v
                 continue;
             }
         }
-        seg_iteration(ctx, m, A, w, b, x, tol2, maxit, i % 50 == 0, i);
+        seg_iteration(ctx, m, A, w, b, x, tol2, maxit, i % 50 == 0, i, false);
         MG_CHECK_CUDA(cudaMemcpyAsync(w->h_counter, sc.counter, 3 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
         sync(ctx);
         ++i;

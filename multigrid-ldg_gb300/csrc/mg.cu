@@ -697,9 +697,16 @@ static void ensure_pcg(mgldg_mg* m, mgldg_ctx* ctx, int64_t n, int maxit) {
     }
 }
 
-// Captures one preconditioner application (x = 0, b = r, V-cycle, s = x) as
-// a CUDA graph.  Returns null (and stops trying) if the capture is refused.
-static mgldg_mg::Graph* capture_precon(mgldg_mg* m, const double* r, double* s, double* part) {
+// where the V-cycle leaves its result (the sweeps swap it with a second array)
+static void* level_x(const mgldg_mg* m) {
+    return m->p.precision != MGLDG_PREC_FP64 ? (void*)m->L[0].x32 : (void*)m->L[0].x;
+}
+
+// Captures one preconditioner application -- x = 0, b = r, V-cycle, s = x, or
+// without s the in-place form -- as a CUDA graph.  Returns null (and stops
+// trying) if the capture is refused.
+static void inplace_vcycle(mgldg_mg* m, double* r);
+static mgldg_mg::Graph* capture_precon(mgldg_mg* m, double* r, double* s, double* part) {
     mgldg_ctx* ctx = m->ctx;
     mgldg_mg::Graph& g = m->graphs[m->next_graph];
     m->next_graph ^= 1;
@@ -717,7 +724,8 @@ static mgldg_mg::Graph* capture_precon(mgldg_mg* m, const double* r, double* s, 
     }
     bool ok = true;
     try {
-        vcycle_dev(m, r, s, true, part);
+        if (s) vcycle_dev(m, r, s, true, part);
+        else inplace_vcycle(m, r);
     } catch (...) {
         ok = false;
     }
@@ -740,39 +748,48 @@ static mgldg_mg::Graph* capture_precon(mgldg_mg* m, const double* r, double* s, 
     g.in = r;
     g.out = s;
     g.part = part;
+    g.z = level_x(m);
     return &g;
 }
 
+// replays that application's graph (made on first use); false: issue its
+// launches directly (per-kernel event timing needs them, or no graph)
+static bool replay_precon(mgldg_mg* m, double* r, double* s, double* part) {
+    mgldg_ctx* ctx = m->ctx;
+    if (ctx->prof || m->graphs_off) return false;
+    mgldg_mg::Graph* g = nullptr;
+    for (auto& c : m->graphs)
+        if (c.exec && c.in == r && c.out == s && c.part == part) g = &c;
+    if (!g) g = capture_precon(m, r, s, part);
+    if (!g) return false;
+    MG_CHECK_CUDA(cudaGraphLaunch(g->exec, ctx->stream));
+    for (int k = 0; k < MGLDG_K_NCLASS; ++k) ctx->launches[k] += g->launches[k];
+    LevelData& L = m->L[0];
+    if (level_x(m) != g->z) {
+        if (m->p.precision != MGLDG_PREC_FP64) std::swap(L.x32, L.xt32);
+        else std::swap(L.x, L.xt);
+    }
+    return true;
+}
+
 // s = M(r); with `part`, also the partial sums of r.s (reduce_grid(n) of them)
-static void precon(mgldg_mg* m, const double* r, double* s, double* part = nullptr) {
+static void precon(mgldg_mg* m, double* r, double* s, double* part = nullptr) {
     mgldg_ctx* ctx = m->ctx;
     if (m->L.empty()) {
         MG_CHECK_CUDA(cudaMemcpyAsync(s, r, m->pcg_n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
         return;
     }
-    // per-kernel event timing needs eager launches
-    if (!ctx->prof && !m->graphs_off) {
-        mgldg_mg::Graph* g = nullptr;
-        for (auto& c : m->graphs)
-            if (c.exec && c.in == r && c.out == s && c.part == part) g = &c;
-        if (!g) g = capture_precon(m, r, s, part);
-        if (g) {
-            MG_CHECK_CUDA(cudaGraphLaunch(g->exec, ctx->stream));
-            for (int k = 0; k < MGLDG_K_NCLASS; ++k) ctx->launches[k] += g->launches[k];
-            return;
-        }
-    }
-    vcycle_dev(m, r, s, true, part);
+    if (!replay_precon(m, r, s, part)) vcycle_dev(m, r, s, true, part);
 }
 
-void mg_precon(mgldg_mg* m, const double* r, double* s) { precon(m, r, s); }
+void mg_precon(mgldg_mg* m, double* r, double* s) { precon(m, r, s); }
 void mg_take_errors(mgldg_mg* m) { take_errors(m); }
 
 // z = V-cycle(r) from x = 0 for the CG, without copies of the FP64 vectors:
 // in the mixed forms the level's FP32 right-hand side has been written by the
 // caller, in FP64 the level reads r itself (unless the one-level hierarchy
 // projects its right-hand side in place); the result stays in the level's x.
-void mg_precon_inplace(mgldg_mg* m, double* r) {
+static void inplace_vcycle(mgldg_mg* m, double* r) {
     mgldg_ctx* ctx = m->ctx;
     LevelData& L = m->L[0];
     struct LevelReset {
@@ -799,11 +816,17 @@ void mg_precon_inplace(mgldg_mg* m, double* r) {
     vcycle<double>(m, 0, z);
 }
 
+// `eager`: launches issued directly (inside a graph capture), else replayed
+// from a graph of their own where there is one
+void mg_precon_inplace(mgldg_mg* m, double* r, bool eager) {
+    if (eager || !replay_precon(m, r, nullptr, nullptr)) inplace_vcycle(m, r);
+}
+
 // partial sums of r.z, z the level's x after mg_precon_inplace
-static void cg_precon(mgldg_mg* m, double* r, double* part, int grid) {
+static void cg_precon(mgldg_mg* m, double* r, double* part, int grid, bool eager) {
     mgldg_ctx* ctx = m->ctx;
     LevelData& L = m->L[0];
-    mg_precon_inplace(m, r);
+    mg_precon_inplace(m, r, eager);
     Launch K(ctx, MGLDG_K_VECTOR);
     if (m->p.precision != MGLDG_PREC_FP64) k_out_part<float><<<grid, 256, 0, ctx->stream>>>(L.n, L.x32, r, part);
     else k_out_part<double><<<grid, 256, 0, ctx->stream>>>(L.n, L.x, r, part);
@@ -814,9 +837,9 @@ static void cg_precon(mgldg_mg* m, double* r, double* part, int grid) {
 // alpha, r -= alpha q (or, when `replace`, x += alpha d and r = b - A x),
 // s = M(r), ||r|| into the history at the device-side iteration index,
 // delta_new = r.s, beta (which advances the iteration counter), x += alpha d,
-// d = s + beta d.
+// d = s + beta d.  `eager`: inside a graph capture.
 static void pcg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const double* b, double* x, int64_t n,
-                          bool df, int grid_vec, bool replace) {
+                          bool df, int grid_vec, bool replace, bool eager) {
     double* part = ctx->d_partials;
     double* prr = part + ctx->n_partials / 2;   // r.r partials, read with r.z's
     const bool mixed = m->p.precision != MGLDG_PREC_FP64;
@@ -849,7 +872,7 @@ static void pcg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const
     // s = M(r) ; delta_new = r.s ; beta ; x += alpha d ; d = s + beta d
     np = grid_vec;
     if (m->L.empty()) dot_partials<double>(ctx, (int)n, m->r, m->r, part, &np);
-    else cg_precon(m, m->r, part, grid_vec);
+    else cg_precon(m, m->r, part, grid_vec, eager);
     {
         Launch L(ctx, MGLDG_K_VECTOR);
         k_pcg_beta<<<1, 256, 0, ctx->stream>>>(m->sc, prr, nrr, part, np, m->hist);
@@ -889,7 +912,7 @@ static bool build_pcg_graph(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, con
     }
     cudaGraph_t body = nullptr;
     try {
-        pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, true);
+        pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, true, true);
         for (int k = 0; k < MGLDG_K_NCLASS; ++k) G.pro_launches[k] = ctx->launches[k] - before[k];
         cudaStreamCaptureStatus st;
         cudaGraph_t cg = nullptr;
@@ -919,7 +942,7 @@ static bool build_pcg_graph(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, con
             std::memcpy(b2, ctx->launches, sizeof b2);
             MG_CHECK_CUDA(cudaStreamBeginCaptureToGraph(ctx->stream, body, nullptr, nullptr, 0,
                                                         cudaStreamCaptureModeThreadLocal));
-            pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, false);
+            pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, false, true);
             k_pcg_cond<<<1, 1, 0, ctx->stream>>>(m->sc, tol2, maxit, h);
             check_launch();
             cudaGraph_t bg = nullptr;
@@ -1012,7 +1035,7 @@ static void pcg_dev(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, const doubl
                 continue;
             }
         }
-        pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, i % 50 == 0);
+        pcg_iteration(ctx, m, A, b, x, n, df, grid_vec, i % 50 == 0, false);
         MG_CHECK_CUDA(cudaMemcpyAsync(m->h_sc, m->sc, sizeof(PcgScalars), cudaMemcpyDeviceToHost, ctx->stream));
         sync(ctx);
         ++i;

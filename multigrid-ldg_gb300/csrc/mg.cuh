@@ -48,11 +48,11 @@ struct SegWork;
 void seg_free(SegWork* w);
 // one preconditioner application s = V-cycle(r) from x = 0 (graph replay
 // when possible) and the collection of device-side error reports (mg.cu)
-void mg_precon(mgldg_mg* m, const double* r, double* s);
-// z = V-cycle(r) from x = 0 with every launch issued directly (for capture
-// into a graph), z left in level 0's x (x32 in the mixed forms, whose FP32
-// right-hand side b32 the caller has written)
-void mg_precon_inplace(mgldg_mg* m, double* r);
+void mg_precon(mgldg_mg* m, double* r, double* s);
+// z = V-cycle(r) from x = 0, left in level 0's x (x32 in the mixed forms, whose
+// FP32 right-hand side b32 the caller has written); eager: every launch issued
+// directly (for capture into a graph)
+void mg_precon_inplace(mgldg_mg* m, double* r, bool eager);
 void mg_take_errors(mgldg_mg* m);
 // true when level i's V-cycle starts from x = 0 with a Jacobi sweep that
 // reads neither x nor the operator, so x need not be zeroed (mg.cu)
@@ -85,6 +85,7 @@ struct mgldg_mg {
         const double* in = nullptr;
         double* out = nullptr;
         double* part = nullptr;   // r.s partial sums written by the graph (or none)
+        void* z = nullptr;        // level 0's x after it (out null: the result)
         cudaGraphExec_t exec = nullptr;
         int64_t launches[MGLDG_K_NCLASS] = {0};
     };

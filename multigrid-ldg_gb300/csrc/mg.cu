@@ -1105,12 +1105,13 @@ static void level_alloc(mgldg_ctx* ctx, mgldg_mg* m, LevelData& L, bool need_sch
         L.Dinv = dalloc<double>((size_t)L.ne * L.b * L.b);
         block_inverse(ctx, L.A, L.Dinv, dstatus);
         int h = 0, distinct = 0;
-        const bool sampled = rep_sample(ctx, L.A, &distinct);
+        const bool finest = &L == &m->L[0];
+        const bool sampled = rep_sample(ctx, L.A, m->p.precision, finest, &distinct);
         download(ctx, &h, dstatus, 1);
         sync(ctx);
         MG_REQUIRE(h == 0, MGLDG_ERR_NOT_SPD, "singular diagonal block in a level matrix");
         // operators made of a few distinct blocks get their table form
-        if (sampled) rep_build(ctx, const_cast<mgldg_bsr*>(L.A), L.Dinv, distinct);
+        if (sampled) rep_build(ctx, const_cast<mgldg_bsr*>(L.A), L.Dinv, m->p.precision, finest, distinct);
     } catch (...) {
         dfree(dstatus);
         throw;

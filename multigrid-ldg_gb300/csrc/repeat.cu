@@ -293,22 +293,74 @@ __global__ void __launch_bounds__(256) k_rep_tables(const double* __restrict__ v
     }
 }
 
-// Rows from which a level is looked at: below, a launch is latency (copying
-// the images, one class after another) and the general kernels, with a warp
-// per row, end sooner.  Measured Jacobi sweeps (event times, us, slot /
-// general): 16 x 16 FP32 16,384 rows 13.1 / 20.3, 4,096 rows 12.6 / 10.0; FP64
-// 16,384 rows 36.9 / 55.9, 4,096 rows 27.8 / 20.0; 9 x 9 FP32 65,536 rows
-// 14.7 / 29.8, 16,384 rows 11.2 / 10.9; FP64 16,384 rows 25.8 / 27.9; 4 x 4
-// FP32 65,536 rows 9.7 / 11.0, 16,384 rows 8.1 / 7.4.
-static int rep_min_rows(int b) { return b == 16 ? 8192 : (b == 9 ? 16384 : 32768); }
+// Where the table kernels pay (event times in us, general / table; u: 26
+// images as on uniform grids, otherwise quadtree levels).  A launch copies the
+// images (nuniq blocks, ndiag inverse diagonal ones) to every CTA, their size
+// bounds the CTAs of an SM, and a warp's rows of one class lie apart in the
+// vectors: many rows and few images pay, the more the wider the block and in
+// FP64, whose pipes the general kernels load with the zeros.
+//   4 x 4, FP64 sweep: 47,899 rows 124 images 22.2 / 19.5, 65,536 u 28.2 / 20.2,
+//     30,916 84 18.2 / 18.2 (residual 20.6 / 21.9), 55,567 472 24.6 / 30.6;
+//     FP32: 65,536 u 11.8 / 9.5, 109,825 98 14.5 / 12.7, 47,899 124 9.8 / 9.9,
+//     38,218 148 8.1 / 9.9, 77,575 492 12.2 / 13.9; double-float product: 65,536 u
+//     25.2 / 21.7, 52,210 with 69 distinct 23.3 / 21.6, 47,899 82 20.8 / 22.6
+//   9 x 9, FP64 sweep: 16,384 u 27.4 / 26.0, 50,347 70 67.6 / 54.8, 26,431 84 41.3 /
+//     45.1, 16,765 118 28.9 / 36.6; FP32: 65,536 u 30.1 / 14.8, 50,347 70 24.1 /
+//     21.2, 16,384 u 10.0 / 11.3 (residual 11.4 / 15.1), 47,899 120 23.1 / 26.1
+//     (23.6 / 30.5), 65,593 96 30.3 / 27.2, 143,032 140 55.7 / 41.0; double-float:
+//     50,347 47 73.8 / 60.5, 47,899 80 73.7 / 76.5, 26,431 56 44.8 / 55.5, 16,384 17
+//     30.0 / 31.0
+//   16 x 16, FP64 sweep: 16,384 u 56.2 / 35.2, 4,096 u 20.0 / 27.8; FP32: 16,384 u
+//     20.7 / 11.3, 26,431 84 32.2 / 24.8, 15,559 96 22.5 / 22.9 (21.7 / 19.1),
+//     11,542 88 17.8 / 22.0; FP16 values: 16,384 u 15.3 / 12.6, 65,593 96 49.5 /
+//     32.8, 30,916 98 28.2 / 27.5, 26,431 84 25.2 / 28.5, 15,559 96 17.4 / 25.1
+enum class Form { F64, F32, F16, DF };   // DF: the double-float product, which reads both halves of the blocks
+
+// most images of a form with this many rows, -1: none
+static int64_t rep_most_images(int b, Form f, int64_t rows) {
+    if (b == 4) {
+        if (f == Form::F64) return rows < 40000 ? -1 : rows / 160;
+        if (f == Form::DF) return rows < 50000 ? -1 : rows / 600;
+        return rows < 65536 ? -1 : rows / 400;
+    }
+    if (b == 9) {
+        if (f == Form::F64) return rows < 16384 ? -1 : rows / 500;
+        if (f == Form::DF) return rows < 32768 ? -1 : rows / 700;
+        return rows < 32768 ? -1 : (rows < 65536 ? rows / 650 : rows / 400);
+    }
+    if (rows < 8192) return -1;
+    return f == Form::F64 || f == Form::DF ? 1 << 30 : (f == Form::F16 ? rows / 400 : rows / 160);
+}
+
+constexpr int kRepSmem = 100 * 1024;   // largest shared-memory image (two CTAs per SM)
+
+// bytes of `count` images in shared memory
+static size_t rep_image_bytes(int b, Form f, int64_t count) {
+    if (f == Form::F64) return 8 * count * (b == 16 ? Img<double, 16>::SIZE : b * ((b + 3) / 4 * 4));
+    return (f == Form::DF ? 8 : 4) * count * (b == 16 ? Img<float, 16>::SIZE : b * ((b + 3) / 4 * 4));
+}
+
+static bool rep_pays(int b, Form f, int64_t rows, int64_t nuniq, int64_t ndiag) {
+    const int64_t count = f == Form::DF ? nuniq : nuniq + ndiag;
+    return count <= rep_most_images(b, f, rows) && rep_image_bytes(b, f, count) <= (size_t)kRepSmem;
+}
+
+// the forms a hierarchy's level runs in: its V-cycle's, on the finest level
+// also the outer product's
+static std::vector<Form> rep_forms(int b, int precision, bool finest) {
+    if (precision == MGLDG_PREC_FP64) return {Form::F64};
+    std::vector<Form> f{precision == MGLDG_PREC_MIXED_F16 && b == 16 ? Form::F16 : Form::F32};
+    if (finest) f.push_back(Form::DF);
+    return f;
+}
 
 static bool rep_shape(const mgldg_bsr* A, int min_rows) {
     return A->br == A->bc && A->nbr == A->nbc && !A->blk && (A->br == 4 || A->br == 9 || A->br == 16) &&
            A->nbr >= min_rows && A->nnzb < (1LL << 31);
 }
 
-bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int* distinct, bool batch) {
-    if (A->rep || !rep_shape(A, batch ? kRepMmRows : rep_min_rows(A->br))) return false;
+static bool sample(mgldg_ctx* ctx, const mgldg_bsr* A, int* distinct, int min_rows) {
+    if (A->rep || !rep_shape(A, min_rows)) return false;
     // keys and count in the reduction scratch
     unsigned long long* keys = (unsigned long long*)ctx->d_partials;
     int* count = (int*)(keys + kSampleKeys);
@@ -324,7 +376,15 @@ bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int* distinct, bool batch) {
     return true;
 }
 
-void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, int gs_want) {
+bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int precision, bool finest, int* distinct) {
+    bool any = false;
+    for (Form f : rep_forms(A->br, precision, finest)) any = any || rep_most_images(A->br, f, A->nbr) >= 2;
+    return any && sample(ctx, A, distinct, 1);
+}
+
+// pays(nuniq, ndiag): whether a table of that size is wanted
+template <class F>
+static void build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, int gs_want, F&& pays) {
     // (both hold for all blocks if they hold for a sample)
     if (distinct > kMaxUniq || (int64_t)distinct * 4 > A->nnzb) return;
     const int b = A->br, n = A->nbr, ld = (b + 3) / 4 * 4;
@@ -409,6 +469,7 @@ void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, i
         int& d = drow[cls[(size_t)c * kRepCls + 1]];
         if (d < 0) d = cls_first[c];
     }
+    if (!pays(nu, nu - (int)std::count(drow.begin(), drow.end(), -1))) return;
     // ---- slots: the rows of a chunk sorted by class, each class padded to
     // whole groups.  Chunks of 4,096 consecutive rows keep a warp's gathers
     // within one stretch of the vectors; with many classes one chunk wastes
@@ -506,19 +567,26 @@ void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, i
     A->rep = t.release();
 }
 
+void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int precision, bool finest, int distinct) {
+    build(ctx, A, Dinv, distinct, 0, [&](int nuniq, int ndiag) {
+        bool any = false;
+        for (Form f : rep_forms(A->br, precision, finest))
+            any = any || rep_pays(A->br, f, A->nbr, nuniq, ndiag);
+        return any;
+    });
+}
+
 bool rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv) {
     if (A->rep) return true;
     int distinct = 0;
-    if (!rep_sample(ctx, A, &distinct, true)) return false;
+    if (!sample(ctx, A, &distinct, kRepMmRows)) return false;
     sync(ctx);
-    rep_build(ctx, A, Dinv, distinct, 4);
+    build(ctx, A, Dinv, distinct, 4, [](int, int) { return true; });
     return A->rep != nullptr;
 }
 
 // ---------------------------------------------------------------- kernels --
 namespace {
-
-constexpr int kRepSmem = 100 * 1024;   // largest shared-memory image (two CTAs per SM)
 
 template <class T>
 struct RepArgs {
@@ -1059,11 +1127,9 @@ RepArgs<T> rep_args(const RepTable* t, bool f16) {
 }
 
 // one launch of a slot kernel (128 threads, `smem` bytes of images): as many
-// CTAs as fit at once, so that each copies the images once; false when the
-// images are too large
+// CTAs as fit at once, so that each copies the images once
 template <class K, class A>
-bool rep_launch_k(mgldg_ctx* ctx, K kern, const A& a, size_t smem, int kclass, int* npart) {
-    if (smem > (size_t)kRepSmem) return false;
+void rep_launch_k(mgldg_ctx* ctx, K kern, const A& a, size_t smem, int kclass, int* npart) {
     if (smem > 48 * 1024)
         MG_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRepSmem));
     int per_sm = 0;
@@ -1076,47 +1142,55 @@ bool rep_launch_k(mgldg_ctx* ctx, K kern, const A& a, size_t smem, int kclass, i
     }
     check_launch();
     if (npart) *npart = grid;
-    return true;
 }
 
 template <class T, bool JACOBI>
-bool rep_launch(mgldg_ctx* ctx, const RepTable* t, RepArgs<T>& a, bool f16, int kclass, int* npart) {
+void rep_launch(mgldg_ctx* ctx, const RepTable* t, RepArgs<T>& a, Form form, int kclass, int* npart) {
     const int E = std::is_same<T, float>::value ? t->gs / 16 : 1;
     a.nwarps = t->b == 16 ? t->nslots / (16 * E) : t->nslots / 32;
-    const size_t smem = (size_t)a.nimg * sizeof(T) *
-                        (t->b == 16 ? Img<T, 16>::SIZE : (t->b == 9 ? Img<T, 9>::SIZE : Img<T, 4>::SIZE));
-    if (t->b == 4) return rep_launch_k(ctx, k_repc<T, 4, JACOBI>, a, smem, kclass, npart);
-    if (t->b == 9) return rep_launch_k(ctx, k_repc<T, 9, JACOBI>, a, smem, kclass, npart);
-    if constexpr (std::is_same<T, float>::value) {
+    const size_t smem = rep_image_bytes(t->b, form, a.nimg);
+    if (t->b == 4) {
+        rep_launch_k(ctx, k_repc<T, 4, JACOBI>, a, smem, kclass, npart);
+    } else if (t->b == 9) {
+        rep_launch_k(ctx, k_repc<T, 9, JACOBI>, a, smem, kclass, npart);
+    } else if constexpr (std::is_same<T, float>::value) {
         // two rows per lane pair from 32,768 rows on (four measured no better:
         // 35.7 against 32.5 us per sweep of 262,144 rows)
-        if (f16) {
-            if (E == 2) return rep_launch_k(ctx, k_rep16<float, 2, JACOBI, true>, a, smem, kclass, npart);
-            return rep_launch_k(ctx, k_rep16<float, 1, JACOBI, true>, a, smem, kclass, npart);
+        if (form == Form::F16) {
+            if (E == 2) rep_launch_k(ctx, k_rep16<float, 2, JACOBI, true>, a, smem, kclass, npart);
+            else rep_launch_k(ctx, k_rep16<float, 1, JACOBI, true>, a, smem, kclass, npart);
+        } else {
+            if (E == 2) rep_launch_k(ctx, k_rep16<float, 2, JACOBI, false>, a, smem, kclass, npart);
+            else rep_launch_k(ctx, k_rep16<float, 1, JACOBI, false>, a, smem, kclass, npart);
         }
-        if (E == 2) return rep_launch_k(ctx, k_rep16<float, 2, JACOBI, false>, a, smem, kclass, npart);
-        return rep_launch_k(ctx, k_rep16<float, 1, JACOBI, false>, a, smem, kclass, npart);
     } else {
-        return rep_launch_k(ctx, k_rep16<double, 1, JACOBI, false>, a, smem, kclass, npart);
+        rep_launch_k(ctx, k_rep16<double, 1, JACOBI, false>, a, smem, kclass, npart);
     }
 }
 
 }  // namespace
 
 // (groups of 4 slots, made for multi-vectors, are no whole warps)
-static bool rep_used(const RepTable* t) { return t && t->gs >= 16 && t->nbr >= rep_min_rows(t->b); }
+static bool rep_used(const RepTable* t, Form f) {
+    return t && t->gs >= 16 && rep_pays(t->b, f, t->nbr, t->nuniq, t->ndiag);
+}
+template <class T>
+static Form form_of(const RepTable* t, bool f16) {
+    if (std::is_same<T, double>::value) return Form::F64;
+    return f16 && t && t->b == 16 ? Form::F16 : Form::F32;   // smaller blocks keep FP32 in the F16 form
+}
 
 template <class T>
 bool rep_spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const T* yin, T* y, const T* dotv,
               double* partials, int* npart, int kclass, bool f16) {
     const RepTable* t = A->rep;
-    if (!rep_used(t)) return false;
+    const Form form = form_of<T>(t, f16);
+    if (!rep_used(t, form)) return false;
     // 16 x 16: whole 16-byte words of every vector (the general kernels read
     // only x that way)
     if (t->b == 16 && ((uintptr_t)x | (uintptr_t)(beta != T(0) ? yin : nullptr) | (uintptr_t)y | (uintptr_t)dotv) % 16)
         return false;
-    f16 = f16 && t->b == 16;   // smaller blocks keep FP32 in the F16 form
-    RepArgs<T> a = rep_args<T>(t, f16);
+    RepArgs<T> a = rep_args<T>(t, form == Form::F16);
     a.x = x;
     a.b = yin;
     a.y = y;
@@ -1125,7 +1199,8 @@ bool rep_spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, c
     a.self_dot = (dotv != nullptr && dotv == y) ? 1 : 0;
     a.dotv = a.self_dot ? nullptr : dotv;
     a.partials = partials;
-    return rep_launch<T, false>(ctx, t, a, f16, kclass, npart);
+    rep_launch<T, false>(ctx, t, a, form, kclass, npart);
+    return true;
 }
 template bool rep_spmv<float>(mgldg_ctx*, const mgldg_bsr*, float, const float*, float, const float*, float*,
                               const float*, double*, int*, int, bool);
@@ -1135,15 +1210,16 @@ template bool rep_spmv<double>(mgldg_ctx*, const mgldg_bsr*, double, const doubl
 template <class T>
 bool rep_jacobi(mgldg_ctx* ctx, const mgldg_bsr* A, const T* b, const T* xin, T* xout, T omega, bool xzero, bool f16) {
     const RepTable* t = A->rep;
-    if (!rep_used(t)) return false;
-    f16 = f16 && t->b == 16;   // smaller blocks keep FP32 in the F16 form
-    RepArgs<T> a = rep_args<T>(t, f16);
+    const Form form = form_of<T>(t, f16);
+    if (!rep_used(t, form)) return false;
+    RepArgs<T> a = rep_args<T>(t, form == Form::F16);
     a.x = xin;
     a.b = b;
     a.y = xout;
     a.omega = omega;
     a.xzero = xzero ? 1 : 0;
-    return rep_launch<T, true>(ctx, t, a, f16, MGLDG_K_JACOBI, nullptr);
+    rep_launch<T, true>(ctx, t, a, form, MGLDG_K_JACOBI, nullptr);
+    return true;
 }
 template bool rep_jacobi<float>(mgldg_ctx*, const mgldg_bsr*, const float*, const float*, float*, float, bool, bool);
 template bool rep_jacobi<double>(mgldg_ctx*, const mgldg_bsr*, const double*, const double*, double*, double, bool,
@@ -1152,7 +1228,7 @@ template bool rep_jacobi<double>(mgldg_ctx*, const mgldg_bsr*, const double*, co
 bool rep_df64(mgldg_ctx* ctx, const mgldg_bsr* A, const float* dhi, const float* dlo, const double* d, double* q,
               double* partials, int* npart) {
     const RepTable* t = A->rep;
-    if (!rep_used(t)) return false;
+    if (!rep_used(t, Form::DF)) return false;
     RepDfArgs a{};
     a.nwarps = t->nslots / (t->b == 16 ? 16 : 32);
     a.nslots = t->nslots;
@@ -1169,10 +1245,11 @@ bool rep_df64(mgldg_ctx* ctx, const mgldg_bsr* A, const float* dhi, const float*
     a.d = d;
     a.q = q;
     a.partials = partials;
-    const size_t s = 2 * sizeof(float) * t->nuniq;
-    if (t->b == 4) return rep_launch_k(ctx, k_repc_df64<4>, a, s * Img<float, 4>::SIZE, MGLDG_K_SPMV, npart);
-    if (t->b == 9) return rep_launch_k(ctx, k_repc_df64<9>, a, s * Img<float, 9>::SIZE, MGLDG_K_SPMV, npart);
-    return rep_launch_k(ctx, k_rep16_df64, a, s * Img<float, 16>::SIZE, MGLDG_K_SPMV, npart);
+    const size_t smem = rep_image_bytes(t->b, Form::DF, t->nuniq);
+    if (t->b == 4) rep_launch_k(ctx, k_repc_df64<4>, a, smem, MGLDG_K_SPMV, npart);
+    else if (t->b == 9) rep_launch_k(ctx, k_repc_df64<9>, a, smem, MGLDG_K_SPMV, npart);
+    else rep_launch_k(ctx, k_rep16_df64, a, smem, MGLDG_K_SPMV, npart);
+    return true;
 }
 
 }  // namespace mg

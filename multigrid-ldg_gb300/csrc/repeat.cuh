@@ -44,15 +44,15 @@ struct RepTable : RepView {
 constexpr int kRepMaxNb = 12;            // longest row
 constexpr int kRepCls = 2 * kRepMaxNb + 4;   // ints per class
 
-// Looks for repeated blocks in A (square blocks of 4, 9 or 16).  rep_sample
-// queues a count of the distinct blocks in a sample, so that its result travels
-// with a synchronisation of the caller; false: not a level for a table.
-// rep_build, given that count, looks at all blocks, checks each against its
-// table entry and attaches the table to A (or leaves A as it is).
-// Dinv: A's inverse diagonal blocks; gs: slots per group (0: the single-vector
-// kernels' choice).
-bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int* distinct, bool batch = false);
-void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, int gs = 0);
+// Looks for repeated blocks in a level operator (square blocks of 4, 9 or 16).
+// rep_sample queues a count of the distinct blocks in a sample, so that its
+// result travels with a synchronisation of the caller; false: no form that the
+// hierarchy's precision runs on this level would use a table.  rep_build, given
+// that count, looks at all blocks, checks each against its table entry and
+// attaches the table to A where one of the forms is faster with it.  Dinv: A's
+// inverse diagonal blocks.
+bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int precision, bool finest, int* distinct);
+void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int precision, bool finest, int distinct);
 
 // the table for multi-vector products (levels from kRepMmRows rows on, also
 // those too small for the single-vector kernels); false: none

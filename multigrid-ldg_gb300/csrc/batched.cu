@@ -1167,9 +1167,14 @@ static void ensure_batch(mgldg_mg* m, int k, const mgldg_bsr* A_outer) {
         b->mean = b->prr + rows * k;
     }
     Batch* b = m->batch;
+    // tables: of every level in FP64, in the mixed forms (FP32 sweeps keep the
+    // general kernels) of the finest for the double-float outer product
     if (!b->tuned)
-        for (auto& L : m->L)
-            if (L.Dinv) rep_ensure_batch(ctx, const_cast<mgldg_bsr*>(L.A), L.Dinv);
+        for (size_t l = 0; l < m->L.size(); ++l) {
+            const bool df64 = m->p.precision != MGLDG_PREC_FP64;
+            if (m->L[l].Dinv && (l == 0 || !df64))
+                rep_ensure_batch(ctx, const_cast<mgldg_bsr*>(m->L[l].A), m->L[l].Dinv, df64);
+        }
     if (!b->tuned) {
         // tile widths per level operator and kernel, on the level buffers
         // (their contents are overwritten before every use)

@@ -576,13 +576,14 @@ void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int precision, 
     });
 }
 
-bool rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv) {
-    if (A->rep) return true;
+void rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, bool df64) {
     int distinct = 0;
-    if (!sample(ctx, A, &distinct, kRepMmRows)) return false;
+    auto pays = [&](int nuniq, int) {
+        return df64 ? rep_mm_df64_pays(A->br, A->nbr) : rep_mm_pays(A->br, A->nbr, nuniq);
+    };
+    if (!pays(1, 1) || !sample(ctx, A, &distinct, kRepMmRows)) return;
     sync(ctx);
-    build(ctx, A, Dinv, distinct, 4, [](int, int) { return true; });
-    return A->rep != nullptr;
+    build(ctx, A, Dinv, distinct, 4, pays);
 }
 
 // ---------------------------------------------------------------- kernels --

@@ -55,9 +55,12 @@ bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int precision, bool finest, 
 void rep_build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int precision, bool finest, int distinct);
 
 // the table for multi-vector products (levels from kRepMmRows rows on, also
-// those too small for the single-vector kernels); false: none
-bool rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv);
+// those too small for the single-vector kernels) where they are faster with it:
+// FP64 sweeps and products, or (df64) the double-float outer product
+void rep_ensure_batch(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, bool df64);
 constexpr int kRepMmRows = 2048;
+bool rep_mm_pays(int b, int64_t rows, int64_t nuniq);
+bool rep_mm_df64_pays(int b, int64_t rows);
 
 // FP64 Y = alpha A X + beta Yin, or (Jacobi) Y = X + omega Dinv (B - A X), on
 // row-major multi-vectors of k columns (spmm_rep.cu); false: no table

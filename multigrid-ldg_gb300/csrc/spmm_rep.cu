@@ -315,9 +315,25 @@ void mm_dispatch(mgldg_ctx* ctx, MMArgs<double>& a, bool two, bool jacobi, int k
 
 }  // namespace
 
+// Where the tables pay (us per sweep, general / table).  FP64 4 x 4 blocks have
+// little to skip, and a warp's rows lose their locality: 49,645 quadtree rows
+// 229 / 238 with 1 column, 456 / 473 with 64; 4,096 of a uniform grid 26 / 28, 45
+// / 53.  9 x 9: 4,096 uniform rows (17 distinct blocks) 95 / 88, 185 / 174, 3,709
+// rows of a quadtree's third coarse level 98 / 89, 176 / 176, but levels with few rows
+// per distinct block 2,230 64 / 74, 111 / 141; 4,096 with 744 blocks 97 / 104, 185 /
+// 203.  16 x 16: 2,230 rows 184 / 203 up to 32 columns, 336 / 306 with 33; 4,096
+// uniform rows 286 / 258.
+bool rep_mm_pays(int b, int64_t rows, int64_t nuniq) {
+    return b == 16 || (b == 9 && rows >= 10 * nuniq);
+}
+// double-float products: 4 x 4 4,096 rows 21 / 23, 10,036 38 / 40, 16,384 even,
+// 25,597 and more faster; the others from kRepMmRows on
+bool rep_mm_df64_pays(int b, int64_t rows) { return b != 4 || rows >= 20000; }
+
 bool rep_spmm(mgldg_ctx* ctx, const mgldg_bsr* A, const RepMM& m, int kclass) {
     const RepTable* t = A->rep;
-    if (!t || t->nbr < kRepMmRows) return false;
+    if (!t || t->nbr < kRepMmRows || !rep_mm_pays(t->b, t->nbr, t->nuniq)) return false;
+    if (t->b == 16 && m.k <= 32 && t->nbr < 3072) return false;
     MMArgs<double> a = mm_args<double>(t, m.k);
     a.X = m.X;
     a.Yin = m.Yin;
@@ -330,16 +346,14 @@ bool rep_spmm(mgldg_ctx* ctx, const mgldg_bsr* A, const RepMM& m, int kclass) {
     const size_t al = 2 * sizeof(double);
     const bool two = m.k % 2 == 0 && m.k > 32 && aligned_to(m.X, al) && aligned_to(m.Yin, al) && aligned_to(m.B, al) &&
                      aligned_to(m.Y, al);
-    switch (t->b) {
-        case 4: mm_dispatch<4>(ctx, a, two, m.jacobi != 0, kclass); return true;
-        case 9: mm_dispatch<9>(ctx, a, two, m.jacobi != 0, kclass); return true;
-        case 16: mm_dispatch<16>(ctx, a, two, m.jacobi != 0, kclass); return true;
-    }
-    return false;
+    if (t->b == 9) mm_dispatch<9>(ctx, a, two, m.jacobi != 0, kclass);
+    else mm_dispatch<16>(ctx, a, two, m.jacobi != 0, kclass);
+    return true;
 }
+
 bool rep_spmm_df64(mgldg_ctx* ctx, const mgldg_bsr* A, int k, const float* Dhi, const float* Dlo, double* Q) {
     const RepTable* t = A->rep;
-    if (!t || t->nbr < kRepMmRows) return false;
+    if (!t || t->nbr < kRepMmRows || !rep_mm_df64_pays(t->b, t->nbr)) return false;
     MMArgs<float> a = mm_args<float>(t, k);
     a.X = Dhi;
     a.ngroups = t->nslots;

@@ -1408,37 +1408,71 @@ extern "C" int mgldg_gs_pass_levels(int nbr, const int* row_ptr, const int* col_
     return MGLDG_OK;
 }
 
-// Runs the Gauss-Seidel kernel on a two-row system in which row 1 waits for
+namespace mg {
+
+// One forward sweep over blocks of B, FP64, of a system of two rows of which
+// only row 1 is scheduled (`pass` fills the work list): it waits for row 0
+// until the time limit.  True if the kernel reported that.
+template <int B, class F>
+static bool wait_runs_out(mgldg_ctx* ctx, int64_t timeout_ns, F&& pass) {
+    std::vector<int> rp{0, 2, 4}, ci{0, 1, 0, 1};
+    mgldg_bsr* A = bsr_new(ctx, 2, 2, B, B, rp, ci);
+    Sched S;
+    double* v = nullptr;   // Dinv, b, x
+    bool out = false;
+    auto clean = [&]() {
+        sched_free(S);
+        dfree(v);
+        delete A;
+    };
+    try {
+        std::vector<double> av(4 * B * B, 0.0), dv(2 * B * B, 0.0);
+        for (int k = 0; k < 4; ++k)
+            for (int r = 0; r < B; ++r) av[((size_t)k * B + r) * B + r] = k == 1 || k == 2 ? 1.0 : 2.0;
+        for (int r = 0; r < 2 * B; ++r) dv[(size_t)r * B + r % B] = 0.5;
+        upload(ctx, A->val, av.data(), av.size());
+        v = dalloc<double>(dv.size() + 4 * B);
+        double *b = v + dv.size(), *x = b + 2 * B;
+        upload(ctx, v, dv.data(), dv.size());
+        MG_CHECK_CUDA(cudaMemsetAsync(b, 0, 4 * B * sizeof(double), ctx->stream));
+        sched_build(ctx, A, S);
+        S.timeout_ns = timeout_ns;
+        S.passes.emplace_back();
+        GsPass& P = S.passes.back();
+        P.nsw = P.nitems = P.depth = 1;
+        pass(P);
+        gs_sweeps<double>(ctx, A, A->val, v, b, x, S, 1.0, false, 1);
+        sync(ctx);
+        MG_REQUIRE(S.passes.size() == 1, MGLDG_ERR_ARG, "self-test: the work list was not taken");
+        out = gs_take_error(ctx, S) != 0;
+        // the context must still work: a plain SpMV
+        spmv<double>(ctx, A, 1.0, b, 0.0, nullptr, x);
+        sync(ctx);
+    } catch (...) {
+        clean();
+        throw;
+    }
+    clean();
+    return out;
+}
+
+}  // namespace mg
+
+// Runs the Gauss-Seidel kernels on two-row systems in which row 1 waits for
 // row 0 but row 0 is never scheduled (a pass whose only item is row 1), so
-// the wait can only end by its time limit.  Reports the status the kernel
+// the wait can only end by its time limit.  Reports the status the kernels
 // left and checks that the stream is still usable afterwards.
 extern "C" int mgldg_selftest_wait_timeout(mgldg_ctx* ctx, int64_t timeout_ns, int* status) {
     MG_API_BEGIN(ctx)
     MG_REQUIRE(status && timeout_ns > 0 && timeout_ns <= 2000000000LL, MGLDG_ERR_ARG, "bad self-test arguments");
-    std::vector<int> rp{0, 2, 4}, ci{0, 1, 0, 1};
-    mgldg_bsr* A = bsr_new(ctx, 2, 2, 1, 1, rp, ci);
-    Sched S;
-    double *dinv = nullptr, *b = nullptr, *x = nullptr;
-    try {
-        const double av[4] = {2.0, 1.0, 1.0, 2.0}, dv[2] = {0.5, 0.5}, zero[2] = {0.0, 0.0};
-        upload(ctx, A->val, av, 4);
-        dinv = dalloc<double>(2); b = dalloc<double>(2); x = dalloc<double>(2);
-        upload(ctx, dinv, dv, 2); upload(ctx, b, dv, 2); upload(ctx, x, zero, 2);
-        sched_build(ctx, A, S);
-        S.timeout_ns = timeout_ns;
-        *status = MGLDG_ERR_TIMEOUT;
-        // row 0 is never run: row 1 waits for it as another CTA's row (in
-        // global memory), then as its own CTA's (in shared memory)
-        // (the number of an item that its list does not have)
-        for (int tag0 = 0; tag0 >= -1; --tag0) {
-            S.passes.emplace_back();
-            GsPass& P = S.passes.back();
+    bool out = true;
+    // tiles: as another CTA's row (in global memory), then as its own CTA's (in
+    // shared memory), under the number of an item that the list does not have
+    for (int tag0 = 0; tag0 >= -1; --tag0)
+        out = wait_runs_out<1>(ctx, timeout_ns, [&](GsPass& P) {
             const signed char tag[4] = {0, 0, (signed char)tag0, 0};
             int tab[7] = {(1 << 3) | 0, 2, 2, 0, /* items */ 0, 1, /* tags */ 0};
             std::memcpy(tab + 6, tag, sizeof tag);
-            P.nsw = 1;
-            P.nitems = 1;
-            P.depth = 1;
             P.grid = 1;
             P.tile = kGsTile<double, 1>;
             P.slots = GsTile<double, 1>::SLOTS;
@@ -1447,23 +1481,15 @@ extern "C" int mgldg_selftest_wait_timeout(mgldg_ctx* ctx, int64_t timeout_ns, i
             P.cta_ptr = P.items + 4;
             P.ltag = reinterpret_cast<signed char*>(P.items + 6);
             upload(ctx, P.items, tab, 7);
-            gs_sweeps<double>(ctx, A, A->val, dinv, b, x, S, 1.0, false, 1);
             sync(ctx);
-            if (!gs_take_error(ctx, S)) *status = MGLDG_OK;
-            pass_free(P);
-            S.passes.pop_back();
-        }
-        // the context must still work: a plain SpMV
-        spmv<double>(ctx, A, 1.0, b, 0.0, nullptr, x);
+        }) && out;
+    // row by row (blocks of 25 and 27)
+    out = wait_runs_out<25>(ctx, timeout_ns, [&](GsPass& P) {
+        const int item = (1 << 3) | 0;
+        P.items = dalloc<int>(1);
+        upload(ctx, P.items, &item, 1);
         sync(ctx);
-    } catch (...) {
-        sched_free(S);
-        dfree(dinv); dfree(b); dfree(x);
-        delete A;
-        throw;
-    }
-    sched_free(S);
-    dfree(dinv); dfree(b); dfree(x);
-    delete A;
+    }) && out;
+    *status = out ? MGLDG_ERR_TIMEOUT : MGLDG_OK;
     MG_API_END
 }

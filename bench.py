@@ -200,10 +200,10 @@ def level_bytes(mg, nlev, s, f16=False):
     blocks, b and x_out only), one SpMV.  f16: the level operator is read from
     its block-scaled FP16 copy (2 bytes per entry + one 4-byte scale per
     block; inverse diagonal blocks and vectors in FP32, s = 4).  The uniform
-    grid's operators have 17 distinct blocks; from TABLE_ROWS block rows on,
-    Jacobi sweeps and products keep them on chip and move indices and vectors
-    only."""
-    TABLE_ROWS = {4: 32768, 9: 16384, 16: 8192}
+    grid's operators have 17 distinct blocks and 9 inverse diagonal ones; from
+    these block rows on (rep_most_images in repeat.cu, for 26 images), Jacobi
+    sweeps and products keep them on chip and move indices and vectors only."""
+    TABLE_ROWS = {16: 10400} if f16 else ({4: 40000, 9: 16384, 16: 8192} if s == 8 else {4: 65536, 9: 32768, 16: 8192})
     out = []
     for l in range(nlev):
         nbr, nbc, br, bc, nnzb = mg.level_op(l, 4).info()

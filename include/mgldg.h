@@ -439,9 +439,9 @@ int mgldg_gs_levels(int nbr, const int* row_ptr, const int* col_idx, int reverse
 int mgldg_gs_pass_levels(int nbr, const int* row_ptr, const int* col_idx, int reverse, int nsw,
                          int* level, int* nlevels);
 /* Failure-detection self test (no reference counterpart): runs the
- * Gauss-Seidel kernel on a two-row system whose dependency is never
- * released, so its bounded wait expires after timeout_ns.  *status receives
- * MGLDG_ERR_TIMEOUT when the kernel reported the expiry; the call itself
+ * Gauss-Seidel kernels on two-row systems whose dependency is never
+ * released, so their bounded waits expire after timeout_ns.  *status receives
+ * MGLDG_ERR_TIMEOUT when every kernel reported the expiry; the call itself
  * returns MGLDG_OK when the context stayed usable. */
 int mgldg_selftest_wait_timeout(mgldg_ctx* ctx, int64_t timeout_ns, int* status);
 

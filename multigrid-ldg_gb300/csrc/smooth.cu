@@ -445,7 +445,8 @@ constexpr int kGsRing = 64;   // most slots
 
 // Rows that go to one CTA: 4 x 4 patches, whose diagonals have a row for each
 // of the SM's warp schedulers (8 x 8: 858 us instead of 449 for the 256 x 256
-// pass; 2 x 2: 382 against 344).  FP64 blocks of 16 are bound by the SM's FP64
+// pass, both before the copies to shared memory; 2 x 2: 382 against 344 with
+// them).  FP64 blocks of 16 are bound by the SM's FP64
 // pipes, which a patch's rows share: 2 x 2 (219 us against 233 for 64 x 64).
 template <class T, int B>
 constexpr int kGsTile = sizeof(T) == 8 && B == 16 ? 4 : 16;

@@ -960,12 +960,12 @@ struct RepDfArgs {
 // q = A d in double-float arithmetic, 16 x 16 blocks, two lanes per row: a
 // float-pair sum per row and column half, the two pairs added as in FP64
 // (PairSum), q and the partial d.q in FP64.  Blocks read by columns take two
-// rows at a time (packed FP32 operations).  Bound by the FP32 pipes (11
-// operations per product, zero block rows and columns skipped; 46 % busy) and
-// the FP64 ones (three operations per entry; adding the halves as float pairs
-// and widening without conversions took away five more; 30 %).  262,144 rows:
-// 122 us with four CTAs an SM and x loaded a block ahead, 110 us with five and
-// without.
+// rows at a time (packed FP32 operations).  The work is on the FP32 pipes (11
+// operations per product, zero block rows and columns skipped; 34 % of the
+// cycles at 65,536 rows, one wave of CTAs) and the FP64 ones (three operations
+// per entry; adding the halves as float pairs and widening without conversions
+// took away five more; 21 %).  262,144 rows: 122 us with four CTAs an SM and x
+// loaded a block ahead, 110 us with five and without.
 __global__ void __launch_bounds__(128, 5) k_rep16_df64(const RepDfArgs a) {
     using I = Img<float, 16>;
     extern __shared__ __align__(16) unsigned char smraw[];

@@ -385,8 +385,8 @@ bool rep_sample(mgldg_ctx* ctx, const mgldg_bsr* A, int precision, bool finest, 
 // pays(nuniq, ndiag): whether a table of that size is wanted
 template <class F>
 static void build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct, int gs_want, F&& pays) {
-    // (both hold for all blocks if they hold for a sample)
-    if (distinct > kMaxUniq || (int64_t)distinct * 4 > A->nnzb) return;
+    // (what rules the sample out rules all blocks out)
+    if (distinct > kMaxUniq || (int64_t)distinct * 4 > A->nnzb || !pays(distinct, 1)) return;
     const int b = A->br, n = A->nbr, ld = (b + 3) / 4 * 4;
     const int* rp = A->h_row_ptr.data();
     if (A->nnzb > (int64_t)kRepMaxNb * n) return;
@@ -428,7 +428,7 @@ static void build(mgldg_ctx* ctx, mgldg_bsr* A, const double* Dinv, int distinct
     sync(ctx);
     // a table pays when a block is used several times
     const int nu = hd[0];
-    if (hd[1] || nu < 1 || (int64_t)nu * 4 > A->nnzb) return;
+    if (hd[1] || nu < 1 || (int64_t)nu * 4 > A->nnzb || !pays(nu, 1)) return;
     std::vector<int> first, cls_first;
     number(slots, first);
     {

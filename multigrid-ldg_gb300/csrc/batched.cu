@@ -689,7 +689,8 @@ struct BatchScalars {
     double *delta_new, *delta_old, *delta0, *alpha, *beta;
     int *active, *iters, *broken;
     int* counter;   // [0] = active columns after the iteration, [1] = broken,
-                    // [2] = completed iterations (segmented PCG only)
+                    // [2] = iterations begun, [3] = the current one's index
+                    // (segmented PCG in a graph only)
 };
 
 __device__ double col_total(const double* partials, int np, int k, int c) {
@@ -858,9 +859,16 @@ __device__ __forceinline__ void column_totals(const double* p1, int n1, const do
     }
 }
 
-// (also clears the counts that k_bpcg_end adds up)
-__global__ void __launch_bounds__(1024) k_bpcg_alpha(int k, BatchScalars sc, const double* partials, int np) {
+// (also clears the counts that k_bpcg_end adds up; `advance`: the device-side
+// iteration index counter[2] moves on, counter[3] keeps this iteration's)
+__global__ void __launch_bounds__(1024) k_bpcg_alpha(int k, BatchScalars sc, const double* partials, int np,
+                                                     int advance) {
     if (blockIdx.x == 0 && threadIdx.x < 2) sc.counter[threadIdx.x] = 0;
+    if (advance && blockIdx.x == 0 && threadIdx.x == 0) {
+        const int at = sc.counter[2];
+        sc.counter[3] = at;
+        sc.counter[2] = at + 1;
+    }
     column_totals(partials, np, nullptr, 0, k, [&](int c, double dq, double) {
         double a = 0;
         if (sc.active[c]) {
@@ -877,13 +885,14 @@ __global__ void __launch_bounds__(1024) k_bpcg_alpha(int k, BatchScalars sc, con
 
 // the end of an iteration: ||r_c|| into the history, delta_new = r_c.z_c,
 // beta, the stopping test and the counts of active and broken columns.
-// it < 0: the iteration index is the device-side counter[2], which advances
-// (one CTA then).
+// it < 0: the iteration index is the device-side counter[3].  (One CTA for all
+// columns, which then advanced the index itself, took 20,000 segments' solves
+// from 13 to 87 ms.)
 __global__ void __launch_bounds__(1024) k_bpcg_end(int k, BatchScalars sc, const double* prr, int nrr,
                                                    const double* prz, int nrz, double* hist, int maxit, double tol2,
                                                    int it) {
     __shared__ int cnt[2];
-    const int at = it >= 0 ? it : sc.counter[2];
+    const int at = it >= 0 ? it : sc.counter[3];
     if (threadIdx.x < 2) cnt[threadIdx.x] = 0;
     __syncthreads();
     column_totals(prr, nrr, prz, nrz, k, [&](int c, double rr, double rs) {
@@ -908,7 +917,6 @@ __global__ void __launch_bounds__(1024) k_bpcg_end(int k, BatchScalars sc, const
     });
     __syncthreads();
     if (threadIdx.x < 2 && cnt[threadIdx.x]) atomicAdd(&sc.counter[threadIdx.x], cnt[threadIdx.x]);
-    if (threadIdx.x == 0 && it < 0) sc.counter[2] = at + 1;
 }
 
 // ---------------------------------------------------- multi-RHS coarse solve
@@ -1614,7 +1622,7 @@ static void bpcg(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, int k, const d
         coldot<double>(ctx, n, k, b->D, b->Q, b->partials, &np);
         {
             Launch L(ctx, MGLDG_K_VECTOR);
-            k_bpcg_alpha<<<(k + 31) / 32, 1024, 0, ctx->stream>>>(k, sc, b->partials, np);
+            k_bpcg_alpha<<<(k + 31) / 32, 1024, 0, ctx->stream>>>(k, sc, b->partials, np, 0);
         }
         check_launch();
         // R -= alpha Q (or X += alpha D, R = B - A X), its column norms and
@@ -1823,7 +1831,7 @@ static SegWork* ensure_seg(mgldg_mg* m, const std::vector<int64_t>& off, int max
         w->partials = dalloc<double>(2 * (size_t)w->gx * nseg);
         w->prr = w->partials + (size_t)w->gx * nseg;
         w->sc_mem = dalloc<double>(5 * (size_t)nseg);
-        w->sc_int = dalloc<int>(3 * (size_t)nseg + 3);
+        w->sc_int = dalloc<int>(3 * (size_t)nseg + 4);
         w->sc.delta_new = w->sc_mem;
         w->sc.delta_old = w->sc_mem + nseg;
         w->sc.delta0 = w->sc_mem + 2 * nseg;
@@ -1874,7 +1882,7 @@ static void seg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, SegWo
     segdot(w->D, w->Q, w->partials);
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_bpcg_alpha<<<(nseg + 31) / 32, 1024, 0, ctx->stream>>>(nseg, sc, w->partials, w->gx);
+        k_bpcg_alpha<<<(nseg + 31) / 32, 1024, 0, ctx->stream>>>(nseg, sc, w->partials, w->gx, it < 0 ? 1 : 0);
     }
     check_launch();
     if (replace) {
@@ -1899,7 +1907,8 @@ static void seg_iteration(mgldg_ctx* ctx, mgldg_mg* m, const mgldg_bsr* A, SegWo
     }
     {
         Launch L(ctx, MGLDG_K_VECTOR);
-        k_bpcg_end<<<1, 1024, 0, ctx->stream>>>(nseg, sc, w->prr, w->gx, w->partials, w->gx, w->hist, maxit, tol2, it);
+        k_bpcg_end<<<(nseg + 31) / 32, 1024, 0, ctx->stream>>>(nseg, sc, w->prr, w->gx, w->partials, w->gx, w->hist,
+                                                              maxit, tol2, it);
     }
     {
         Launch L(ctx, MGLDG_K_VECTOR);

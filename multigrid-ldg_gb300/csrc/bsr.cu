@@ -700,8 +700,11 @@ void spmv(mgldg_ctx* ctx, const mgldg_bsr* A, T alpha, const T* x, T beta, const
     MG_SPMV_ROWS_CASE(9, 9)
     MG_SPMV_ROWS_CASE(10, 10)
 #undef MG_SPMV_ROWS_CASE
+    // (kernels that read x in 16-byte words: a caller's vector may be 8-byte
+    // aligned only, which the generic kernel takes)
+    const bool x16 = (uintptr_t)x % 16 == 0;
 #define MG_SPMV_CASE(R, Cc)                                                                            \
-    if (br == R && bc == Cc) {                                                                         \
+    if (br == R && bc == Cc && (x16 || !RowVec<T, R, Cc>::ok)) {                                       \
         launch_spmv<T, R, Cc>(ctx, A, alpha, x, beta, yin, y, dotv, partials, npart, kclass);          \
         return;                                                                                        \
     }

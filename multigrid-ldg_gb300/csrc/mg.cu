@@ -53,8 +53,8 @@ static void convert(mgldg_ctx* ctx, int64_t n, const A* a, B* b) {
 // coarsest level: x = Cinv b in FP64, one warp per row over all SMs (each
 // CTA stages b in shared memory; Cinv, at most 128 MB, stays L2-resident
 // across V-cycles when it fits).  The optional b -= mean(b) runs first in
-// k_mean_project.  3,942 unknowns: 48 us with one 8-byte load in flight per
-// lane, 41 us with four 16-byte ones; the FP64 pipes alone take 27 us.
+// k_mean_project.  3,942 unknowns: 40 us, of which the FP64 pipes alone take 27;
+// 48 us with the rows in blocks of eight per CTA.
 template <class T>
 __global__ void __launch_bounds__(256) k_coarse_solve(int n, const T* __restrict__ b, T* __restrict__ x,
                                                       const double* __restrict__ Cinv) {

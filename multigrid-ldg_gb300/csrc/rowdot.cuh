@@ -95,14 +95,20 @@ __device__ __forceinline__ void df_fma2(unsigned long long& sh, unsigned long lo
 // (valid in every lane): four 16-byte loads per lane in flight, four partial
 // sums per lane added in a fixed order.  Rows of an odd n start on an odd
 // entry every second time; the entry before the first 16-byte word and one
-// after the last are added apart.  b in shared memory.  Up to kCoarseNarrow
-// unknowns a lane has eight entries at most, and the plain loop ends sooner (144
-// unknowns: 6.2 us against 7.1).
-constexpr int kCoarseNarrow = 256;
+// after the last are added apart.  b in shared memory.
+//
+// The plain loop (up to four 8-byte loads in flight) is the shorter one where a
+// lane has eight entries at most: 256 unknowns 2.4 us against 3.2 with Cinv in
+// L2, 3.0 / 3.5 from HBM.  Between, the wide loads win when Cinv comes from HBM
+// (1,053 unknowns 8.6 / 7.7 us, 1,944 14.3 / 13.0) by more than they lose from L2
+// (5.5 / 6.1, 11.1 / 11.6).  Beyond, a CTA's eight warps have rows enough to
+// cover the latency, and the plain loop has the fewer instructions: 2,304 16.1 /
+// 16.6 (L2 13.6 / 15.2), 4,096 in FP64 V-cycles 40.7 / 43.1.
+constexpr int kCoarseWideMin = 257, kCoarseWideMax = 2048;
 __device__ __forceinline__ double coarse_row(const double* __restrict__ Cinv, const double* b, int n, int row,
                                              int lane) {
     const double* cr = Cinv + (size_t)row * n;
-    if (n <= kCoarseNarrow) {
+    if (n < kCoarseWideMin || n > kCoarseWideMax) {
         double s = 0;
         for (int c = lane; c < n; c += 32) s += __ldg(cr + c) * b[c];
 #pragma unroll
